@@ -263,7 +263,9 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
         copy_set(P.A, a_row0[j], rows_off_a[j]);
         if (!self) copy_set(P.B, b_row0[j], rows_off_b[j]);
         fill_tc_job(&hjobs[j], form, J.d, J.eps * J.eps, P.op_scale, P.maxabs, a_row0[j], P.na_eff, b_row0[j],
-                    P.nb_eff, self, b->d_counts + j, srows + rows_off_a[j], srows + rows_off_b[j], nullptr, nullptr);
+                    P.nb_eff, self, b->d_counts + j, srows + rows_off_a[j], srows + rows_off_b[j], P.A.fold, nullptr,
+                    nullptr);
+        O.fold |= P.A.fold;
         // work items rebased onto the matrix
         if (P.idx_tc.n_items) {
             WorkItem *w = (WorkItem *)b->alloc(P.idx_tc.n_items * sizeof(WorkItem));
@@ -325,7 +327,7 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
         return engine_fail(HJ_ERR_CUDA, std::string("batch planning: ") + cudaGetErrorString(e));
     }
     // size the band queue with one run (regrown once if it overflows)
-    b->band_cap = std::max<uint64_t>(1ull << 20, b->candidate_pairs / 4096);
+    b->band_cap = std::max<uint64_t>(1ull << 20, b->candidate_pairs / 4096) + band_slack(b->num_sms, false);
     for (int attempt = 0; attempt < 3; ++attempt) {
         b->band = (uint2 *)b->alloc(b->band_cap * kBandEntryBytes);
         if (!b->band) return engine_fail(HJ_ERR_OOM, "out of device memory (band queue)");

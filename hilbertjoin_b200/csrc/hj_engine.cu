@@ -243,7 +243,8 @@ static int prepare_set(Ctx *c, cudaStream_t st, const void *x, uint64_t n, int d
     s.dtype_bytes = dtype_bytes;
     s.src = x;
     s.center = center;
-    s.op_scale = form == HJ_FORM_TC_FP16 ? op_scale : 1.0;
+    s.fold = form_is_tc(form) && tc_fold(form, g.d);
+    s.op_scale = form != HJ_FORM_TC_FP16 ? 1.0 : (s.fold ? std::ldexp(op_scale, -kBcScaleShift) : op_scale);
     const uint32_t W = g.W;
     const bool norm_order = form_is_tc(form);
     uint32_t *keys_wm = (uint32_t *)slot_alloc_impl(c, st, is_b ? kSlotKeysWmB : kSlotKeysWmA,
@@ -600,7 +601,7 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
         // scale and 3d + 3 columns)
         auto fill_job = [&]() {
             fill_tc_job(c->h_job, form, d, T, bc ? bc_scale : A.op_scale, maxabs, 0, na_eff, 0, nb_eff, in.self,
-                        d_count, A.rows, B.rows, &c_rel, &c_abs);
+                        d_count, A.rows, B.rows, !bc && A.fold, &c_rel, &c_abs);
             if (bc) {
                 c->h_job->ka = tc_atoms(form, bc_cols(d, form));
                 c->h_job->ksteps = tc_ksteps(form, bc_cols(d, form));
@@ -677,7 +678,7 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
             // centres, whose wider tiles stay on the tensor cores; 1/256 for
             // BF16x3, whose bound adds three products per K step)
             const uint64_t div = !bc ? 4096 : (form == HJ_FORM_TC_BF16X3 ? 256 : 512);
-            uint64_t cap = std::max<uint64_t>(1ull << 20, cand_tc / div);
+            uint64_t cap = std::max<uint64_t>(1ull << 20, cand_tc / div) + band_slack(c->num_sms, bc);
             const uint64_t cap_limit = std::max<uint64_t>(1ull << 27, cand_tc / 64);
             bool done = false, fallback = false;
             for (int grow = 0; grow < 4; ++grow) {
@@ -1124,7 +1125,7 @@ int engine_prepare_job(cudaStream_t st_in, const void *a, const void *b, uint64_
     J.form = P.form;
     J.num_sms = c->num_sms;
     int launches = P.launches;
-    tc_band_constants(P.form, d, P.maxabs, &J.c_rel, &J.c_abs);
+    tc_band_constants(P.form, d, P.maxabs, P.A.fold, &J.c_rel, &J.c_abs);
     const double T_tc = eps * eps * J.op_scale * J.op_scale;
     AllocCtx actx{c, st};
     int sr = split_items_by_precision(P.idx, J.A, J.B, J.c_rel, J.c_abs, 0.5 * T_tc, nullptr, slot_alloc_cb, &actx,

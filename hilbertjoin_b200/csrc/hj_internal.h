@@ -99,6 +99,7 @@ struct SortedSet {
     uint16_t *bf_lo = nullptr;
     const double *center = nullptr;  // per-dim shift of the tensor-core operands (shared by A and B)
     double op_scale = 1.0;       // FP16 form: power of two applied to operands (norms: its square)
+    bool fold = false;           // operand columns d .. d + 2 hold the pieces of |x - center|^2 / 2 (tc_fold)
     float *norms = nullptr;      // FP32(|x - center|^2 in FP64); padding rows hold kPadNorm
     float *tile_maxnorm_a = nullptr;  // per kTcTileA-row tile
     float *tile_maxnorm_b = nullptr;  // per 256-row tile
@@ -308,6 +309,8 @@ void launch_pairs_fp64(const SortedSet &A, const SortedSet &B, bool self, uint64
 // caller regrows), of which *d_band_holes were left unused (the recheck skips
 // them). Band entries are 16 bytes (kBandEntryBytes).
 constexpr size_t kBandEntryBytes = 16;
+// Slots that the kernel's warps may reserve and leave unused.
+uint64_t band_slack(int num_sms, bool bc);
 // One join of a tensor-core launch. A launch runs the work items of one or
 // more jobs (WorkItem.pad = job index) over operand matrices whose rows hold
 // all jobs' sets; rows are global ranks of those matrices.
@@ -325,13 +328,14 @@ struct TcJob {
     uint32_t ksteps;              // MMA K steps of this job (16 columns each; TF32 8): the columns
                                   // holding data, rounded up; zero columns beyond are not multiplied
     uint32_t d;
+    uint32_t fold;                // the norms of the B ranks are in the accumulator (tc_fold)
 };
 // Fills a job for form `form`, dimension d, eps^2 = T, FP16 operand scale
 // op_scale (1 for other forms), largest |coordinate| maxabs. Returns the
 // error-bound constants through c_rel / c_abs (operand units) if non-null.
 void fill_tc_job(TcJob *j, int form, uint32_t d, double T, double op_scale, double maxabs, uint64_t a_row0,
                  uint64_t na_eff, uint64_t b_row0, uint64_t nb_eff, bool self, unsigned long long *count,
-                 const void *rows_a, const void *rows_b, double *c_rel, double *c_abs);
+                 const void *rows_a, const void *rows_b, bool fold, double *c_rel, double *c_abs);
 
 // Launches the tensor-core kernel over `idx` with the job table d_jobs (device).
 // A and B describe the operand matrices (layout pointers, npad_tc rows, kpad,
@@ -344,6 +348,20 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
                    const IndexResult &idx, uint2 *band, uint64_t band_cap, unsigned long long *d_band_total,
                    uint32_t *d_err, int num_sms, cudaStream_t st, std::string *err, const BcConsts *bc = nullptr,
                    unsigned long long *d_band_holes = nullptr);
+// Folded norms (one global centre): when three more columns fit the operand's
+// last 128-byte atom, so that they cost no operand bytes, columns d .. d + 2 of
+// a row hold the pieces of half its squared norm (FP16: at scales 2^15, 2^4,
+// 2^-7, TF32 and BF16: at 1). As a B row they meet the constants that the
+// kernel writes over the same columns of the A tile, and the accumulator is
+// w = a.b - |b|^2 / 2: the columns of a row order by w alone, so the maximum
+// over 32 columns decides exactly whether any of them is near, also where 32
+// consecutive ranks differ widely in norm (many occupied cells). At
+// 200k x 200k x 20, 20 partners per point, the distance kernel took 15.2 ms
+// with the bound min |b|^2 - 2 max a.b, which sent most groups to the slow
+// path, and 7.2 ms with the norms folded and nothing else changed. At d = 64 the columns would take a second atom, and a group's norms are
+// nearly equal where all points share a cell (the headline): not folded. FP16
+// operands are scaled by a further 2^-kBcScaleShift, so that the pieces fit.
+bool tc_fold(int form, uint32_t d);
 // K atoms (128-byte operand column groups) of a form's operand rows of kcols columns.
 uint32_t tc_atoms(int form, uint32_t kcols);
 // MMA K steps that cover kcols columns (16 per kind::f16 instruction, 8 per kind::tf32),
@@ -362,7 +380,7 @@ void set_tc_debug_output(float *dbg);
 // barrier that nothing arrives on, then raises kErrTimeout (0 = off).
 void set_tc_wait_gate(uint64_t ns);
 // Error-bound constant of a tensor-core form for dimension d.
-void tc_band_constants(int form, uint32_t d, double maxabs, double *c_rel, double *c_abs);
+void tc_band_constants(int form, uint32_t d, double maxabs, bool fold, double *c_rel, double *c_abs);
 
 // ---------------------------------------------------------------- batching
 // One job prepared by the engine for a batched tensor-core launch: its sorted

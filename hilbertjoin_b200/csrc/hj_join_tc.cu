@@ -6,16 +6,19 @@
 //     |a - b|^2 = |a|^2 + |b|^2 - 2 a.b      (egojoin.h:182-195, :329-381),
 // and the a.b tile on the 5th-generation tensor cores:
 //
-//   * one persistent CTA per SM, 6 warps, warp-specialised:
+//   * one persistent CTA per SM, 12 warps, warp-specialised:
 //       warp 0   TMA producer: the A tile (128 EGO ranks x K) once per work
 //                item into one of two A buffers, then the B tiles (256 ranks)
 //                one 128-byte K atom (32 KB) at a time into a ring of stages;
-//       warp 1   MMA issuer (one thread): tcgen05.mma, M=128, N=256, operands
-//                from shared memory (128-byte swizzled, K-major), accumulator
-//                in tensor memory, two accumulators in flight (512 columns);
-//       warps 2-9 epilogue: tcgen05.ld of the accumulator rows (TMEM lane
+//       warp 1   MMA issuer (one elected lane): tcgen05.mma, M=128, N=256,
+//                operands from shared memory (128-byte swizzled, K-major),
+//                accumulator in tensor memory, two accumulators (512 columns);
+//       warps 2, 3  near warps: classify the queued rows that may hold near
+//                pairs, 32 at a time (warp 2 instead completes the A tiles of
+//                joins with folded norms);
+//       warps 4-11 epilogue: tcgen05.ld of the accumulator rows (TMEM lane
 //                quadrant = warp % 4, two warps per quadrant on 128 columns
-//                each), dist^2 estimate, classification, count;
+//                each), dist^2 estimate, near rows found and queued;
 //   * TF32: operands rounded to TF32 on the device (round to nearest), one
 //     MMA per K step; BF16X3: a = a_hi + a_lo in BF16, a.b =
 //     a_hi.b_hi + a_lo.b_hi + a_hi.b_lo (three MMAs per K step); FP16: the
@@ -29,10 +32,27 @@
 //     certainly outside, and every other pair (the band) is queued and
 //     re-evaluated by k_recheck with the FP64 pair test. So the count equals
 //     the plain FP64 form's, bit for bit.
-//   * fast path: per row and 32-column half the epilogue takes the minimum of
-//     |b|^2 - 2 v; only if that can still reach eps^2 + bound (rare: neighbours
-//     are a small fraction of the candidates) does the warp classify the half,
-//     branch-free against per-tile bounds, and queue the band pairs.
+//   * fast path: per row and 32-column group the epilogue takes the minimum of
+//     |b|^2 - 2 v (of -2 v where the norms are folded into the accumulator); only
+//     if that can still reach eps^2 + bound (rare: neighbours are a small fraction
+//     of the candidates) is the row queued for the near warps, or, where several
+//     rows of the group are near, the group classified by the warp itself,
+//     branch-free from its registers.
+//
+// What bounds it (one B200, 1.965 GHz, distance kernel alone, before -> after the
+// epilogue took this form): one global centre, 1M x 64 FP16, 32 neighbours: 79.7 ->
+// 70 ms; 200k x 64: 4.25 -> 3.7; 200k x 200k x 20 (folded norms): 15.4 -> 6.6; 30k x
+// 70k x 100: 1.17 -> 0.56; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
+// clustered FP16: 53 -> 38.3; 300k x 32 TF32: 2.9 -> 1.96. At K = 64 a tile's MMAs
+// take 512 clocks and a tile without near rows about 1100: the chain MMA -> commit
+// -> TMEM load -> release -> MMA over two accumulators. Near rows add the rest. An
+// instruction of the epilogue costs its warp four to six clocks and a ready barrier,
+// a vote or a tcgen05 fence 30 to 50, with two epilogue warps per scheduler; so the
+// tile loop is kept short: 64 columns per TMEM load, one vote per load, item data
+// one item ahead, group minima in registers (one load per 32 tiles). Measured and
+// dropped: 32-column loads double-buffered (more votes and waits: +25%), 128
+// columns at once (spills), two issuing warps, each set of four epilogue warps on
+// one accumulator, near rows worked off by the epilogue warps between tiles.
 //
 // Every mbarrier wait is bounded in time (hj_common.cuh); on a timeout the
 // kernel raises kErrTimeout (with the number of the wait that gave up in bits
@@ -54,33 +74,51 @@
 
 namespace hj {
 
-// Epilogue warps: kEpiWarps / 4 per TMEM lane quadrant, each on kEpiCols of the
-// 256 accumulator columns, in two chunks of kChunkCols (one TMEM load each).
+// Epilogue warps: two per TMEM lane quadrant, each on kEpiCols of the 256
+// accumulator columns, read kChunkCols at a time.
 constexpr int kEpiWarps = 8;
-constexpr int kEpiCols = 4 * kTcTileB / kEpiWarps;
-// 8 warps: two 64-column chunks each; 16 warps: one 64-column chunk each
+constexpr int kEpiCols = 128;
 constexpr int kChunkCols = 64;
-constexpr int kChunkGroups = kChunkCols / 32;  // 32-column groups per chunk
-constexpr int kEpiChunks = kEpiCols / kChunkCols;
-constexpr int kEpiVec = kEpiCols / 32;  // norms per lane, group minima per warp
-// Block centring, where tiles in which near pairs are common make up much of
-// the work: the lanes classify their own rows against a 32-column group (the
-// dense path) instead of the warp walking row by row, and band slots are
-// reserved by each epilogue warp in chunks (one atomic per chunk); slots a
-// warp leaves unused are marked with ia = kBandHole. With one global centre
-// (near pairs rare) both measured slower, the row walk with one atomic per
-// band pair stays.
-constexpr uint32_t kBandChunk = 256;
+// Band slots are reserved by each warp in chunks (one atomic, whose latency the warp
+// waits for, per chunk); slots a warp leaves unused are marked with ia = kBandHole.
+// Block centring, where near pairs are common, takes larger chunks.
+constexpr uint32_t kBandChunk = 256, kBandChunkRare = 32;
 constexpr uint32_t kBandHole = 0xffffffffu;
-// 16 epilogue warps (4 per quadrant) were measured slower: at 18 warps the
-// register cap is 96 (spills) and the static shared memory no longer fits next
-// to the 225 KB operand plan.
-static_assert(kEpiWarps == 8, "the shared-memory plan and register budget assume 8 epilogue warps");
-constexpr int kTcThreads = 64 + 32 * kEpiWarps;
+static_assert(kEpiWarps * kEpiCols == 4 * kTcTileB && kEpiCols == 2 * kChunkCols && kChunkCols == 64, "the shared-memory plan and the epilogue assume 8 warps of two chunks");
+// Warpgroup 0 holds the control and near warps, warpgroups 1 and 2 the epilogue. The
+// block launches with 168 registers a thread (64512); warpgroup 0 gives part of its
+// share to the epilogue: 128 x 88 + 256 x 208 = 64512.
+constexpr int kFoldWarp = 2;
+constexpr int kEpiWarp0 = 4;
+constexpr int kTcThreads = 32 * (kEpiWarp0 + kEpiWarps);
+constexpr int kCtlRegs = 88, kEpiRegs = 208;
+static_assert(128 * kCtlRegs + 32 * kEpiWarps * kEpiRegs <= kTcThreads * 168, "register split");
 constexpr uint32_t kAtomBytes = 128;                  // bytes of K per row per swizzle atom
 constexpr uint32_t kAStageBytes = kTcTileA * kAtomBytes;  // 16 KB per A atom
 constexpr uint32_t kBStageBytes = kTcTileB * kAtomBytes;  // 32 KB per B atom
 constexpr uint32_t kTmemCols = 512;
+
+// Near rows are not classified where they are found. A lane whose 32 columns may
+// hold a pair that is not certainly outside copies them, with what classifies
+// them, into its warp's queue in shared memory, and the near warps work the queues
+// off beside the epilogue, up to 32 rows at a time (lane = row). A row's
+// classification takes one to two thousand clocks of latency (the B norms, a slot in
+// the band queue), and one near row in a tile used to hold the accumulator of all
+// eight warps for it; at 1M x 64 and 32 neighbours six tiles in ten have one.
+// An entry: 32 values | |a|^2, thr_in, thr_out, A rank | first B rank, column mask,
+// job, norms folded | 4 unused words (an odd number of 16-byte units, so that lanes
+// reading their rows do not meet in a bank).
+constexpr uint32_t kNearWords = 44;
+constexpr uint32_t kNearCap = 24;    // entries per warp, at most
+// A group with more near rows is classified by the epilogue warp (lane = row): about
+// 1000 clocks however many rows, against the queue's per-row cost. With one centre, 30k x
+// 70k x 100: 0.57 ms at 0, 0.56 at 3, 0.75 at 10; 1M x 64: 78, 70, 70 ms. Block
+// centres, 4M x 28: 40.2 ms at 0, 39.5 at 3, 38.5 at 5 and at 8.
+constexpr uint32_t kNearDenseBc = 6, kNearDenseOne = 3;
+constexpr uint32_t kNearMinCap = 8;  // fewer entries than this are not worth a B stage
+constexpr uint32_t kNearDone = 0x80000000u;  // in a queue's tail: its warp has finished
+
+constexpr uint64_t kIdleLimitNs = 600000000000ull;  // the near warps' longest run: 10 minutes
 
 struct BandEntry {
     uint32_t ia, jb;  // EGO ranks in A and B
@@ -93,6 +131,7 @@ struct TcArgs {
                         // (each job multiplies only its own ksteps)
     uint32_t a_bufs;    // 1 or 2 A buffers
     uint32_t nst;       // B ring stages
+    uint32_t near_cap;  // entries of each epilogue warp's near queue (>= 1)
     const WorkItem *items;
     uint64_t n_items;
     const float *norm_a, *norm_b;   // FP32 |x|^2 per EGO rank (padding: kPadNorm)
@@ -108,6 +147,7 @@ struct TcArgs {
     float *dbg;                     // optional: s_hat for every pair, input order [na][nb] (tests)
     const uint32_t *perm_a, *perm_b;  // EGO rank -> input index (for dbg)
     uint32_t a_xoff;                // first column of the A operand in its rows (block centring: dp)
+    uint32_t fold;                  // some job's norms are folded: the fold warp completes every A tile
     uint64_t gate_ns;               // test hook: > 0 makes the epilogue wait this long on a barrier
                                     // that nothing arrives on, then raise kErrTimeout
     // per-block centring (BC kernels): norm_a is then q of the A rows (norm_b and
@@ -135,6 +175,21 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
+// Register share of a warpgroup (every warp of it executes one of these once).
+template <int R>
+__device__ __forceinline__ void reg_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
+}
+template <int R>
+__device__ __forceinline__ void reg_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+}
+
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
@@ -160,29 +215,40 @@ __device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t adesc, uint6
     }
 }
 
-// 64 consecutive accumulator columns of this thread's TMEM lane (two x32
-// loads, one wait).
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
-    uint32_t r[64];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-            "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-            : "=r"(r[32 * h + 0]), "=r"(r[32 * h + 1]), "=r"(r[32 * h + 2]), "=r"(r[32 * h + 3]),
-              "=r"(r[32 * h + 4]), "=r"(r[32 * h + 5]), "=r"(r[32 * h + 6]), "=r"(r[32 * h + 7]),
-              "=r"(r[32 * h + 8]), "=r"(r[32 * h + 9]), "=r"(r[32 * h + 10]), "=r"(r[32 * h + 11]),
-              "=r"(r[32 * h + 12]), "=r"(r[32 * h + 13]), "=r"(r[32 * h + 14]), "=r"(r[32 * h + 15]),
-              "=r"(r[32 * h + 16]), "=r"(r[32 * h + 17]), "=r"(r[32 * h + 18]), "=r"(r[32 * h + 19]),
-              "=r"(r[32 * h + 20]), "=r"(r[32 * h + 21]), "=r"(r[32 * h + 22]), "=r"(r[32 * h + 23]),
-              "=r"(r[32 * h + 24]), "=r"(r[32 * h + 25]), "=r"(r[32 * h + 26]), "=r"(r[32 * h + 27]),
-              "=r"(r[32 * h + 28]), "=r"(r[32 * h + 29]), "=r"(r[32 * h + 30]), "=r"(r[32 * h + 31])
-            : "r"(taddr + 32 * h));
-    }
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = __uint_as_float(r[i]);
+// 64 consecutive accumulator columns of this thread's TMEM lane: the load is
+// issued here and its registers may be read after tmem_wait on them.
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[64]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, "
+        "%38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, "
+        "%56, %57, %58, %59, %60, %61, %62, %63}, [%64]; "
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]),
+          "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]),
+          "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]),
+          "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31]), "=f"(v[32]),
+          "=f"(v[33]), "=f"(v[34]), "=f"(v[35]), "=f"(v[36]), "=f"(v[37]), "=f"(v[38]), "=f"(v[39]), "=f"(v[40]),
+          "=f"(v[41]), "=f"(v[42]), "=f"(v[43]), "=f"(v[44]), "=f"(v[45]), "=f"(v[46]), "=f"(v[47]), "=f"(v[48]),
+          "=f"(v[49]), "=f"(v[50]), "=f"(v[51]), "=f"(v[52]), "=f"(v[53]), "=f"(v[54]), "=f"(v[55]), "=f"(v[56]),
+          "=f"(v[57]), "=f"(v[58]), "=f"(v[59]), "=f"(v[60]), "=f"(v[61]), "=f"(v[62]), "=f"(v[63])
+        : "r"(taddr)
+        : "memory");
+}
+
+// Waits for the warp's outstanding TMEM loads. The registers are operands, so
+// that no use of them is scheduled before the wait.
+__device__ __forceinline__ void tmem_wait(float (&v)[64]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
+                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]),
+                   "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]),
+                   "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]),
+                   "+f"(v[29]), "+f"(v[30]), "+f"(v[31]), "+f"(v[32]), "+f"(v[33]), "+f"(v[34]), "+f"(v[35]),
+                   "+f"(v[36]), "+f"(v[37]), "+f"(v[38]), "+f"(v[39]), "+f"(v[40]), "+f"(v[41]), "+f"(v[42]),
+                   "+f"(v[43]), "+f"(v[44]), "+f"(v[45]), "+f"(v[46]), "+f"(v[47]), "+f"(v[48]), "+f"(v[49]),
+                   "+f"(v[50]), "+f"(v[51]), "+f"(v[52]), "+f"(v[53]), "+f"(v[54]), "+f"(v[55]), "+f"(v[56]),
+                   "+f"(v[57]), "+f"(v[58]), "+f"(v[59]), "+f"(v[60]), "+f"(v[61]), "+f"(v[62]), "+f"(v[63])::"memory");
 }
 
 // max(a, b, c) in one instruction (three-input max.f32, sm_100).
@@ -190,6 +256,16 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float r;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
+}
+
+// The largest of the 32 values from v: 16 instructions in a tree of depth 4.
+__device__ __forceinline__ float max32(const float *v) {
+    float t[10];
+#pragma unroll
+    for (int i = 0; i < 10; ++i) t[i] = fmax3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
+    const float u0 = fmax3(t[0], t[1], t[2]), u1 = fmax3(t[3], t[4], t[5]);
+    const float u2 = fmax3(t[6], t[7], t[8]), u3 = fmax3(t[9], v[30], v[31]);
+    return fmaxf(fmax3(u0, u1, u2), u3);
 }
 
 // Shared-memory matrix descriptor: K-major operand in 128-byte swizzle atoms
@@ -205,12 +281,79 @@ __device__ __forceinline__ constexpr uint32_t instr_desc() {
     return (1u << 4) | (ab << 7) | (ab << 10) | ((uint32_t)(kTcTileB >> 3) << 17) | ((uint32_t)(kTcTileA >> 4) << 24);
 }
 
+// Whether the phase has completed, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Waits for a phase regardless of the error word, until `deadline`
 // (%globaltimer): the drain of copies and MMAs already issued.
 __device__ __forceinline__ void drain_until(uint64_t *bar, uint32_t parity, uint64_t deadline) {
     while (!mbar_try_wait(bar, parity)) {
         if (globaltimer_ns() > deadline) break;
     }
+}
+
+// A warp's slots in the band queue, taken in chunks (one atomic per chunk; all
+// state warp-uniform).
+struct BandSlots {
+    unsigned long long k0, nb;
+    uint32_t rem;
+    // the slot of the entry of rank r: r < rem ? k0 + r : nb + (r - rem)
+    __device__ unsigned long long at(uint32_t r) const { return r < rem ? k0 + r : nb + (r - rem); }
+};
+struct BandWriter {
+    const TcArgs &p;
+    uint32_t lane, chunk;
+    unsigned long long slot = 0, end = 0;  // the current chunk
+    __device__ BandWriter(const TcArgs &p_, uint32_t lane_, uint32_t chunk_) : p(p_), lane(lane_), chunk(chunk_) {}
+    // c new slots: the rest of the chunk first, then a new one
+    __device__ BandSlots reserve(uint32_t c) {
+        BandSlots b{slot, 0, (uint32_t)(end - slot)};
+        if (c <= b.rem) {
+            slot += c;
+            return b;
+        }
+        const uint32_t need = c - b.rem, size = need > chunk ? need : chunk;
+        unsigned long long nb = 0;
+        if (lane == 0) nb = atomicAdd(p.band_total, (unsigned long long)size);
+        b.nb = __shfl_sync(0xffffffffu, nb, 0);
+        slot = b.nb + need;
+        end = b.nb + size;
+        return b;
+    }
+    __device__ void store(unsigned long long k, uint32_t ia, uint32_t jb, float s_hat, uint32_t job) const {
+        if (k >= p.band_cap) return;
+        BandEntry e;
+        e.ia = ia;
+        e.jb = jb;
+        e.s_hat = s_hat;
+        e.pad = job;
+        p.band[k] = e;
+    }
+    // the unused rest of the chunk: marked for the recheck to skip
+    __device__ void finish() {
+        for (unsigned long long k = slot + lane; k < end; k += 32) store(k, kBandHole, 0, 0.f, 0);
+        if (lane == 0 && end > slot && p.band_holes) atomicAdd(p.band_holes, end - slot);
+        slot = end;
+    }
+};
+
+__device__ __forceinline__ uint32_t lds_acquire(const uint32_t *a) {
+    uint32_t v;
+    asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"(smem_u32(a)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_release(uint32_t *a, uint32_t v) {
+    asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(a)), "r"(v) : "memory");
 }
 
 // ---------------------------------------------------------------- the kernel
@@ -227,10 +370,11 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t a_buf_bytes = a_atoms * kAStageBytes;
 
     extern __shared__ unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bar_afull[2], bar_aempty[2], bar_accfull[2], bar_accempty[2], bar_drain, bar_gate;
+    __shared__ __align__(8) uint64_t bar_afull[2], bar_aempty[2], bar_aready[2], bar_accfull[2], bar_accempty[2];
+    __shared__ __align__(8) uint64_t bar_drain, bar_gate;
     __shared__ __align__(8) uint64_t bar_bfull[8], bar_bempty[8];
     __shared__ uint32_t tmem_base_sh;
-    __shared__ __align__(16) float epi_row[kEpiWarps][32];
+    __shared__ uint32_t near_tail[kEpiWarps], near_head[kEpiWarps];  // entries queued (| kNearDone), worked off
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t a_base = smem_base;
@@ -242,6 +386,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         for (int i = 0; i < 2; ++i) {
             mbar_init(&bar_afull[i], 1);
             mbar_init(&bar_aempty[i], 1);
+            mbar_init(&bar_aready[i], 1);
             mbar_init(&bar_accfull[i], 1);
             mbar_init(&bar_accempty[i], kEpiWarps);
         }
@@ -250,6 +395,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             mbar_init(&bar_bempty[i], 1);
         }
         mbar_init(&bar_drain, 1);
+        for (int i = 0; i < kEpiWarps; ++i) near_tail[i] = near_head[i] = 0;
         mbar_init(&bar_gate, 1);
         fence_barrier_init();
     }
@@ -268,18 +414,27 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_sh;
+    const uint64_t stride = gridDim.x;
+    float *near_base = reinterpret_cast<float *>(smem_raw + (b_base + p.nst * kBStageBytes - smem_u32(smem_raw)));
+    const uint32_t near_ring = p.near_cap * kNearWords;  // floats per epilogue warp
+    // item `i` of the list, an empty one past its end
+    auto item_at = [&](uint64_t i) { return i < p.n_items ? p.items[i] : WorkItem{0, 0, 0, 0}; };
 
     if (warp == 0) {
         // ------------------------------------------------ TMA producer
+        reg_dec<kCtlRegs>();
         if (lane == 0) {
             uint32_t a_cnt = 0, b_cnt = 0;
+            uint32_t abuf = 0, aph = 1;  // A buffer of the next item, parity of its last release
+            uint32_t s = 0, sph = 1;     // B stage of the next atom, parity of its last release
             bool ok = true;
-            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += gridDim.x) {
-                const WorkItem w = p.items[it];
+            WorkItem w = item_at(blockIdx.x);
+            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
+                const WorkItem wn = item_at(it + stride);
                 const uint32_t ka = p.jobs[w.pad].ka;  // this job's K atoms (<= p.ka)
                 const uint32_t ja_atoms = kBf ? 2 * ka : ka;
-                const uint32_t abuf = a_cnt % p.a_bufs, au = a_cnt / p.a_bufs;
-                if (au >= 1 && !mbar_wait(&bar_aempty[abuf], (au - 1) & 1u, err, 1)) break;
+                // parity 1 of a barrier that never completed a phase counts as passed: the first uses do not wait
+                if (!mbar_wait(&bar_aempty[abuf], aph, err, 1)) break;
                 mbar_arrive_expect_tx(&bar_afull[abuf], ja_atoms * kAStageBytes);
                 const uint32_t adst = a_base + abuf * a_buf_bytes;
                 for (uint32_t q = 0; q < ja_atoms; ++q) {
@@ -289,10 +444,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 (int32_t)(kq * kAtomElems + p.a_xoff), (int32_t)(w.a * kTcTileA), &bar_afull[abuf]);
                 }
                 ++a_cnt;
+                if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
                 for (uint32_t bt = w.b0; ok && bt < w.b1; ++bt) {
                     for (uint32_t q = 0; q < ja_atoms; ++q) {
-                        const uint32_t s = b_cnt % p.nst, u = b_cnt / p.nst;
-                        if (u >= 1 && !mbar_wait(&bar_bempty[s], (u - 1) & 1u, err, 2)) {
+                        if (!mbar_wait(&bar_bempty[s], sph, err, 2)) {
                             ok = false;
                             break;
                         }
@@ -302,8 +457,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         tma_load_2d(smem_raw + (b_base + s * kBStageBytes - smem_u32(smem_raw)), lo ? &tm_b2 : &tm_b,
                                     (int32_t)(kq * kAtomElems), (int32_t)(bt * kTcTileB), &bar_bfull[s]);
                         ++b_cnt;
+                        if (++s == p.nst) s = 0, sph ^= 1u;
                     }
                 }
+                w = wn;
             }
             // Drain: on the normal path every copy has been consumed; after an
             // error (the loops stop at the first failed wait) every copy issued
@@ -322,52 +479,68 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
     } else if (warp == 1) {
         // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        // An MMA is accepted about when the one before it ends (128 clocks at N =
+        // 256), so what the thread does between two MMAs beyond that adds to the
+        // tile: the next stage and the next accumulator are looked at before the
+        // current stage's MMAs are issued, descriptors advance by additions, and the
+        // whole warp runs the loop with one elected lane issuing (a lane running it
+        // alone took a third longer per tile).
+        reg_dec<kCtlRegs>();
+        {
+            const bool el = elect_one();
             constexpr uint32_t idesc = instr_desc<FORM>();
-            uint32_t a_cnt = 0, b_cnt = 0, t_cnt = 0;
+            uint64_t *bar_a = p.fold ? bar_aready : bar_afull;
+            uint32_t abuf = 0, aph = 0;      // A buffer of the item, its phase
+            uint32_t s = 0, sph = 0;         // B stage of the next atom, its phase
+            uint32_t acc = 0, accph = 1;     // accumulator of the next tile, parity of its last release
+            bool acc_ready = true, b_ready = false;
             bool issued_any = false, ok = true;
-            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += gridDim.x) {
-                const WorkItem w = p.items[it];
+            const uint64_t b_desc0 = sw128_desc(b_base);
+            WorkItem w = item_at(blockIdx.x);
+            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
+                const WorkItem wn = item_at(it + stride);
                 const uint32_t ka = p.jobs[w.pad].ka, ksteps = p.jobs[w.pad].ksteps;
                 const uint32_t jb_atoms = kBf ? 2 * ka : ka;
-                const uint32_t abuf = a_cnt % p.a_bufs, au = a_cnt / p.a_bufs;
-                if (!mbar_wait(&bar_afull[abuf], au & 1u, err, 3)) break;
+                if (!mbar_wait(&bar_a[abuf], aph, err, 3)) break;
                 tc_fence_after();
-                const uint32_t abase = a_base + abuf * a_buf_bytes;
-                for (uint32_t bt = w.b0; ok && bt < w.b1; ++bt) {
-                    const uint32_t acc = t_cnt & 1u, tu = t_cnt >> 1;
-                    if (tu >= 1 && !mbar_wait(&bar_accempty[acc], (tu - 1) & 1u, err, 4)) {
+                const uint64_t a_desc0 = sw128_desc(a_base + abuf * a_buf_bytes);
+                for (uint32_t n = w.b1 - w.b0; ok && n > 0; --n) {
+                    if (!acc_ready && !mbar_wait(&bar_accempty[acc], accph, err, 4)) {
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t dcol = tmem + acc * kTcTileB;
+                    uint64_t *bar_full = &bar_accfull[acc];
+                    acc ^= 1u;
+                    accph ^= acc ^ 1u;
                     uint32_t accumulate = 0;
                     for (uint32_t q = 0; q < jb_atoms; ++q) {
-                        const uint32_t s = b_cnt % p.nst;
-                        if (!mbar_wait(&bar_bfull[s], (b_cnt / p.nst) & 1u, err, 5)) {
+                        if (!b_ready && !mbar_wait(&bar_bfull[s], sph, err, 5)) {
                             ok = false;
                             break;
                         }
-                        tc_fence_after();
-                        const uint32_t bsm = b_base + s * kBStageBytes;
+                        const uint64_t bdesc = b_desc0 + s * (kBStageBytes / 16);
+                        uint64_t *bar_release = &bar_bempty[s];
+                        if (++s == p.nst) s = 0, sph ^= 1u;
+                        b_ready = mbar_test(&bar_bfull[s], sph);
+                        if (q + 1 == jb_atoms) acc_ready = mbar_test(&bar_accempty[acc], accph);
+                        // a K step advances both descriptors by 32 bytes (2 in their 16-byte units)
                         if constexpr (!kBf) {
-                            const uint32_t asm_ = abase + q * kAStageBytes;
+                            const uint64_t adesc = a_desc0 + q * (kAStageBytes / 16);
                             // 4 K steps per atom, fewer in the last (zero columns not multiplied)
                             const uint32_t kk_end = ksteps - 4 * q < 4 ? ksteps - 4 * q : 4;
                             if (kk_end == 4) {
 #pragma unroll
                                 for (uint32_t kk = 0; kk < 4; ++kk) {
-                                    mma_issue<FORM>(dcol, sw128_desc(asm_ + kk * 32), sw128_desc(bsm + kk * 32), idesc,
-                                                    accumulate);
+                                    if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                     accumulate = 1;
                                 }
                             } else {
 #pragma unroll
                                 for (uint32_t kk = 0; kk < 3; ++kk) {
                                     if (kk < kk_end) {
-                                        mma_issue<FORM>(dcol, sw128_desc(asm_ + kk * 32), sw128_desc(bsm + kk * 32),
-                                                        idesc, accumulate);
+                                        if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
                                     }
                                 }
@@ -375,51 +548,199 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                         } else {
                             const uint32_t kq = q >> 1;
                             const uint32_t kk_end = ksteps - 4 * kq < 4 ? ksteps - 4 * kq : 4;
-                            const uint32_t a_hi = abase + kq * kAStageBytes;
-                            const uint32_t a_lo = abase + (ka + kq) * kAStageBytes;
+                            const uint64_t a_hi = a_desc0 + kq * (kAStageBytes / 16);
+                            const uint64_t a_lo = a_desc0 + (ka + kq) * (kAStageBytes / 16);
                             if ((q & 1u) == 0) {  // B_hi atom: A_hi.B_hi + A_lo.B_hi
 #pragma unroll
                                 for (uint32_t kk = 0; kk < 4; ++kk) {
                                     if (kk >= kk_end) break;
-                                    mma_issue<FORM>(dcol, sw128_desc(a_hi + kk * 32), sw128_desc(bsm + kk * 32),
-                                                    idesc, accumulate);
+                                    if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                     accumulate = 1;
-                                    mma_issue<FORM>(dcol, sw128_desc(a_lo + kk * 32), sw128_desc(bsm + kk * 32),
-                                                    idesc, 1);
+                                    if (el) mma_issue<FORM>(dcol, a_lo + 2 * kk, bdesc + 2 * kk, idesc, 1);
                                 }
                             } else {  // B_lo atom: A_hi.B_lo
 #pragma unroll
                                 for (uint32_t kk = 0; kk < 4; ++kk)
-                                    if (kk < kk_end)
-                                        mma_issue<FORM>(dcol, sw128_desc(a_hi + kk * 32), sw128_desc(bsm + kk * 32),
-                                                        idesc, 1);
+                                    if (kk < kk_end) if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, 1);
                             }
                         }
-                        mma_commit(&bar_bempty[s]);  // stage free once these MMAs have read it
-                        ++b_cnt;
+                        if (el) mma_commit(bar_release);  // stage free once these MMAs have read it
                         issued_any = true;
                     }
                     if (!ok) break;
-                    mma_commit(&bar_accfull[acc]);
-                    ++t_cnt;
+                    if (el) mma_commit(bar_full);
                 }
-                mma_commit(&bar_aempty[abuf]);
-                ++a_cnt;
+                if (el) mma_commit(&bar_aempty[abuf]);
+                if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
+                w = wn;
             }
             // all MMAs complete before the tensor memory is released
             if (issued_any) {
-                mma_commit(&bar_drain);
+                if (el) mma_commit(&bar_drain);
                 drain_until(&bar_drain, 0, globaltimer_ns() + kWaitLimitNs);
             }
         }
+    } else if (warp == kFoldWarp && p.fold) {
+        // ------------------------------------------------ A side of folded norms
+        reg_dec<kCtlRegs>();
+        // A folded row holds the pieces of |x|^2 / 2 in its columns d .. d + 2.
+        // As a B operand they meet the A side's constants; here those replace
+        // the pieces of the A tile that has landed (once per item, 128 rows of
+        // 3 columns), before the MMA warp is told that the tile is ready.
+        uint32_t abuf = 0, aph = 0;
+        for (uint64_t it = blockIdx.x; it < p.n_items; it += stride) {
+            const TcJob &J = p.jobs[p.items[it].pad];
+            const bool fold = J.fold != 0;
+            const uint32_t d = J.d, ka = J.ka;
+            const bool landed = mbar_wait(&bar_afull[abuf], aph, err, 7);
+            if (!__all_sync(0xffffffffu, landed)) break;
+            if (fold) {
+                const uint32_t abase = a_base + abuf * a_buf_bytes;
+                for (uint32_t r = lane; r < (uint32_t)kTcTileA; r += 32) {
+#pragma unroll
+                    for (uint32_t m = 0; m < 3; ++m) {
+                        const uint32_t col = d + m, q = col / kAtomElems;
+                        const uint32_t byte = (col % kAtomElems) * (kAtomBytes / kAtomElems);
+                        const uint32_t off = q * kAStageBytes + r * kAtomBytes + (((byte >> 4) ^ (r & 7u)) << 4) +
+                                             (byte & 15u);
+                        if constexpr (FORM == HJ_FORM_TC_TF32) {
+                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(abase + off), "r"(0xBF800000u) : "memory");
+                        } else if constexpr (kBf) {  // -1 and 0
+                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"((uint16_t)0xBF80) : "memory");
+                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + ka * kAStageBytes + off),
+                                         "h"((uint16_t)0)
+                                         : "memory");
+                        } else {  // -2^15, -2^4, -2^-7
+                            const uint16_t c = m == 0 ? 0xF800 : (m == 1 ? 0xCC00 : 0xA000);
+                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"(c) : "memory");
+                        }
+                    }
+                }
+                fence_proxy_async();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar_aready[abuf]);
+            if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
+        }
+    } else if (warp < kEpiWarp0) {
+        // ------------------------------------------------ near warps
+        // Warp 3, and warp 2 where no job folds its norms: each works off the queues
+        // of its share of the epilogue warps. Lane r < kEpiWarps keeps queue r.
+        reg_dec<kCtlRegs>();
+        const bool mine = lane < (uint32_t)kEpiWarps && (p.fold || (lane & 1u) == (warp & 1u));
+        uint32_t head = 0, slot = 0;  // entries worked off, and the next one's slot
+        uint32_t job = 0xffffffffu;
+        unsigned long long cnt = 0;
+        BandWriter band(p, lane, BC ? kBandChunk : kBandChunkRare);
+        auto flush = [&]() {
+            const unsigned long long wc = warp_sum_u64(cnt);
+            if (lane == 0 && wc) atomicAdd(p.jobs[job].count, wc);
+            cnt = 0;
+        };
+        // every epilogue warp ends its queue (its own waits are bounded), so this
+        // loop ends; the time limit is a second line only
+        const uint64_t t0 = globaltimer_ns();
+        for (uint32_t idle = 0;;) {
+            const uint32_t tail = mine ? lds_acquire(&near_tail[lane]) : kNearDone;
+            __syncwarp();  // the acquiring lanes' view becomes the warp's
+            const uint32_t avail = mine ? (tail - head) & ~kNearDone : 0u;
+            if (!__any_sync(0xffffffffu, avail != 0)) {
+                if (__all_sync(0xffffffffu, (tail & kNearDone) != 0)) break;
+                if ((++idle & 1023u) == 0 && globaltimer_ns() - t0 > kIdleLimitNs) {
+                    atomicOr((uint32_t *)err, kErrTimeout | (10u << 8));
+                    break;
+                }
+                __nanosleep(64);
+                continue;
+            }
+            // lane i takes row i of the queues in order
+            uint32_t my_q = 0, my_i = 0, taken = 0, took = 0;
+#pragma unroll
+            for (uint32_t r = 0; r < (uint32_t)kEpiWarps; ++r) {
+                const uint32_t have = __shfl_sync(0xffffffffu, avail, r), n = have < 32 - taken ? have : 32 - taken;
+                if (lane >= taken && lane < taken + n) my_q = r, my_i = lane - taken;
+                if (lane == r) took = n;
+                taken += n;
+            }
+            const bool row = lane < taken;
+            uint32_t at = __shfl_sync(0xffffffffu, slot, my_q) + my_i;
+            if (at >= p.near_cap) at -= p.near_cap;
+            const float *ent = near_base + my_q * near_ring + at * kNearWords;
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint4 u = make_uint4(0u, 0u, 0u, 0u);
+            uint32_t g_in = 0, bbits = 0;
+            if (row) {
+                q = *reinterpret_cast<const float4 *>(ent + 32);
+                u = *reinterpret_cast<const uint4 *>(ent + 36);
+                const float4 *nrm = reinterpret_cast<const float4 *>(BC || u.w ? nullptr : p.norm_b + u.x);
+                float4 nb[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) nb[k] = nrm ? __ldg(nrm + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                uint32_t g_out = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float4 v = *reinterpret_cast<const float4 *>(ent + 4 * k);
+                    const float t[4] = {fmaf(-2.0f, v.x, nb[k].x), fmaf(-2.0f, v.y, nb[k].y),
+                                        fmaf(-2.0f, v.z, nb[k].z), fmaf(-2.0f, v.w, nb[k].w)};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        g_in |= t[j] <= q.y ? 1u << (4 * k + j) : 0u;
+                        g_out |= t[j] <= q.z ? 1u << (4 * k + j) : 0u;
+                    }
+                }
+                g_in &= u.y;
+                bbits = g_out & u.y & ~g_in;
+            }
+            // counts, into the job that every row of the batch belongs to as a rule
+            const uint32_t j0 = __shfl_sync(0xffffffffu, u.z, 0);
+            if (__all_sync(0xffffffffu, !row || u.z == j0)) {
+                if (j0 != job) {
+                    if (job != 0xffffffffu) flush();
+                    job = j0;
+                }
+                cnt += __popc(g_in);
+            } else if (g_in) {
+                atomicAdd(p.jobs[u.z].count, (unsigned long long)__popc(g_in));
+            }
+            if (__any_sync(0xffffffffu, bbits != 0)) {
+                const uint32_t nbits = __popc(bbits);
+                uint32_t incl = nbits;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= (uint32_t)o) incl += y;
+                }
+                const BandSlots sl = band.reserve(__shfl_sync(0xffffffffu, incl, 31));
+                uint32_t rank = incl - nbits;
+                while (bbits) {
+                    const int j = __ffs(bbits) - 1;
+                    bbits &= bbits - 1;
+                    const float t = fmaf(-2.0f, ent[j], BC || u.w ? 0.f : __ldg(p.norm_b + u.x + j));
+                    band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[u.z].s_unscale, u.z);
+                }
+            }
+            __syncwarp();  // the rows have been read
+            if (took) {
+                head = (head + took) & ~kNearDone;
+                slot = slot + took < p.near_cap ? slot + took : slot + took - p.near_cap;
+                sts_release(&near_head[lane], head);
+            }
+        }
+        if (job != 0xffffffffu) flush();
+        band.finish();
     } else {
         // ------------------------------------------------ epilogue
+        reg_inc<kEpiRegs>();
         const uint32_t quad = warp & 3u;
-        const uint32_t half = (warp - 2) >> 2;  // columns [kEpiCols half, kEpiCols (half + 1))
+        const uint32_t half = (warp - kEpiWarp0) >> 2;  // columns [kEpiCols half, kEpiCols (half + 1))
         const uint32_t lane_base = (quad * 32u) << 16;
-        float *srow = epi_row[warp - 2];
+        // this warp's near queue: entries queued, the next one's slot, and the entries
+        // worked off when last looked at (warp-uniform)
+        const uint32_t ew = warp - kEpiWarp0;
+        float *near = near_base + ew * near_ring;
+        uint32_t n_tail = 0, n_slot = 0, n_head = 0;
         unsigned long long cnt = 0;
-        uint32_t t_cnt = 0;
+        uint32_t acc = 0, accph = 0;
         bool run = true;
         if (p.gate_ns) {  // test hook: a wait that nothing ends
             const uint64_t t0 = globaltimer_ns();
@@ -435,109 +756,93 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // and the bound rounded up; the FP32 rounding of the epilogue itself is
         // part of c_rel. A pair is inside if s + tau <= T_lo, outside if
         // s - tau > T_hi, and in the band otherwise.
-        // Walk over (item, B tile). Per item: this lane's row (A rank), its norm
-        // and the classification thresholds, taken against the largest B-tile
-        // norm of the item (a band at least as wide as any tile's: still
-        // exact). Per tile only the group minima are needed on the fast path;
-        // they are loaded one tile ahead so that their latency overlaps the
-        // current tile. B norms and column bounds are read on the slow path.
-        const uint64_t stride = gridDim.x;
-        uint64_t it = run ? blockIdx.x : p.n_items;
-        WorkItem w = it < p.n_items ? p.items[it] : WorkItem{0, 0, 0, 0};
-        WorkItem wn = it + stride < p.n_items ? p.items[it + stride] : WorkItem{0, 0, 0, 0};
-        uint32_t bt = w.b0;
+        // Per item: this lane's row (A rank), its norm and the classification
+        // thresholds, taken against the largest B-tile norm of the item (a band at
+        // least as wide as any tile's: still exact). The next item's rows and the
+        // item after it are loaded one item ahead, so that a change of item waits
+        // for no memory. Per tile only the group minima are needed on the fast
+        // path (none when the norms are folded); they are loaded one tile ahead. B
+        // norms and column bounds are read on the slow path.
+        WorkItem w = run ? item_at(blockIdx.x) : WorkItem{0, 0, 0, 0};
+        WorkItem wn = item_at(blockIdx.x + stride), wnn = item_at(blockIdx.x + 2 * stride);
         // per-block centring: the row's p, |h| and |p|, its block's |c| and centre
         // coordinates (lane, lane + 32), the job's eps^2 bounds; per tile the B
         // block's summary and centre, prefetched one tile ahead with the minima
         float p_row = 0.f, xa = 0.f, pa = 0.f, cna = 0.f, t_lo = 0.f, t_hi = 0.f;
         float ca[2] = {0.f, 0.f}, pf_cb[2] = {0.f, 0.f};
         float4 pf_blk = make_float4(0.f, 0.f, 0.f, 0.f);
-        float pf_gmin[kEpiVec];
-        auto prefetch = [&](uint32_t b) {
-            const uint64_t g = (uint64_t)b * kTcTileB + half * kEpiCols;
-            if constexpr (!BC) {
-                const float4 m = __ldg(reinterpret_cast<const float4 *>(p.gmin_b + g / 32));
-                pf_gmin[0] = m.x, pf_gmin[1] = m.y, pf_gmin[2] = m.z, pf_gmin[3] = m.w;
-            } else {
-                const uint64_t blkb = g / kBcBlock;
+        bool fold = false;  // the current item's column norms are in the accumulator
+        // block centring: the B block of the kEpiCols columns from rank g
+        auto prefetch = [&](uint32_t g) {
+            if constexpr (BC) {
+                const uint32_t blkb = g / kBcBlock;
                 pf_blk = __ldg(p.blk_b + blkb);
                 pf_cb[0] = __ldg(p.cent_b + blkb * kBcCentStride + lane);
                 pf_cb[1] = __ldg(p.cent_b + blkb * kBcCentStride + 32 + lane);
             }
         };
-#pragma unroll
-        for (int q = 0; q < kEpiVec; ++q) pf_gmin[q] = 0.f;
-        if (it < p.n_items) prefetch(bt);
+        // one centre: the group minima of the warp's columns in tile b + lane (a load
+        // per 32 tiles; a tile's four are read from its lane)
+        auto load_gmin = [&](uint32_t b, uint32_t b1) {
+            return b + lane < b1
+                       ? __ldg(reinterpret_cast<const float4 *>(p.gmin_b + (b + lane) * (kTcTileB / 32) + half * (kEpiCols / 32)))
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        // an item's row data, loaded one item ahead (norm arrays cover the padded ranks)
+        struct Rows {
+            float n, x, c0, c1, cn;
+            float4 gmin;
+        };
+        auto load_rows = [&](const WorkItem &ww) {
+            Rows r;
+            const uint64_t g = (uint64_t)ww.a * kTcTileA + quad * 32 + lane;
+            r.n = __ldg(p.norm_a + g);
+            if constexpr (BC) {
+                r.x = __ldg(p.xn_a + g);
+                const uint64_t blka = (uint64_t)ww.a * kTcTileA / kBcBlock;
+                r.cn = __ldg(&p.blk_a[blka].y);
+                r.c0 = __ldg(p.cent_a + blka * kBcCentStride + lane);
+                r.c1 = __ldg(p.cent_a + blka * kBcCentStride + 32 + lane);
+            } else {
+                // the largest B-tile norm of the item: this lane's share
+                r.x = 0.f;
+                for (uint32_t b = ww.b0 + lane; b < ww.b1; b += 32) r.x = fmaxf(r.x, __ldg(p.tmax_b + b));
+                r.cn = r.c0 = r.c1 = 0.f;
+                r.gmin = load_gmin(ww.b0, ww.b1);
+            }
+            return r;
+        };
         // per-item row state, and the job whose count the warp is accumulating
-        uint64_t gi = 0, b_end = 0;
+        uint32_t gi = 0, b_end = 0;  // ranks are below 2^31
         bool row_ok = false, self = false;
         float na = kPadNorm, thr_out = -3.0e38f, thr_in = -3.0e38f, s_unscale = 1.f;
         uint32_t job = 0xffffffffu;
+        BandWriter band(p, lane, BC ? kBandChunk : kBandChunkRare);
         auto flush = [&]() {
             const unsigned long long wc = warp_sum_u64(cnt);
             if (lane == 0 && wc) atomicAdd(p.jobs[job].count, wc);
             cnt = 0;
         };
-        // the warp's current chunk of band slots [bslot, bend) (warp-uniform);
-        // slot of the entry of rank `rank` among `c` <= 32 new entries
-        unsigned long long bslot = 0, bend = 0;
-        // the unused rest of the warp's chunk: marked for the recheck to skip
-        auto band_holes = [&]() {
-            for (unsigned long long k = bslot + lane; k < bend; k += 32)
-                if (k < p.band_cap) {
-                    BandEntry e;
-                    e.ia = kBandHole;
-                    e.jb = 0;
-                    e.s_hat = 0.f;
-                    e.pad = 0;
-                    p.band[k] = e;
-                }
-            if (lane == 0 && bend > bslot && p.band_holes) atomicAdd(p.band_holes, bend - bslot);
-            bslot = bend;
-        };
-        // c new slots (warp-uniform c): the rest of the warp's chunk first, then a
-        // new chunk of max(kBandChunk, the remainder); the slot of rank r is
-        // r < rem ? k0 + r : nb + (r - rem)
-        struct BandSlots {
-            unsigned long long k0, nb;
-            uint32_t rem;
-            __device__ unsigned long long at(uint32_t r) const { return r < rem ? k0 + r : nb + (r - rem); }
-        };
-        auto band_reserve = [&](uint32_t c) -> BandSlots {
-            BandSlots b{bslot, 0, (uint32_t)(bend - bslot)};
-            if (c <= b.rem) {
-                bslot += c;
-                return b;
-            }
-            const uint32_t need = c - b.rem, size = need > kBandChunk ? need : kBandChunk;
-            unsigned long long nb = 0;
-            if (lane == 0) nb = atomicAdd(p.band_total, (unsigned long long)size);
-            b.nb = __shfl_sync(0xffffffffu, nb, 0);
-            bslot = b.nb + need;
-            bend = b.nb + size;
-            return b;
-        };
-        auto item_rows = [&](const WorkItem &ww) {
+        auto item_rows = [&](const WorkItem &ww, const Rows &r) {
             if (ww.pad != job) {
                 if (job != 0xffffffffu) flush();
                 job = ww.pad;
             }
             const TcJob &J = p.jobs[job];
             const float T_lo = J.T_lo, T_hi = J.T_hi, crel = J.c_rel_f, cabs = J.c_abs_f;
-            b_end = J.b_end;
+            b_end = (uint32_t)J.b_end;
             self = J.self != 0;
             s_unscale = J.s_unscale;
-            gi = (uint64_t)ww.a * kTcTileA + quad * 32 + lane;
+            gi = ww.a * kTcTileA + quad * 32 + lane;
             row_ok = gi >= J.a_row0 && gi < J.a_end;
             if constexpr (BC) {
                 // thresholds per tile (they depend on the B block): see the tile loop
-                p_row = row_ok ? __ldg(p.norm_a + gi) : 0.f;
-                xa = row_ok ? __ldg(p.xn_a + gi) : 0.f;
+                p_row = row_ok ? r.n : 0.f;
+                xa = row_ok ? r.x : 0.f;
                 pa = fabsf(p_row);
-                const uint64_t blka = (uint64_t)ww.a * kTcTileA / kBcBlock;
-                cna = __ldg(&p.blk_a[blka].y);
-                ca[0] = __ldg(p.cent_a + blka * kBcCentStride + lane);
-                ca[1] = __ldg(p.cent_a + blka * kBcCentStride + 32 + lane);
+                cna = r.cn;
+                ca[0] = r.c0;
+                ca[1] = r.c1;
                 t_lo = T_lo;
                 t_hi = T_hi;
                 na = p_row;
@@ -546,9 +851,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 (void)cabs;
                 return;
             }
-            na = row_ok ? __ldg(p.norm_a + gi) : kPadNorm;
-            float tmaxb = 0.f;
-            for (uint32_t b = ww.b0 + lane; b < ww.b1; b += 32) tmaxb = fmaxf(tmaxb, __ldg(p.tmax_b + b));
+            fold = J.fold != 0;
+            na = row_ok ? r.n : kPadNorm;
+            float tmaxb = r.x;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) tmaxb = fmaxf(tmaxb, __shfl_xor_sync(0xffffffffu, tmaxb, o));
             // With tau_max = c_rel (|a|^2 + max |b|^2) + c_abs >= tau of every pair
@@ -556,211 +861,211 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             //   t_j <= thr_in  => s_j + tau <= eps^2  (certainly inside),
             //   t_j >  thr_out => s_j - tau >  eps^2  (certainly outside),
             // anything between is a band pair. Both thresholds carry margins
-            // for their own FP32 rounding (rounded inward / outward).
+            // for their own FP32 rounding (rounded inward / outward). With folded
+            // norms the accumulator holds w_j = v_j - |b_j|^2 / 2 and t_j = -2 w_j.
             const float tau_max = fmaf(crel, na + tmaxb, cabs) * 1.001f;
             const float marg = 8.0f * 5.9604645e-8f * (fabsf(T_hi) + fabsf(na) + tmaxb + tau_max);
             thr_out = (T_hi + tau_max) - na + marg;
             thr_in = (T_lo - tau_max) - na - marg;
             if (!row_ok) thr_out = thr_in = -3.0e38f;
         };
-        if (it < p.n_items) item_rows(w);
-        while (it < p.n_items) {
-            float gmin[kEpiVec];
+        // columns of the 32 from rank gj that the lane's row may count: below
+        // b_end, and above the row's own rank for a self-join
+        auto col_mask = [&](uint32_t gj) -> uint32_t {
+            const int hi = (int)b_end - (int)gj, lo = self ? (int)gi + 1 - (int)gj : 0;
+            const uint32_t mh = hi >= 32 ? 0xffffffffu : (hi <= 0 ? 0u : (1u << hi) - 1u);
+            const uint32_t ml = lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
+            return row_ok ? mh & ml : 0u;
+        };
+        // Band entries of a lane's row: the columns `bbits` of the 32 from rank gj.
+        // Ranks by a warp prefix sum, slots from one warp-wide reservation. The
+        // estimates are not kept here: NaN, which the recheck's error statistic skips.
+        auto put_band_bits = [&](uint32_t bbits, uint32_t gj) {
+            if (!__any_sync(0xffffffffu, bbits != 0)) return;
+            const uint32_t nbits = __popc(bbits);
+            uint32_t incl = nbits;
 #pragma unroll
-            for (int q = 0; q < kEpiVec; ++q) gmin[q] = pf_gmin[q];
-            if constexpr (BC) {
-                // this tile's B block: D = |c_A - c_B|^2 (FP32, lanes over the
-                // dims), the band half-width of the lane's row against the block,
-                // and the thresholds on t = -2 w (s = q_row + D + t; |w| <= S)
-                float D = 0.f;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            const BandSlots sl = band.reserve(__shfl_sync(0xffffffffu, incl, 31));
+            uint32_t rank = incl - nbits;
+            while (bbits) {
+                const int j = __ffs(bbits) - 1;
+                bbits &= bbits - 1;
+                band.store(sl.at(rank++), gi, gj + j, __int_as_float(0x7fc00000), job);
+            }
+        };
+        // Groups of 32 columns in which many rows are near: every lane classifies its
+        // own row from its registers.
+        auto dense_rows = [&](const float *v, bool need, uint32_t gj) {
+            const uint32_t colmask = need ? col_mask(gj) : 0u;
+            uint32_t g_in = 0, g_out = 0;
+            if (BC || fold) {
+                // t = -2 w, so t <= thr  <=>  w >= -thr / 2 (exact scaling)
+                const float w_in = -0.5f * thr_in, w_out = -0.5f * thr_out;
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    const float df = ca[m] - pf_cb[m];
-                    D = fmaf(df, df, D);
+                for (int j = 0; j < 32; ++j) {
+                    g_in |= v[j] >= w_in ? (1u << j) : 0u;
+                    g_out |= v[j] >= w_out ? (1u << j) : 0u;
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) D += __shfl_xor_sync(0xffffffffu, D, o);
-                float S;
-                const float tau = bc_tau(xa, cna, pa, pf_blk.x, pf_blk.y, pf_blk.z, D, p.bc, &S);
-                const float marg = 8.0f * 5.9604645e-8f * (fabsf(t_hi) + pa + pf_blk.z + D + tau + 2.0f * S);
-                na = p_row + D;
-                thr_out = row_ok ? (t_hi + tau) - p_row - D + marg : -3.0e38f;
-                thr_in = row_ok ? (t_lo - tau) - p_row - D - marg : -3.0e38f;
-            }
-            const uint32_t cur_bt = bt;
-            // the item's rows stay for its last tile; the next item's are set after it
-            const bool last_tile = bt + 1 >= w.b1;
-            if (!last_tile) {
-                ++bt;
             } else {
-                it += stride;
-                w = wn;
-                bt = w.b0;
-                wn = it + stride < p.n_items ? p.items[it + stride] : WorkItem{0, 0, 0, 0};
-            }
-            if (it < p.n_items) prefetch(bt);
-            {
-                const uint32_t acc = t_cnt & 1u;
-                const uint64_t gj0 = (uint64_t)cur_bt * kTcTileB + half * kEpiCols;
-                if (!mbar_wait(&bar_accfull[acc], (t_cnt >> 1) & 1u, err, 6)) break;
-                tc_fence_after();
+                const float4 *nrm = reinterpret_cast<const float4 *>(p.norm_b + gj);
 #pragma unroll
-                for (uint32_t c = 0; c < kEpiChunks; ++c) {
+                for (int k = 0; k < 8; ++k) {
+                    const float4 nb = __ldg(nrm + k);
+                    const float t[4] = {fmaf(-2.0f, v[4 * k], nb.x), fmaf(-2.0f, v[4 * k + 1], nb.y),
+                                        fmaf(-2.0f, v[4 * k + 2], nb.z), fmaf(-2.0f, v[4 * k + 3], nb.w)};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        g_in |= t[j] <= thr_in ? (1u << (4 * k + j)) : 0u;
+                        g_out |= t[j] <= thr_out ? (1u << (4 * k + j)) : 0u;
+                    }
+                }
+            }
+            g_in &= colmask;
+            cnt += __popc(g_in);
+            put_band_bits(g_out & colmask & ~g_in, gj);
+        };
+        // A group's near rows (bits of `rows`) into the near queue; waits for room
+        auto queue_rows = [&](const float *v, uint32_t rows, uint32_t gj) {
+            while (rows) {
+                uint32_t room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
+                if (room == 0) {
+                    const uint64_t t0 = globaltimer_ns();
+                    for (uint32_t i = 1; room == 0; ++i) {
+                        n_head = lds_acquire(&near_head[ew]);
+                        room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
+                        if ((i & 255u) == 0 && (*err != 0 || globaltimer_ns() - t0 > kWaitLimitNs)) {
+                            if (lane == 0 && *err == 0) atomicOr((uint32_t *)err, kErrTimeout | (8u << 8));
+                            break;
+                        }
+                    }
+                    if (!__all_sync(0xffffffffu, room != 0)) return;  // the error word is set: the count is void
+                    n_head = __shfl_sync(0xffffffffu, n_head, 0);
+                    room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
+                }
+                const uint32_t k = __popc(rows), rank = __popc(rows & ((1u << lane) - 1u));
+                const uint32_t take = k < room ? k : room;
+                const bool put = (rows >> lane) & 1u && rank < take;
+                if (put) {
+                    const uint32_t at = n_slot + rank < p.near_cap ? n_slot + rank : n_slot + rank - p.near_cap;
+                    float *ent = near + at * kNearWords;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        reinterpret_cast<float4 *>(ent)[q] =
+                            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    reinterpret_cast<float4 *>(ent)[8] = make_float4(na, thr_in, thr_out, __uint_as_float(gi));
+                    reinterpret_cast<uint4 *>(ent)[9] = make_uint4(gj, col_mask(gj), job, BC || fold ? 1u : 0u);
+                }
+                n_slot = n_slot + take < p.near_cap ? n_slot + take : n_slot + take - p.near_cap;
+                n_tail = (n_tail + take) & ~kNearDone;
+                rows &= ~__ballot_sync(0xffffffffu, put);
+                __syncwarp();
+                if (lane == 0) sts_release(&near_tail[ew], n_tail);
+            }
+        };
+        Rows rn{};
+        if (w.b0 < w.b1) {
+            rn = load_rows(w);
+            prefetch(w.b0 * kTcTileB + half * kEpiCols);
+        }
+        for (uint64_t it = blockIdx.x; run && it < p.n_items; it += stride) {
+            item_rows(w, rn);
+            float4 gmin32 = rn.gmin;
+            const bool more = it + stride < p.n_items;
+            if (more) rn = load_rows(wn);
+            // testing hook: every pair is estimated
+            float thr_fast = p.dbg != nullptr && row_ok ? 3.0e38f : thr_out;
+            uint32_t gj = w.b0 * kTcTileB + half * kEpiCols;
+            const uint32_t gj_end = w.b1 * kTcTileB;
+            // after the item's last tile, the next item's first (prefetch)
+            const uint32_t gj_next = more ? wn.b0 * kTcTileB + half * kEpiCols : gj;
+            for (; gj < gj_end; gj += kTcTileB) {
+                if constexpr (BC) {
+                    // the half's B block: D = |c_A - c_B|^2 (FP32, lanes over the
+                    // dims), the band half-width of the lane's row against the block,
+                    // and the thresholds on t = -2 w (s = q_row + D + t; |w| <= S)
+                    float D = 0.f;
+#pragma unroll
+                    for (int m = 0; m < 2; ++m) {
+                        const float df = ca[m] - pf_cb[m];
+                        D = fmaf(df, df, D);
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) D += __shfl_xor_sync(0xffffffffu, D, o);
+                    float S;
+                    const float tau = bc_tau(xa, cna, pa, pf_blk.x, pf_blk.y, pf_blk.z, D, p.bc, &S);
+                    const float marg = 8.0f * 5.9604645e-8f * (fabsf(t_hi) + pa + pf_blk.z + D + tau + 2.0f * S);
+                    na = p_row + D;
+                    thr_out = row_ok ? (t_hi + tau) - p_row - D + marg : -3.0e38f;
+                    thr_in = row_ok ? (t_lo - tau) - p_row - D - marg : -3.0e38f;
+                    thr_fast = p.dbg != nullptr && row_ok ? 3.0e38f : thr_out;
+                    prefetch(gj + kTcTileB < gj_end ? gj + kTcTileB : gj_next);
+                }
+                float gmin[4] = {0.f, 0.f, 0.f, 0.f};
+                if (!BC && !fold) {
+                    const uint32_t k = (gj / kTcTileB - w.b0) & 31u;
+                    if (k == 0 && gj / kTcTileB != w.b0) gmin32 = load_gmin(gj / kTcTileB, w.b1);
+                    gmin[0] = __shfl_sync(0xffffffffu, gmin32.x, k), gmin[1] = __shfl_sync(0xffffffffu, gmin32.y, k);
+                    gmin[2] = __shfl_sync(0xffffffffu, gmin32.z, k), gmin[3] = __shfl_sync(0xffffffffu, gmin32.w, k);
+                }
+                if (!mbar_wait(&bar_accfull[acc], accph, err, 6)) {
+                    run = false;
+                    break;
+                }
+                tc_fence_after();
+                // The warp's columns in two chunks. With two accumulators a tile's period
+                // is half the chain MMA -> commit -> load -> release -> MMA, so the
+                // accumulator goes back as soon as the second chunk is in registers,
+                // before it is reduced.
+                const uint32_t taddr = tmem + lane_base + acc * kTcTileB + half * kEpiCols;
+#pragma unroll 1
+                for (uint32_t c = 0; c < (uint32_t)kEpiCols; c += kChunkCols) {
                     float v[kChunkCols];
-                    const uint32_t taddr = tmem + lane_base + acc * kTcTileB + half * kEpiCols + c * kChunkCols;
-                    tmem_ld64(taddr, v);
-                    if (c + 1 == kEpiChunks) {
-                        // the last chunk is in registers (its slow path too works from
-                        // them): the accumulator goes back to the MMA warp before the
-                        // chunk is classified
+                    tmem_ld(taddr + c, v);
+                    tmem_wait(v);
+                    if (c) {
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&bar_accempty[acc]);
                     }
-                    // max_j v_j per 32-column group: with the group's minimum norm,
-                    // min_j (|b_j|^2 - 2 v_j) >= gmin - 2 max_j v_j
-                    float mg[kChunkGroups];
+                    // min_j (|b_j|^2 - 2 v_j) >= gmin - 2 max_j v_j per 32-column group, gmin
+                    // the group's minimum norm (0 where the norms are in the accumulator:
+                    // exact); one vote for the chunk
+                    const float m0 = fmaf(-2.0f, max32(v), c ? gmin[2] : gmin[0]);
+                    const float m1 = fmaf(-2.0f, max32(v + 32), c ? gmin[3] : gmin[1]);
+                    if (!__any_sync(0xffffffffu, fminf(m0, m1) <= thr_fast)) continue;
+                    // groups of a few near rows go to the queue
+                    const uint32_t r0 = __ballot_sync(0xffffffffu, m0 <= thr_fast);
+                    const uint32_t r1 = __ballot_sync(0xffffffffu, m1 <= thr_fast);
+                    const uint32_t k0 = __popc(r0), k1 = __popc(r1);
+                    constexpr uint32_t kNearDense = BC ? kNearDenseBc : kNearDenseOne;
+                    const bool dense0 = k0 > kNearDense, dense1 = k1 > kNearDense;
+                    if (!dense0) queue_rows(v, r0, gj + c);
+                    if (!dense1) queue_rows(v + 32, r1, gj + c + 32);
+                    if (dense0) dense_rows(v, (r0 >> lane) & 1u, gj + c);
+                    if (dense1) dense_rows(v + 32, (r1 >> lane) & 1u, gj + c + 32);
+                    if (p.dbg != nullptr && gi < p.na) {  // testing hook: every estimate
 #pragma unroll
-                    for (int g = 0; g < kChunkGroups; ++g) {
-                        // 16 three-input maxima in a tree of depth 4 (10 + 4 + 1, then one
-                        // two-input max) for the group's 32 values
-                        const float *vg = v + 32 * g;
-                        float t[10];
-#pragma unroll
-                        for (int i = 0; i < 10; ++i) t[i] = fmax3(vg[3 * i], vg[3 * i + 1], vg[3 * i + 2]);
-                        const float u0 = fmax3(t[0], t[1], t[2]), u1 = fmax3(t[3], t[4], t[5]);
-                        const float u2 = fmax3(t[6], t[7], t[8]), u3 = fmax3(t[9], vg[30], vg[31]);
-                        mg[g] = fmaf(-2.0f, fmaxf(fmax3(u0, u1, u2), u3), gmin[c * kChunkGroups + g]);
-                    }
-#pragma unroll
-                    for (int h2 = 0; h2 < kChunkGroups; ++h2) {
-                        // Rare: a 32-column half of some rows of the warp may hold a
-                        // pair that is not certainly outside. For each such row the
-                        // owning lane publishes its 32 values through shared memory
-                        // and the whole warp classifies the 32 columns at once (lane
-                        // = column), branch-free; band pairs are queued.
-                        const bool need = mg[h2] <= thr_out || (p.dbg != nullptr && row_ok);
-                        uint32_t rows = __ballot_sync(0xffffffffu, need);
-                        if (!rows) continue;
-                        const int cb = (int)(c * kChunkCols + h2 * 32);
-                        // the column's |b|^2 (block centring: 0, q_j / 2 is in the accumulator)
-                        const float nbl = BC ? 0.f : __ldg(p.norm_b + gj0 + cb + lane);
-                        // columns that may be counted at all: gj < nb, and gj > gi for a self-join
-                        int jlo = 0, jhi = kEpiCols;
-                        {
-                            const int64_t lim = (int64_t)b_end - (int64_t)gj0;
-                            jhi = lim < kEpiCols ? (lim < 0 ? 0 : (int)lim) : kEpiCols;
-                            if (self) {
-                                const int64_t first = (int64_t)gi + 1 - (int64_t)gj0;
-                                jlo = first > 0 ? (first > kEpiCols ? kEpiCols : (int)first) : 0;
-                            }
-                        }
-                        if constexpr (BC) {
-                            if (p.dbg == nullptr) {
-                                // Dense path: every lane classifies its own row against the
-                                // group's 32 columns (the column norm is in the accumulator);
-                                // band entries straight from the lane's registers: ranks by a
-                                // warp prefix sum, slots from one warp-wide reservation
-                                // t = -2 w, so t <= thr  <=>  w >= -thr / 2 (exact scaling);
-                                // the columns the row may count form one mask per group
-                                const float *vg = v + h2 * 32;
-                                const float w_in = -0.5f * thr_in, w_out = -0.5f * thr_out;
-                                const int lo = jlo - cb > 0 ? jlo - cb : 0, hi = jhi - cb < 32 ? jhi - cb : 32;
-                                const uint32_t colmask =
-                                    (need && row_ok && lo < hi)
-                                        ? ((hi >= 32 ? 0xffffffffu : (1u << hi) - 1u) & ~((1u << lo) - 1u))
-                                        : 0u;
-                                uint32_t g_in = 0, g_out = 0;
-#pragma unroll
-                                for (int j = 0; j < 32; ++j) {
-                                    g_in |= vg[j] >= w_in ? (1u << j) : 0u;
-                                    g_out |= vg[j] >= w_out ? (1u << j) : 0u;
-                                }
-                                g_in &= colmask;
-                                uint32_t bbits = g_out & colmask & ~g_in;
-                                cnt += __popc(g_in);
-                                const uint32_t nbits = __popc(bbits);
-                                uint32_t incl = nbits;
-#pragma unroll
-                                for (int o = 1; o < 32; o <<= 1) {
-                                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                                    if (lane >= (uint32_t)o) incl += y;
-                                }
-                                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-                                if (total) {
-                                    // the estimate is not kept here (reading it back by column
-                                    // index would take the values out of registers): NaN, which
-                                    // the recheck's error statistic skips
-                                    const BandSlots sl = band_reserve(total);
-                                    uint32_t rank = incl - nbits;
-                                    while (bbits) {
-                                        const int j = __ffs(bbits) - 1;
-                                        bbits &= bbits - 1;
-                                        const unsigned long long k = sl.at(rank++);
-                                        if (k < p.band_cap) {
-                                            BandEntry e;
-                                            e.ia = (uint32_t)gi;
-                                            e.jb = (uint32_t)(gj0 + cb + j);
-                                            e.s_hat = __int_as_float(0x7fc00000);
-                                            e.pad = job;
-                                            p.band[k] = e;
-                                        }
-                                    }
-                                }
-                                continue;
-                            }
-                        }
-                        while (rows) {
-                            const int L = __ffs(rows) - 1;
-                            rows &= rows - 1;
-                            if (lane == (uint32_t)L) {
-#pragma unroll
-                                for (int q = 0; q < 8; ++q)
-                                    reinterpret_cast<float4 *>(srow)[q] =
-                                        make_float4(v[h2 * 32 + 4 * q], v[h2 * 32 + 4 * q + 1], v[h2 * 32 + 4 * q + 2],
-                                                    v[h2 * 32 + 4 * q + 3]);
-                            }
-                            __syncwarp();
-                            const float naL = __shfl_sync(0xffffffffu, na, L);
-                            const float tinL = __shfl_sync(0xffffffffu, thr_in, L);
-                            const float toutL = __shfl_sync(0xffffffffu, thr_out, L);
-                            const int jloL = __shfl_sync(0xffffffffu, jlo, L);
-                            const int jhiL = __shfl_sync(0xffffffffu, jhi, L);
-                            const uint64_t giL = gi - (uint64_t)lane + (uint64_t)L;
-                            const float t = fmaf(-2.0f, srow[lane], nbl);
-                            const int col = cb + (int)lane;
-                            const bool rokL = __shfl_sync(0xffffffffu, row_ok, L);
-                            const bool ok = (unsigned)(col - jloL) < (unsigned)(jhiL - jloL) && rokL;
-                            cnt += (ok && t <= tinL) ? 1ull : 0ull;
-                            if (p.dbg != nullptr && giL < p.na && gj0 + col < p.nb)
-                                p.dbg[(uint64_t)p.perm_a[giL] * p.nb + p.perm_b[gj0 + col]] = (naL + t) * s_unscale;
-                            // band pairs of the row: one reservation for the warp
-                            const bool isb = ok && t > tinL && t <= toutL;
-                            unsigned long long k = 0;
-                            if constexpr (BC) {
-                                const uint32_t bm = __ballot_sync(0xffffffffu, isb);
-                                if (bm) k = band_reserve(__popc(bm)).at(__popc(bm & ((1u << lane) - 1u)));
-                            } else if (isb) {  // band pair: rare with one centre
-                                k = atomicAdd(p.band_total, 1ull);
-                            }
-                            if (isb && k < p.band_cap) {
-                                BandEntry e;
-                                e.ia = (uint32_t)giL;
-                                e.jb = (uint32_t)(gj0 + col);
-                                e.s_hat = (naL + t) * s_unscale;
-                                e.pad = job;
-                                p.band[k] = e;
-                            }
-                            __syncwarp();
-                        }
+                        for (int j = 0; j < kChunkCols; ++j)
+                            if (gj + c + j < p.nb)
+                                p.dbg[(uint64_t)p.perm_a[gi] * p.nb + p.perm_b[gj + c + j]] =
+                                    (na + fmaf(-2.0f, v[j], BC || fold ? 0.f : p.norm_b[gj + c + j])) * s_unscale;
                     }
                 }
-                ++t_cnt;
+                acc ^= 1u;
+                accph ^= acc ^ 1u;
             }
-            if (last_tile && it < p.n_items) item_rows(w);
+            w = wn;
+            wn = wnn;
+            wnn = item_at(it + 3 * stride);
         }
         if (job != 0xffffffffu) flush();
-        if constexpr (BC) band_holes();
+        band.finish();
+        __syncwarp();
+        if (lane == 0) sts_release(&near_tail[ew], n_tail | kNearDone);
     }
     tc_fence_before();
     __syncthreads();
@@ -874,9 +1179,18 @@ __global__ void k_recheck(const TcJob *__restrict__ jobs, const BandEntry *__res
 // products as TF32's; FP16 subnormals (|v| < 2^-14) carry an absolute error up
 // to 2^-25 instead, at most 2 * 2^-25 * 2^15 per product term, d terms, twice
 // in s: c_abs = 1.25 * d * 2^-8.
-void tc_band_constants(int form, uint32_t d, double maxabs, double *c_rel, double *c_abs) {
+//
+// Folded norms (tc_fold): the accumulator sums the products and the pieces of
+// -|b|^2 / 2, so its terms sum to at most (|a|^2 + |b|^2) / 2 + |b|^2 / 2, within
+// twice the dot product's: the accumulation budget doubles, over K = d + 3
+// columns. The split of the norm is off by 2^-33 |b|^2 + 2^-32, far inside the
+// FP32 rounding of |b|^2 that it replaces; its absolute part (2^-31 in s) joins
+// c_abs. FP16 coordinates are below 2^10 there: subnormals cost 2 * 2^-25 *
+// 2^10 per product term, d terms, twice: c_abs = 1.25 * (d * 2^-13 + 2^-31).
+void tc_band_constants(int form, uint32_t d, double maxabs, bool fold, double *c_rel, double *c_abs) {
     const double u24 = std::ldexp(1.0, -24), acc = std::ldexp(1.0, -22);
-    const double kpad = (double)tc_kterms(form, d);  // product terms summed (zero columns are not multiplied)
+    // product terms summed (zero columns are not multiplied)
+    const double kpad = fold ? 2.0 * (double)tc_kterms(form, d + 3) : (double)tc_kterms(form, d);
     double dot;
     if (form == HJ_FORM_TC_TF32 || form == HJ_FORM_TC_FP16) {
         const double u = std::ldexp(1.0, -11);
@@ -886,7 +1200,8 @@ void tc_band_constants(int form, uint32_t d, double maxabs, double *c_rel, doubl
     }
     *c_rel = 1.25 * (dot + 12 * u24 + (double)d * std::ldexp(1.0, -50));
     if (form == HJ_FORM_TC_FP16)
-        *c_abs = 1.25 * (double)d * std::ldexp(1.0, -8);
+        *c_abs = fold ? 1.25 * ((double)d * std::ldexp(1.0, -13) + std::ldexp(1.0, -31))
+                      : 1.25 * (double)d * std::ldexp(1.0, -8);
     else
         *c_abs = 1e-30 + 4.0 * (double)d * std::ldexp(std::fmax(maxabs, 1e-30), -100) * std::fmax(maxabs, 1.0);
 }
@@ -933,24 +1248,33 @@ static bool make_map(CUtensorMap *m, const void *base, CUtensorMapDataType type,
 }
 
 struct TcLayout {
-    uint32_t ka, a_bufs, nst;
+    uint32_t ka, a_bufs, nst, near_cap;
     size_t smem;
 };
 
+constexpr int kTcSmemMax = 225 * 1024 + kEpiWarps * kNearWords * 4;  // 224 KB + 1 KB + one near entry per warp
 static TcLayout tc_layout(int form, uint32_t d) {
     TcLayout L;
     L.ka = form == HJ_FORM_TC_TF32 ? (d + 31) / 32 : (d + 63) / 64;
     const uint32_t a_atoms = form == HJ_FORM_TC_BF16X3 ? 2 * L.ka : L.ka;
     const size_t a_bytes = (size_t)a_atoms * kAStageBytes;
-    const size_t budget = 224 * 1024;  // + 1 KB alignment + ~1.3 KB static smem <= 227 KB per block
-    L.a_bufs = 2 * a_bytes + 3 * kBStageBytes <= budget ? 2 : 1;
-    size_t left = budget - L.a_bufs * a_bytes;
+    // + 1 KB alignment and 0.3 KB static <= 227 KB per block
+    const size_t budget = 224 * 1024;
+    const size_t near_entry = (size_t)kEpiWarps * kNearWords * 4;
+    // the near queues take the place of a B stage where three stages remain, or of
+    // the second A buffer (an item's tiles then wait for its A tile) where four do
+    L.a_bufs = 2 * a_bytes + 3 * kBStageBytes + kNearMinCap * near_entry <= budget ? 2 : 1;
+    const size_t left = budget - L.a_bufs * a_bytes;
     L.nst = (uint32_t)(left / kBStageBytes);
     if (L.nst > 8) L.nst = 8;
-    L.smem = L.a_bufs * a_bytes + (size_t)L.nst * kBStageBytes + 1024;  // <= 225 KB
+    if (left - (size_t)L.nst * kBStageBytes < kNearMinCap * near_entry && L.nst > 3) --L.nst;
+    const size_t cap = (left - (size_t)L.nst * kBStageBytes) / near_entry;
+    L.near_cap = (uint32_t)(cap < 1 ? 1 : (cap < kNearCap ? cap : kNearCap));
+    L.smem = L.a_bufs * a_bytes + (size_t)L.nst * kBStageBytes + L.near_cap * near_entry + 1024;
     return L;
 }
 
+bool tc_fold(int form, uint32_t d) { return tc_layout(form, d + 3).ka == tc_layout(form, d).ka; }
 uint32_t tc_atoms(int form, uint32_t kcols) { return tc_layout(form, kcols).ka; }
 uint32_t tc_ksteps(int form, uint32_t kcols) {
     const uint32_t k = form == HJ_FORM_TC_TF32 ? 8u : 16u;
@@ -1010,9 +1334,9 @@ static uint64_t g_gate_ns = 0;      // set by tests through hj_debug_set_wait_ga
 
 void fill_tc_job(TcJob *j, int form, uint32_t d, double T, double op_scale, double maxabs, uint64_t a_row0,
                  uint64_t na_eff, uint64_t b_row0, uint64_t nb_eff, bool self, unsigned long long *count,
-                 const void *rows_a, const void *rows_b, double *c_rel_out, double *c_abs_out) {
+                 const void *rows_a, const void *rows_b, bool fold, double *c_rel_out, double *c_abs_out) {
     double c_rel = 0, c_abs = 0;
-    tc_band_constants(form, d, maxabs, &c_rel, &c_abs);
+    tc_band_constants(form, d, maxabs, fold, &c_rel, &c_abs);
     const double s2 = op_scale * op_scale;  // FP16: the units of the norms; 1 otherwise
     const double T_tc = T * s2;
     memset(j, 0, sizeof(*j));
@@ -1033,8 +1357,9 @@ void fill_tc_job(TcJob *j, int form, uint32_t d, double T, double op_scale, doub
     j->s_unscale = (float)(1.0 / s2);  // a power of two: exact
     j->self = self ? 1u : 0u;
     j->ka = tc_layout(form, d).ka;
-    j->ksteps = tc_ksteps(form, d);
+    j->ksteps = tc_ksteps(form, fold ? d + 3 : d);
     j->d = d;
+    j->fold = fold ? 1u : 0u;
     if (c_rel_out) *c_rel_out = c_rel;
     if (c_abs_out) *c_abs_out = c_abs;
 }
@@ -1091,6 +1416,7 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
     a.ka = L.ka;
     a.a_bufs = L.a_bufs;
     a.nst = L.nst;
+    a.near_cap = L.near_cap;
     a.items = idx.items;
     a.n_items = idx.n_items;
     a.norm_a = A.norms;
@@ -1109,6 +1435,7 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
     a.perm_a = A.perm;
     a.perm_b = B.perm;
     a.gate_ns = g_gate_ns;
+    a.fold = !bc && A.fold ? 1u : 0u;
     if (bc) {
         a.norm_a = A.bc_norms;
         a.norm_b = nullptr;  // q_j / 2 is folded into the accumulator
@@ -1125,22 +1452,22 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
     uint64_t grid = (uint64_t)num_sms;
     if (grid > idx.n_items) grid = idx.n_items;
     if (bc && form == HJ_FORM_TC_TF32) {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_TF32, true>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_TF32, true>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_TF32, true><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     } else if (bc && form == HJ_FORM_TC_BF16X3) {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_BF16X3, true>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_BF16X3, true>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_BF16X3, true><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     } else if (bc) {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_FP16, true>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_FP16, true>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_FP16, true><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     } else if (form == HJ_FORM_TC_TF32) {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_TF32, false>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_TF32, false>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_TF32, false><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     } else if (form == HJ_FORM_TC_FP16) {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_FP16, false>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_FP16, false>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_FP16, false><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     } else {
-        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_BF16X3, false>, 225 * 1024);
+        ensure_max_dynamic_smem((const void *)k_join_tc<HJ_FORM_TC_BF16X3, false>, kTcSmemMax);
         k_join_tc<HJ_FORM_TC_BF16X3, false><<<(unsigned)grid, kTcThreads, L.smem, st>>>(ma, ma2, mb, mb2, a);
     }
     cudaError_t e = cudaGetLastError();
@@ -1149,6 +1476,10 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
         return 1;
     }
     return 0;
+}
+
+uint64_t band_slack(int num_sms, bool bc) {
+    return (uint64_t)num_sms * (kEpiWarps + 2) * (bc ? kBandChunk : kBandChunkRare);
 }
 
 void launch_recheck(const TcJob *d_jobs, int dtype_bytes, const uint2 *band, const unsigned long long *d_band_total,

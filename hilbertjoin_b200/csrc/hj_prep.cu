@@ -959,18 +959,65 @@ __device__ __forceinline__ float to_tf32_rn(float v) {
     return __uint_as_float(u);
 }
 
+// Operand element of a tensor-core form: FP16 bits, or a TF32 value in an FP32
+// container (rounded to nearest through FP32; the error stays within the 2^-11
+// relative radius the bounds allow, with their 1.001 margin).
+template <int OP> struct BcElem;
+template <> struct BcElem<2> {  // FP16
+    using E = uint16_t;
+    __device__ static E round(double v, double *back) {
+        const __half h = __double2half(v);
+        *back = (double)__half2float(h);
+        return __half_as_ushort(h);
+    }
+};
+template <> struct BcElem<0> {  // TF32
+    using E = uint32_t;
+    __device__ static E round(double v, double *back) {
+        const float f = to_tf32_rn((float)v);
+        *back = (double)f;
+        return __float_as_uint(f);
+    }
+};
+template <> struct BcElem<1> {  // BF16 hi + lo (BF16x3): hi in the low 16 bits, lo in the high 16 bits;
+    using E = uint32_t;         // the stored value hi + lo is within 2^-17 |v| of v
+    __device__ static E round(double v, double *back) {
+        const __nv_bfloat16 hi = __double2bfloat16(v);
+        const double h = (double)__bfloat162float(hi);
+        const __nv_bfloat16 lo = __double2bfloat16(v - h);  // v - h exact in FP64
+        *back = h + (double)__bfloat162float(lo);
+        return (uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16);
+    }
+};
+
+// v in three operand elements, FP16 at scales 2^15, 2^4, 2^-7, TF32 and BF16
+// hi + lo at scale 1: |v - sum| <= 2^-33 |v| + 2^-32 (the pieces of a norm that
+// the MMA adds through constant columns of the other operand).
+template <int OP>
+__device__ __forceinline__ void norm_pieces(double v, typename BcElem<OP>::E (&m)[3]) {
+    const double s1 = OP == 2 ? 0x1p15 : 1.0, s2 = OP == 2 ? 0x1p4 : 1.0, s3 = OP == 2 ? 0x1p-7 : 1.0;
+    double b1, b2, b3;
+    m[0] = BcElem<OP>::round(v / s1, &b1);
+    const double v2 = v - b1 * s1;
+    m[1] = BcElem<OP>::round(v2 / s2, &b2);
+    const double v3 = v2 - b2 * s2;
+    m[2] = BcElem<OP>::round(v3 / s3, &b3);
+}
+
 // Tensor-core forms: sorted keys (row-major [n][W]), sorted rows (input
 // precision), the operand matrix ([npad][kp]: TF32, BF16 hi/lo, or FP16) of
 // the centred coordinates, and the FP64 centred norm of every rank (FP32,
 // padding ranks kPadNorm). FP16 operands are (x - center) * scale rounded once
 // from FP64 (scale a power of two: exact); TF32 and BF16 from the FP32 value
 // of x - center, BF16 as hi + lo with lo the BF16 of the exact remainder.
+// With `fold`, columns d .. d + 2 hold the pieces of half the rank's norm
+// (norm_pieces; padding ranks a norm that no pair reaches).
 template <typename T, int OP>  // OP: 0 TF32, 1 BF16 hi/lo, 2 FP16
 __global__ void __launch_bounds__(256) k_gather_tc_fused(const T *__restrict__ x, uint64_t n, uint32_t d,
                                                          const uint32_t *__restrict__ perm,
                                                          const uint32_t *__restrict__ keys_wm, uint32_t W,
                                                          const double *__restrict__ center, uint64_t npad, uint32_t kp,
-                                                         double scale, double scale2, bool vec,
+                                                         double scale, double scale2, bool vec, bool fold,
                                                          uint32_t *__restrict__ keys_rm, T *__restrict__ rows_out,
                                                          void *__restrict__ op_hi, uint16_t *__restrict__ op_lo,
                                                          float *__restrict__ norms) {
@@ -1035,6 +1082,21 @@ __global__ void __launch_bounds__(256) k_gather_tc_fused(const T *__restrict__ x
     part += __shfl_xor_sync(0xffffffffu, part, 2);
     part += __shfl_xor_sync(0xffffffffu, part, 1);
     if (in && j == 0) norms[r] = real ? (float)(part * scale2) : kPadNorm;
+    if (fold) {
+        __syncwarp();  // after the chunk stores of the same columns
+        if (in && j < 3) {
+            typename BcElem<OP>::E m[3];
+            norm_pieces<OP>(real ? 0.5 * (part * scale2) : (OP == 2 ? 0x1.ffcp30 : 1.0e30), m);
+            const typename BcElem<OP>::E e = j == 0 ? m[0] : (j == 1 ? m[1] : m[2]);
+            const uint64_t at = r * kp + d + j;
+            if (OP == 0) {
+                static_cast<uint32_t *>(op_hi)[at] = e;
+            } else {
+                static_cast<uint16_t *>(op_hi)[at] = (uint16_t)e;
+                if (OP == 1) op_lo[at] = (uint16_t)((uint32_t)e >> 16);
+            }
+        }
+    }
     if (real && keys_rm)
         for (uint32_t w = j; w < W; w += 8) keys_rm[r * W + w] = keys_wm[(uint64_t)w * n + src];
 }
@@ -1117,37 +1179,6 @@ __global__ void k_group_min(const float *__restrict__ v, uint64_t npad, int grou
 // |x - center| * scale < 2^10 per coordinate, |h_t| < 2^10 (1 + 2^-11) and
 // |q| < 3 2^20 d <= 3 2^26, so every piece is below 2^12 in magnitude.
 // Ranks past n (up to npad) are padding: zero rows, q = kPadNorm, |h| = 0.
-// Operand element of the block-centred rows: FP16 bits, or a TF32 value in an
-// FP32 container (rounded to nearest through FP32; the error stays within the
-// 2^-11 relative radius the bound allows, with its 1.001 margin).
-template <int OP> struct BcElem;
-template <> struct BcElem<2> {  // FP16
-    using E = uint16_t;
-    __device__ static E round(double v, double *back) {
-        const __half h = __double2half(v);
-        *back = (double)__half2float(h);
-        return __half_as_ushort(h);
-    }
-};
-template <> struct BcElem<0> {  // TF32
-    using E = uint32_t;
-    __device__ static E round(double v, double *back) {
-        const float f = to_tf32_rn((float)v);
-        *back = (double)f;
-        return __float_as_uint(f);
-    }
-};
-template <> struct BcElem<1> {  // BF16 hi + lo (BF16x3): hi in the low 16 bits, lo in the high 16 bits;
-    using E = uint32_t;         // the stored value hi + lo is within 2^-17 |v| of v
-    __device__ static E round(double v, double *back) {
-        const __nv_bfloat16 hi = __double2bfloat16(v);
-        const double h = (double)__bfloat162float(hi);
-        const __nv_bfloat16 lo = __double2bfloat16(v - h);  // v - h exact in FP64
-        *back = h + (double)__bfloat162float(lo);
-        return (uint32_t)__bfloat16_as_ushort(hi) | ((uint32_t)__bfloat16_as_ushort(lo) << 16);
-    }
-};
-
 // Shared memory of k_bc_prepare for dimension d and element size eb: the rows
 // in FP64 with an odd row stride (fewer bank conflicts when a thread walks its
 // own row), the centre, per-part minima and maxima, and the operand bits of the
@@ -1267,17 +1298,9 @@ __global__ void __launch_bounds__(kBcBlock) k_bc_prepare(const T *__restrict__ r
         my_p = fabsf((float)q) * (1.0f + 2.4e-7f);
         my_x = (float)sqrt(hh) * (1.0f + 2.4e-7f);
         if (xn) xn[r0 + r] = my_x;
-        // q / 2 in three pieces: FP16 at scales 2^15, 2^4, 2^-7 (the A side's
-        // constants); TF32 and BF16 hi + lo at scale 1
-        const double s1 = OP == 2 ? 0x1p15 : 1.0, s2 = OP == 2 ? 0x1p4 : 1.0, s3 = OP == 2 ? 0x1p-7 : 1.0;
-        double b1, b2, b3;
-        const double v1 = 0.5 * q;
-        mb0 = El::round(v1 / s1, &b1);
-        const double v2 = v1 - b1 * s1;
-        mb1 = El::round(v2 / s2, &b2);
-        const double v3 = v2 - b2 * s2;
-        mb2 = El::round(v3 / s3, &b3);
-        (void)b3;
+        E m[3];  // q / 2 in three pieces (the A side holds their scales)
+        norm_pieces<OP>(0.5 * q, m);
+        mb0 = m[0], mb1 = m[1], mb2 = m[2];
     } else {
         norms[r0 + r] = kPadNorm;
         if (xn) xn[r0 + r] = 0.f;
@@ -1394,7 +1417,7 @@ void launch_gather(const void *x, int dtype_bytes, uint64_t n, uint32_t d, const
         const unsigned blocks = (unsigned)hj_ceil_div(o.npad_tc, kGrpRows);
 #define HJ_GATHER_TC(T, OPV)                                                                                        \
     k_gather_tc_fused<T, OPV><<<blocks, 256, 0, st>>>(static_cast<const T *>(x), n, d, perm, keys_wm, W, o.center,   \
-                                                      o.npad_tc, kp, scale, scale2, vec, keys_rm,                    \
+                                                      o.npad_tc, kp, scale, scale2, vec, o.fold, keys_rm,            \
                                                       static_cast<T *>(rows_out), hi, o.bf_lo, o.norms)
         if (dtype_bytes == 8) {
             if (op == 0) HJ_GATHER_TC(double, 0); else if (op == 1) HJ_GATHER_TC(double, 1); else HJ_GATHER_TC(double, 2);
