@@ -313,11 +313,14 @@ void launch_norm_key(const void *x, int dtype_bytes, uint64_t n, uint32_t d, con
 }
 
 // Dimension cost (the selectivity estimate of the reference's
-// outputStatistics, hilbertjoin/egojoin.cpp:523-592): the sample's cell
-// indices of one dim are sorted in shared memory (bitonic), and every sample
-// position s counts the positions q > s with cell[q] <= cell[s] + 1 by a
-// binary search -- together the pairs in equal cells, sum h(h-1)/2, plus the
-// pairs in adjacent cells, sum h[c-1] h[c].
+// outputStatistics, hilbertjoin/egojoin.cpp:523-592): the pairs of sampled points
+// in equal cells, sum h(h-1)/2, plus the pairs in adjacent cells, sum h[c-1] h[c],
+// of one dim's cell histogram h. A dim of up to kCostSample cells has its histogram
+// in shared memory (a cell more than eps apart from the range's ends holds a
+// sample as a rule, so this is the usual case: 30k x 100 took 85 us sorted, 9 us
+// here). A wider dim's cell indices are sorted (bitonic), and every sample position s
+// counts the positions q > s with cell[q] <= cell[s] + 1 by a binary search -- the
+// same sum.
 __global__ void __launch_bounds__(1024) k_dim_cost(const void *x, int dtype_bytes, uint64_t n, uint32_t d,
                                                    double eps, const DimStats *__restrict__ ds,
                                                    unsigned long long *cost) {
@@ -325,9 +328,14 @@ __global__ void __launch_bounds__(1024) k_dim_cost(const void *x, int dtype_byte
     __shared__ unsigned long long total;
     const uint32_t t = blockIdx.x, tid = threadIdx.x;
     const uint32_t S = (uint32_t)(n < kCostSample ? n : kCostSample);
-    const long long cmin = ds[t].cmin;
+    const long long cmin = ds[t].cmin, range = ds[t].cmax - cmin;
+    const bool hist = range >= 0 && range < (long long)kCostSample;
     if (tid == 0) total = 0;
-    for (uint32_t s = tid; s < kCostSample; s += blockDim.x) {
+    if (hist) {
+        for (uint32_t s = tid; s < kCostSample; s += blockDim.x) v[s] = 0;
+        __syncthreads();
+    }
+    for (uint32_t s = tid; s < kCostSample; s += blockDim.x) {  // whole warps
         uint32_t c = 0xffffffffu;  // padding sorts last
         if (s < S) {
             const uint64_t i = (uint64_t)s * n / S;
@@ -335,36 +343,50 @@ __global__ void __launch_bounds__(1024) k_dim_cost(const void *x, int dtype_byte
             q = q < 0 ? 0 : (q > 0x7fffffffll ? 0x7fffffffll : q);
             c = (uint32_t)q;
         }
-        v[s] = c;
+        if (hist) {
+            // a dim may have two or three cells in all: one add per cell and warp
+            const uint32_t peers = __match_any_sync(0xffffffffu, c);
+            if (s < S && (peers & ((1u << (tid & 31u)) - 1u)) == 0)
+                atomicAdd(&v[c < kCostSample ? c : kCostSample - 1], (uint32_t)__popc(peers));
+        } else {
+            v[s] = c;
+        }
     }
     __syncthreads();
-    for (uint32_t k = 2; k <= kCostSample; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = tid; i < kCostSample; i += blockDim.x) {
-                const uint32_t p = i ^ j;
-                if (p > i) {
-                    const uint32_t a = v[i], b = v[p];
-                    if ((a > b) == ((i & k) == 0)) {
-                        v[i] = b;
-                        v[p] = a;
+    unsigned long long mine = 0;
+    if (hist) {
+        for (uint32_t c = tid; c < kCostSample; c += blockDim.x) {
+            const unsigned long long h = v[c], below = c ? v[c - 1] : 0u;
+            if (h) mine += h * (h - 1) / 2 + h * below;
+        }
+    } else {
+        for (uint32_t k = 2; k <= kCostSample; k <<= 1) {
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                for (uint32_t i = tid; i < kCostSample; i += blockDim.x) {
+                    const uint32_t p = i ^ j;
+                    if (p > i) {
+                        const uint32_t a = v[i], b = v[p];
+                        if ((a > b) == ((i & k) == 0)) {
+                            v[i] = b;
+                            v[p] = a;
+                        }
                     }
                 }
+                __syncthreads();
             }
-            __syncthreads();
         }
-    }
-    unsigned long long mine = 0;
-    for (uint32_t s = tid; s < S; s += blockDim.x) {
-        const uint32_t lim = v[s] + 1;  // cells are below 2^31: no wrap
-        uint32_t lo = s + 1, hi = S;    // first q in (s, S) with v[q] > lim
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (v[mid] <= lim)
-                lo = mid + 1;
-            else
-                hi = mid;
+        for (uint32_t s = tid; s < S; s += blockDim.x) {
+            const uint32_t lim = v[s] + 1;  // cells are below 2^31: no wrap
+            uint32_t lo = s + 1, hi = S;    // first q in (s, S) with v[q] > lim
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (v[mid] <= lim)
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            mine += lo - s - 1;
         }
-        mine += lo - s - 1;
     }
     mine = warp_sum_u64(mine);
     if ((tid & 31u) == 0 && mine) atomicAdd(&total, mine);
@@ -1142,25 +1164,36 @@ __global__ void __launch_bounds__(256) k_gather_plain_tiles(const T *__restrict_
 
 // ------------------------------------------------------------ norm summaries
 
-// Per-tile maximum norm over real rows (padding rows excluded).
-__global__ void k_tile_max(const float *__restrict__ v, uint64_t npad, int tile, float *out) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t * tile >= npad) return;
-    float m = 0.0f;
-    for (int i = 0; i < tile; ++i) {
-        float x = v[t * tile + i];
-        if (x < 1e29f) m = fmaxf(m, x);
+// One warp per B tile (256 ranks), each lane eight consecutive norms in two 128-bit
+// loads: maxima over real rows (padding rows excluded) of the tile and of its two A
+// tiles, and the minima of its eight 32-row groups (four lanes each; padding rows
+// hold kPadNorm and never lower them). Bound by the launch: 100k norms took 70 us in
+// three kernels whose threads each walked a tile, 3 us here.
+constexpr int kNormTilesPerBlock = 8;
+__global__ void __launch_bounds__(32 * kNormTilesPerBlock) k_norm_summaries(const float *__restrict__ norms,
+                                                                            uint64_t tiles, float *tmax_a,
+                                                                            float *tmax_b, float *gmin32) {
+    static_assert(kTcTileB == 256 && kTcTileA == 128, "eight norms per lane");
+    const uint64_t tile = (uint64_t)blockIdx.x * kNormTilesPerBlock + (threadIdx.x >> 5);
+    const uint32_t lane = threadIdx.x & 31u;
+    if (tile >= tiles) return;
+    const float4 *src = reinterpret_cast<const float4 *>(norms + tile * kTcTileB) + 2 * lane;
+    const float4 a = __ldg(src), b = __ldg(src + 1);
+    const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    float mx = 0.0f, mn = 3.0e38f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (v[i] < 1e29f) mx = fmaxf(mx, v[i]);
+        mn = fminf(mn, v[i]);
     }
-    out[t] = m;
-}
-
-// Per-group minimum norm (padding rows hold kPadNorm and never lower it).
-__global__ void k_group_min(const float *__restrict__ v, uint64_t npad, int group, float *out) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t * group >= npad) return;
-    float m = 3.0e38f;
-    for (int i = 0; i < group; ++i) m = fminf(m, v[t * group + i]);
-    out[t] = m;
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+    if ((lane & 3u) == 0) gmin32[tile * 8 + (lane >> 2)] = mn;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((lane & 15u) == 0) tmax_a[tile * 2 + (lane >> 4)] = mx;
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    if (lane == 0) tmax_b[tile] = mx;
 }
 
 // ------------------------------------------------------------ per-block centring
@@ -1426,7 +1459,7 @@ void launch_gather(const void *x, int dtype_bytes, uint64_t n, uint32_t d, const
         }
 #undef HJ_GATHER_TC
         launch_norm_summaries(o.norms, o.npad_tc, o.tile_maxnorm_a, o.tile_maxnorm_b, o.group_minnorm, st);
-        L += 4;
+        L += 2;
     } else if (keys_rm || rows_out) {
         const unsigned blocks = (unsigned)hj_ceil_div(n, kGrpRows);
         if (dtype_bytes == 8)
@@ -1452,9 +1485,9 @@ void launch_gather(const void *x, int dtype_bytes, uint64_t n, uint32_t d, const
 void launch_norm_summaries(const float *norms, uint64_t npad, float *tmax_a, float *tmax_b, float *gmin32,
                            cudaStream_t st) {
     if (npad == 0) return;
-    k_tile_max<<<(unsigned)hj_ceil_div(npad / kTcTileA, 256), 256, 0, st>>>(norms, npad, kTcTileA, tmax_a);
-    k_tile_max<<<(unsigned)hj_ceil_div(npad / kTcTileB, 256), 256, 0, st>>>(norms, npad, kTcTileB, tmax_b);
-    k_group_min<<<(unsigned)hj_ceil_div(npad / 32, 256), 256, 0, st>>>(norms, npad, 32, gmin32);
+    const uint64_t tiles = npad / kTcTileB;
+    k_norm_summaries<<<(unsigned)hj_ceil_div(tiles, kNormTilesPerBlock), 32 * kNormTilesPerBlock, 0, st>>>(
+        norms, tiles, tmax_a, tmax_b, gmin32);
 }
 
 }  // namespace hj

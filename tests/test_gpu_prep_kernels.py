@@ -1,0 +1,48 @@
+"""The preparation kernels at the edges of their tiles and ranges: norm summaries
+(padding rows, one and several tiles) through counts that depend on them, and the
+dimension cost of dims whose cells fit the shared-memory histogram and of dims
+whose cells do not."""
+import numpy as np
+import pytest
+
+import oracle as O
+from hilbertjoin_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hj():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import hilbertjoin_b200 as hj
+    return hj
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 255, 256, 257, 2047, 2049, 4100])
+def test_norm_summaries_at_tile_edges(hj, n):
+    # norms from 1e-6 to 1e2 (d = 64: not folded, every group minimum decides)
+    rng = np.random.default_rng(n)
+    x = (rng.standard_normal((n, 64)) * np.exp(rng.uniform(-6, 0, (n, 1)))).astype(np.float32)
+    x64 = x.astype(np.float64)
+    for eps in (0.05, 1.0):
+        assert hj.self_join_count(x, eps, form="fp16", centring="global") == O.self_count_brute(x64, eps)
+
+
+@pytest.mark.parametrize("n", [5, 8192, 20000])
+def test_dim_cost_narrow_and_wide_dims(hj, n):
+    """Costs against the definition, sum h(h-1)/2 + sum h[c-1] h[c] over the sample's
+    cells: dims of 1, 3, 8192, 8193 and 10^6 cells."""
+    rng = np.random.default_rng(n)
+    x = np.stack([np.zeros(n), *[rng.integers(0, c, n) + 0.5 for c in (3, 8192, 8193, 10**6)]], axis=1)
+    if n > 1:
+        for j, c in enumerate((3, 8192, 8193, 10**6)):
+            x[0, j + 1], x[1, j + 1] = 0.5, c - 0.5  # the whole range occurs
+    _, costs = hj.dim_order(x, 1.0, return_costs=True)
+    s = min(n, 8192)
+    sample = x[(np.arange(s, dtype=np.uint64) * np.uint64(n) // np.uint64(s)).astype(np.int64)]
+    for j in range(x.shape[1]):
+        cell, h = np.unique(np.floor(sample[:, j]).astype(np.int64), return_counts=True)
+        near = sum(int(h[k]) * int(h[k - 1]) for k in range(1, len(cell)) if cell[k] == cell[k - 1] + 1)
+        assert int(costs[j]) == int((h.astype(np.int64) * (h - 1) // 2).sum()) + near, j
