@@ -9,6 +9,7 @@
 // point, when its cell vector is packed into 32-bit key words whose unsigned
 // order is the lexicographic cell order; the sort then only moves 4-byte
 // indices, and every data layout is written once, by the gather.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -546,12 +547,15 @@ __global__ void __launch_bounds__(1024) k_scan_u32(uint32_t *a, uint64_t count, 
 // ------------------------------------------------------------ radix sort
 //
 // Stable LSD radix sort of a permutation by 8-bit windows of word-major keys.
-// Every pass moves (key, index) pairs: the index (the permutation) and the
-// current key word in the current order, so that a pass reads both with
-// coalesced 128-bit loads. Per pass:
+//
+// Up to kRcMax items one cluster of eight CTAs runs every pass in one launch
+// (k_rs_cluster, below). Larger sets take launches per pass, each moving (key,
+// index) pairs: the index (the permutation) and the current key word in the current
+// order, so that a pass reads both with coalesced 128-bit loads. Per pass:
 //   k_rs_count      per 2048-item tile, the 256 digit counts;
-//   k_rs_scan_rows  one block per digit: exclusive scan of that digit's tile
-//                   counts, and the digit's total;
+//   k_rs_scan_rows  above kRsDirectTiles tiles only, one block per digit: exclusive
+//                   scan of that digit's tile counts, and the digit's total (below,
+//                   every scatter block sums the counts it needs: a launch less);
 //   k_rs_scatter    per tile, a stable local sort by digit in shared memory
 //                   (warp match + per-warp running counts, warps in order),
 //                   then coalesced stores of each digit's run at its global
@@ -565,6 +569,10 @@ constexpr int kRsIpt = 8;                       // items per thread
 constexpr int kRsTile = kRsThreads * kRsIpt;    // 2048 items per tile
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsWarpItems = kRsTile / kRsWarps;  // 256 consecutive items per warp
+// Tiles up to which a scatter block sums the tile counts itself: eight warps read
+// 1 KB per tile from L2 (64 tiles: about 1 us; the scan's launch costs 3 to 4). The
+// sums grow with the square of the tiles, so larger sorts scan.
+constexpr uint32_t kRsDirectTiles = 96;
 
 static uint64_t rs_round4(uint64_t n) { return hj_ceil_div(n, 4) * 4; }
 
@@ -593,7 +601,7 @@ __device__ __forceinline__ void rs_load_tile(const uint32_t *__restrict__ a, uin
 }
 
 __global__ void __launch_bounds__(kRsThreads) k_rs_count(const uint32_t *__restrict__ key, uint64_t n, uint32_t shift,
-                                                        uint32_t nb, bool vec, uint32_t *__restrict__ counts) {
+                                                        uint32_t nb, bool vec, bool direct, uint32_t *__restrict__ counts) {
     __shared__ uint32_t h[256];
     __shared__ __align__(16) uint32_t s_key[kRsTile];
     const uint32_t t = threadIdx.x, lane = t & 31u;
@@ -610,7 +618,8 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_count(const uint32_t *__restr
         if (dg < 256u && (peers & lt) == 0) atomicAdd(&h[dg], (uint32_t)__popc(peers));
     }
     __syncthreads();
-    counts[(size_t)t * nb + blockIdx.x] = h[t];
+    // [tile][digit] for the scatter's own sums, [digit][tile] for the scan
+    counts[direct ? (size_t)blockIdx.x * 256 + t : (size_t)t * nb + blockIdx.x] = h[t];
 }
 
 // Exclusive scan of 1024 values held one per thread; returns the thread's
@@ -668,6 +677,7 @@ __global__ void __launch_bounds__(1024) k_rs_scan_rows(uint32_t *__restrict__ co
 // (key, index), the loaded one and the locally sorted one (64 KB).
 constexpr int kRsScatterSmem = 4 * kRsTile * 4;
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__restrict__ key_in,
                                                           const uint32_t *__restrict__ val_in, uint64_t n,
                                                           uint32_t shift, uint32_t nb, bool vec_key,
@@ -689,6 +699,32 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
         rs_load_tile(val_in, base, n, ((uintptr_t)val_in & 15u) == 0, s_val);
     } else {
         for (uint32_t i = t; i < m; i += kRsThreads) s_val[i] = (uint32_t)(base + i);
+    }
+    // direct: this digit's count over all tiles and over the tiles before this one.
+    // Warp w sums tiles w, w + 8, ..; a lane holds eight digits.
+    uint32_t d_all = 0, d_pre = 0;
+    if (DIRECT) {
+        uint32_t all[8] = {}, pre[8] = {};
+#pragma unroll 4
+        for (uint32_t j = warp; j < nb; j += kRsWarps) {
+            const uint4 *c = reinterpret_cast<const uint4 *>(counts + (size_t)j * 256 + 8 * lane);
+            const uint4 a = __ldg(c), b = __ldg(c + 1);
+            const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                all[k] += v[k];
+                if (j < blockIdx.x) pre[k] += v[k];
+            }
+        }
+        // the sorted tile's buffers are free until step 3
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            o_key[warp * 256 + 8 * lane + k] = all[k];
+            o_val[warp * 256 + 8 * lane + k] = pre[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kRsWarps; ++w) d_all += o_key[w * 256 + t], d_pre += o_val[w * 256 + t];
     }
 #pragma unroll
     for (int w = 0; w < kRsWarps; ++w) s_cnt[w][t] = 0;
@@ -726,7 +762,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
         }
         // exclusive scans over the 256 digits of the tile's digit counts (x0)
         // and of the digits' totals over all tiles (x1)
-        const unsigned long long x0 = run, x1 = totals[t];
+        const unsigned long long x0 = run, x1 = DIRECT ? d_all : totals[t];
         unsigned long long a = x0, b = x1;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -739,7 +775,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
         unsigned long long pa = 0, pb = 0;
         for (uint32_t w = 0; w < warp; ++w) pa += sh[w], pb += sh[8 + w];
         s_dstart[t] = (uint32_t)(pa + a - x0);
-        s_gbase[t] = (uint32_t)(pb + b - x1) + counts[(size_t)t * nb + blockIdx.x];
+        s_gbase[t] = (uint32_t)(pb + b - x1) + (DIRECT ? d_pre : counts[(size_t)t * nb + blockIdx.x]);
     }
     __syncthreads();
     // 3. the tile sorted by digit into the second buffer
@@ -766,6 +802,130 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *__res
     }
 }
 
+// The whole sort of up to kRcMax items in one launch: a cluster of eight CTAs holds
+// the (key, index) pairs in its shared memory, CTA c the positions [c seg, (c + 1)
+// seg) of the current order. A pass ranks each CTA's items by digit (warp match and
+// per-warp running counts, as the scatter above), exchanges the digit totals, and
+// writes every pair straight into the CTA of its new position (distributed shared
+// memory). Two cluster barriers stand where the multi-launch sort has two to three
+// launches: a pass takes 3 us at 20k items, against 15 us; above kRcMax the pairs
+// outgrow the cluster.
+constexpr int kRcCtas = 8, kRcThreads = 1024, kRcWarps = kRcThreads / 32;
+constexpr int kRcItems = 4096;  // per CTA
+constexpr uint32_t kRcMax = kRcCtas * kRcItems;
+constexpr uint32_t kRcMaxPasses = 64;
+struct RcPasses {
+    uint32_t np;
+    uint16_t word[kRcMaxPasses];
+    uint8_t shift[kRcMaxPasses];
+};
+constexpr size_t kRcSmem = 4 * (size_t)kRcItems * 4 + (size_t)kRcWarps * 256 * 2 + (4 + 2) * 256 * 4;
+
+__global__ void __cluster_dims__(kRcCtas, 1, 1) __launch_bounds__(kRcThreads)
+    k_rs_cluster(const uint32_t *__restrict__ keys_wm, uint32_t n, uint32_t seg, const __grid_constant__ RcPasses P,
+                 uint32_t *__restrict__ perm_out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) uint32_t rc_smem[];
+    uint32_t *key[2] = {rc_smem, rc_smem + kRcItems}, *val[2] = {rc_smem + 2 * kRcItems, rc_smem + 3 * kRcItems};
+    uint16_t(*cnt)[256] = reinterpret_cast<uint16_t(*)[256]>(rc_smem + 4 * kRcItems);  // [warp][digit]
+    uint32_t *part = rc_smem + 4 * kRcItems + kRcWarps * 128;                          // [4][256]
+    uint32_t *tot = part + 4 * 256, *base = tot + 256;                                 // [256] each
+    __shared__ uint32_t wsum[8];
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31u, rank = cluster.block_rank();
+    const uint32_t p0 = rank * seg, m = p0 >= n ? 0u : (n - p0 < seg ? n - p0 : seg);
+    const uint32_t rounds = (seg + kRcThreads - 1) / kRcThreads;  // <= 4
+    const uint32_t lt = (1u << lane) - 1u;
+    for (uint32_t i = t; i < m; i += kRcThreads) val[0][i] = p0 + i;
+    uint32_t cur = 0;
+    for (uint32_t p = 0; p < P.np; ++p) {
+        const uint32_t shift = P.shift[p];
+        const bool load = p == 0 || P.word[p] != P.word[p - 1];  // another word: gathered by index
+        const uint32_t *word = keys_wm + (size_t)P.word[p] * n;
+        for (uint32_t i = t; i < kRcWarps * 128; i += kRcThreads) reinterpret_cast<uint32_t *>(cnt)[i] = 0;
+        __syncthreads();
+        uint32_t k[kRcItems / kRcThreads], r[kRcItems / kRcThreads];
+#pragma unroll
+        for (uint32_t j = 0; j < kRcItems / kRcThreads; ++j) {
+            const uint32_t i = warp * 32 * rounds + j * 32 + lane;
+            k[j] = j < rounds && i < m ? (load ? __ldg(word + val[cur][i]) : key[cur][i]) : 0u;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kRcItems / kRcThreads; ++j) {
+            if (j >= rounds) break;
+            const uint32_t i = warp * 32 * rounds + j * 32 + lane;
+            const uint32_t dg = i < m ? (k[j] >> shift) & 255u : 256u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, dg);
+            const uint32_t before = dg < 256u ? cnt[warp][dg] : 0u;
+            __syncwarp();
+            if (dg < 256u && (peers & lt) == 0) cnt[warp][dg] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+            r[j] = before + __popc(peers & lt);
+        }
+        __syncthreads();
+        {  // counts -> exclusive prefixes over the warps, four threads per digit
+            const uint32_t dg = t & 255u, q = t >> 8;
+            uint32_t run = 0;
+#pragma unroll
+            for (uint32_t w = 0; w < kRcWarps / 4; ++w) {
+                const uint32_t c = cnt[q * (kRcWarps / 4) + w][dg];
+                cnt[q * (kRcWarps / 4) + w][dg] = (uint16_t)run;
+                run += c;
+            }
+            part[q * 256 + dg] = run;
+        }
+        __syncthreads();
+        if (t < 256) {
+            uint32_t run = 0;
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t c = part[q * 256 + t];
+                part[q * 256 + t] = run;
+                run += c;
+            }
+            tot[t] = run;
+        }
+        cluster.sync();  // every CTA's totals
+        if (t < 256) {
+            uint32_t pre = 0, all = 0;
+#pragma unroll
+            for (uint32_t c = 0; c < (uint32_t)kRcCtas; ++c) {
+                const uint32_t v = cluster.map_shared_rank(tot, c)[t];
+                all += v;
+                if (c < rank) pre += v;
+            }
+            uint32_t incl = all;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            if (lane == 31) wsum[warp] = incl;
+            base[t] = incl - all + pre;
+        }
+        __syncthreads();
+        if (t < 256) {
+            uint32_t before = 0;
+            for (uint32_t w = 0; w < warp; ++w) before += wsum[w];
+            base[t] += before;
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < kRcItems / kRcThreads; ++j) {
+            const uint32_t i = warp * 32 * rounds + j * 32 + lane;
+            if (j >= rounds || i >= m) continue;
+            const uint32_t dg = (k[j] >> shift) & 255u;
+            const uint32_t pos = base[dg] + part[(warp / (kRcWarps / 4)) * 256 + dg] + cnt[warp][dg] + r[j];
+            const uint32_t c = pos / seg, off = pos - c * seg;
+            cluster.map_shared_rank(val[cur ^ 1u], c)[off] = val[cur][i];
+            cluster.map_shared_rank(key[cur ^ 1u], c)[off] = k[j];
+        }
+        cluster.sync();  // the new order is complete, and the totals have been read
+        cur ^= 1u;
+    }
+    for (uint32_t i = t; i < m; i += kRcThreads) perm_out[p0 + i] = val[cur][i];
+}
+
 __global__ void k_iota(uint32_t *p, uint64_t n) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = (uint32_t)i;
@@ -779,13 +939,33 @@ void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32
         if (launches) *launches += 1;
         return;
     }
+    if (n <= kRcMax && np <= kRcMaxPasses) {
+        RcPasses P;
+        P.np = (uint32_t)np;
+        bool fits = true;
+        for (size_t p = 0; p < np; ++p) {
+            fits = fits && passes[p].first < 65536u;
+            P.word[p] = (uint16_t)passes[p].first;
+            P.shift[p] = (uint8_t)passes[p].second;
+        }
+        if (fits) {
+            ensure_max_dynamic_smem((const void *)k_rs_cluster, (int)kRcSmem);
+            // whole warps per CTA; eight CTAs cover n
+            const uint32_t seg = (uint32_t)hj_ceil_div(hj_ceil_div(n, kRcCtas), 32) * 32;
+            k_rs_cluster<<<kRcCtas, kRcThreads, kRcSmem, st>>>(keys_wm, (uint32_t)n, seg, P, perm_out);
+            if (launches) *launches += 1;
+            return;
+        }
+    }
     const uint64_t nn = rs_round4(n);
     uint32_t *vtmp = static_cast<uint32_t *>(scratch);
     uint32_t *kb[2] = {vtmp + nn, vtmp + 2 * nn};
     const uint32_t nb = (uint32_t)hj_ceil_div(n, kRsTile);
     uint32_t *counts = vtmp + 3 * nn;
     uint32_t *totals = counts + (size_t)256 * nb;
-    ensure_max_dynamic_smem((const void *)k_rs_scatter, kRsScatterSmem);
+    const bool direct = nb <= kRsDirectTiles;
+    ensure_max_dynamic_smem(direct ? (const void *)k_rs_scatter<true> : (const void *)k_rs_scatter<false>,
+                            kRsScatterSmem);
     const uint32_t *val_in = nullptr;
     for (size_t p = 0; p < np; ++p) {
         const uint32_t shift = passes[p].second;
@@ -797,11 +977,16 @@ void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32
         uint32_t *key_out = p + 1 < np ? kb[(p + 1) & 1] : nullptr;
         const uint32_t *next_word = nullptr;
         if (key_out && passes[p + 1].first != passes[p].first) next_word = keys_wm + (size_t)passes[p + 1].first * n;
-        k_rs_count<<<nb, kRsThreads, 0, st>>>(key_in, n, shift, nb, vec_key, counts);
-        k_rs_scan_rows<<<256, 1024, 0, st>>>(counts, nb, totals);
-        k_rs_scatter<<<nb, kRsThreads, kRsScatterSmem, st>>>(key_in, val_in, n, shift, nb, vec_key, counts, totals,
-                                                             val_out, key_out, next_word);
-        if (launches) *launches += 3;
+        k_rs_count<<<nb, kRsThreads, 0, st>>>(key_in, n, shift, nb, vec_key, direct, counts);
+        if (direct) {
+            k_rs_scatter<true><<<nb, kRsThreads, kRsScatterSmem, st>>>(key_in, val_in, n, shift, nb, vec_key, counts,
+                                                                       totals, val_out, key_out, next_word);
+        } else {
+            k_rs_scan_rows<<<256, 1024, 0, st>>>(counts, nb, totals);
+            k_rs_scatter<false><<<nb, kRsThreads, kRsScatterSmem, st>>>(key_in, val_in, n, shift, nb, vec_key, counts,
+                                                                        totals, val_out, key_out, next_word);
+        }
+        if (launches) *launches += direct ? 2 : 3;
         val_in = val_out;
     }
 }

@@ -46,3 +46,19 @@ def test_dim_cost_narrow_and_wide_dims(hj, n):
         cell, h = np.unique(np.floor(sample[:, j]).astype(np.int64), return_counts=True)
         near = sum(int(h[k]) * int(h[k - 1]) for k in range(1, len(cell)) if cell[k] == cell[k - 1] + 1)
         assert int(costs[j]) == int((h.astype(np.int64) * (h - 1) // 2).sum()) + near, j
+
+
+# the cluster sort's segments (8 CTAs of whole warps, up to 4096 items each), its
+# largest size and the first above it; the scatter's own sums (96 tiles of 2048) and
+# the first size that scans
+@pytest.mark.parametrize("n", [2, 255, 257, 1025, 8192, 8193, 32767, 32768, 32769, 40961, 96 * 2048, 96 * 2048 + 1])
+@pytest.mark.parametrize("cells", [2, 50])
+def test_ego_order_is_stable_at_the_sort_s_edges(hj, n, cells):
+    """perm is the stable order by cell vector: many equal keys (2 cells per dim) and
+    several key words (50 cells in 9 dims)."""
+    x = np.random.default_rng(n + cells).random((n, 9 if cells > 2 else 3)) * cells
+    perm, srt = hj.ego_sort(x, 1.0)
+    cell = np.floor(x).astype(np.int64)
+    want = np.lexsort([cell[:, t] for t in range(x.shape[1] - 1, -1, -1)])
+    assert np.array_equal(perm.astype(np.int64), want)
+    assert np.array_equal(srt, x[want])
