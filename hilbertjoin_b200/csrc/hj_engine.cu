@@ -152,9 +152,12 @@ static int bitwidth(unsigned long long v) {
 }
 
 // Plans the packed key layout from the per-dim cell ranges. `ord` (empty =
-// identity) lists the dims from the most significant key field down.
+// identity) lists the dims from the most significant key field down. The key ends
+// with the last word that `min_dims` and `min_bits` need (0xffffffff: every dim has
+// a field): a key over the first dims in order is the EGO order of those dims, for
+// which the stripe search is complete, too.
 static int plan_grid(const std::vector<DimStats> &ds, uint32_t d, double eps, double maxabs,
-                     const std::vector<uint32_t> &ord, Grid *g) {
+                     const std::vector<uint32_t> &ord, uint32_t min_dims, uint32_t min_bits, Grid *g) {
     g->d = d;
     g->ord = ord;
     if (g->ord.empty())
@@ -167,7 +170,8 @@ static int plan_grid(const std::vector<DimStats> &ds, uint32_t d, double eps, do
     g->word.resize(d);
     g->shift.resize(d);
     g->range.resize(d);
-    uint32_t w = 0, left = 32;
+    uint32_t w = 0, left = 32, used = 0;
+    g->dk = d;
     for (uint32_t pos = 0; pos < d; ++pos) {
         const uint32_t t = g->ord[pos];
         long long lo = ds[t].cmin, hi = ds[t].cmax;
@@ -178,9 +182,12 @@ static int plan_grid(const std::vector<DimStats> &ds, uint32_t d, double eps, do
                                                            "cells in one dimension");
         uint32_t b = (uint32_t)bitwidth((unsigned long long)range + 4);
         if (b > left) {
-            ++w;
+            if (pos < g->dk && pos >= min_dims && used >= min_bits) g->dk = pos;
+            if (pos < g->dk) ++w;
             left = 32;
         }
+        if (pos >= g->dk) continue;  // no field (the range is checked above)
+        if (range) used += b;
         g->off[t] = lo - 2;
         g->bits[t] = b;
         g->word[t] = w;
@@ -204,6 +211,22 @@ static int plan_grid(const std::vector<DimStats> &ds, uint32_t d, double eps, do
         }
     }
     return HJ_OK;
+}
+
+// How much of the key a join of n points sorts by. What a count needs of the order is
+// the stripes (the active dims and the one after them, in which a stripe is a range)
+// and that a tile's points lie together; log2(n) and some bits of occupied cells
+// give that, and every further word is up to four radix passes and its share of the
+// key, bound and gather traffic. Whole joins, whole key -> 8 bits more than log2(n)
+// -> 24 bits more: 20k x 16 plain 0.536 -> 0.480 -> 0.553 ms, 200k x 200k x 20 7.43 ->
+// 7.20 -> 7.44, 300k x 32 clustered TF32 3.28 -> 2.87 -> 2.87, 4M x 28 clustered FP16
+// 45.4 -> 45.3 -> 44.2 (its sort 2.6 -> 1.4 -> 1.6, its block-centred kernel 38.1 ->
+// 39.9 -> 38.4: tiles are looser in the dims left out). ref_compat drops the last
+// points of the whole EGO order, so it keeps the whole key.
+static void key_budget(uint64_t n, int active_dims, bool ref_compat, uint32_t *min_dims, uint32_t *min_bits) {
+    if (ref_compat) return;
+    *min_dims = (uint32_t)active_dims + 1;
+    *min_bits = (uint32_t)bitwidth(n) + (n > (1u << 18) ? 24u : 8u);
 }
 
 struct JoinIn {
@@ -440,8 +463,11 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
         P->reorder_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
     Grid &g = P->g;
-    if (int r = plan_grid(hds, d, in.eps, maxabs, ord, &g)) return r;
+    uint32_t min_dims = 0xffffffffu, min_bits = 0xffffffffu;
+    key_budget(std::max(in.na, in.nb), active_dims, ref_compat, &min_dims, &min_bits);
+    if (int r = plan_grid(hds, d, in.eps, maxabs, ord, min_dims, min_bits, &g)) return r;
     GridDev &gd = P->gd;
+    gd.dk = g.dk;
     if (!ord.empty()) {
         gd.ord = (uint32_t *)slot_alloc_impl(c, st, kSlotGridOrd, d * 4);
         if (!gd.ord) return fail(HJ_ERR_OOM, "out of device memory");
@@ -973,8 +999,9 @@ static int ego_sort_host(const double *pts, uint64_t n, uint32_t d, double eps, 
     double maxabs;
     std::memcpy(&maxabs, &c->h_small[0], 8);
     Grid g;
-    if (int r = plan_grid(hds, d, eps, maxabs, {}, &g)) return r;
+    if (int r = plan_grid(hds, d, eps, maxabs, {}, 0xffffffffu, 0xffffffffu, &g)) return r;
     GridDev gd;
+    gd.dk = g.dk;
     gd.off = (long long *)slot_alloc_impl(c, st, kSlotGridOff, d * 8);
     gd.bits = (uint32_t *)slot_alloc_impl(c, st, kSlotGridBits, d * 4);
     gd.word = (uint32_t *)slot_alloc_impl(c, st, kSlotGridWord, d * 4);

@@ -76,7 +76,7 @@ __global__ void k_bound_keys(BoundsArgs a) {
     if (r >= a.na) return;
     uint32_t *lo = a.lokeys + r * a.W, *hi = a.hikeys + r * a.W;
     uint32_t cur = 0, al = 0, ah = 0;
-    for (uint32_t pos = 0; pos < a.d; ++pos) {
+    for (uint32_t pos = 0; pos < a.g.dk; ++pos) {
         const uint32_t t = grid_dim_at(a.g, pos), w = a.g.word[t];
         if (w != cur) {
             lo[cur] = al;
@@ -175,8 +175,8 @@ __global__ void __launch_bounds__(kBoundsWarps * 32) k_tile_bounds(BoundsArgs a,
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) kt = min(kt, __shfl_xor_sync(0xffffffffu, kt, o));
     // the upper key's boundary: the field of key position kt (hi from there on)
-    uint32_t mw = 0xffffffffu, mbits = 0;  // kt >= d: every position takes its lo digit
-    if ((uint32_t)kt < a.d) {
+    uint32_t mw = 0xffffffffu, mbits = 0;  // kt >= dk: every position takes its lo digit
+    if ((uint32_t)kt < a.g.dk) {
         const uint32_t t = grid_dim_at(a.g, (uint32_t)kt);
         mw = a.g.word[t];
         mbits = a.g.shift[t] + a.g.bits[t];
@@ -497,7 +497,7 @@ int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const 
     const uint64_t n_tiles = hj_ceil_div(na_eff, tile_a);
     if (n_tiles == 0 || nb_eff == 0) return 0;
     int k = active_dims < 0 ? 0 : (active_dims > kMaxActiveDims ? kMaxActiveDims : active_dims);
-    if ((uint32_t)k > grid.d) k = (int)grid.d;
+    if ((uint32_t)k > grid.dk) k = (int)grid.dk;
     uint2 *runs = (uint2 *)alloc(actx, kSlotRuns, n_tiles * kMaxCombos * sizeof(uint2));
     uint32_t *nruns = (uint32_t *)alloc(actx, kSlotNruns, n_tiles * sizeof(uint32_t));
     uint32_t *counts = (uint32_t *)alloc(actx, kSlotCounts, (n_tiles + 1) * sizeof(uint32_t));

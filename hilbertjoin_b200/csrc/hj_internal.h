@@ -54,6 +54,7 @@ struct Grid {
     uint32_t d = 0;
     double eps = 0, eps_wide = 0, maxabs = 0;
     uint32_t W = 0;                    // 32-bit words per key
+    uint32_t dk = 0;                   // key positions: the first dk dims in key order have a field
     std::vector<long long> off;        // per dim
     std::vector<uint32_t> bits, word, shift;
     std::vector<long long> range;      // max cell - min cell per dim
@@ -70,6 +71,7 @@ struct GridDev {
     long long *off = nullptr;
     uint32_t *bits = nullptr, *word = nullptr, *shift = nullptr;
     uint32_t *ord = nullptr;
+    uint32_t dk = 0;  // dims with a field (plan_grid)
 };
 __host__ __device__ inline uint32_t grid_dim_at(const GridDev &g, uint32_t pos) { return g.ord ? g.ord[pos] : pos; }
 

@@ -142,6 +142,7 @@ extern "C" int hj_ego_sort_device_noalloc(const void *pts, int dtype_bytes, uint
     if (o_rs + rs_bytes > kScratchBytes)
         return engine_fail(HJ_ERR_INVALID_ARG, "packed keys of this input exceed the fixed 32 MiB scratch array");
     GridDev gd;
+    gd.dk = d;
     gd.off = reinterpret_cast<long long *>(base + o_off);
     gd.bits = reinterpret_cast<uint32_t *>(base + o_bits);
     gd.word = reinterpret_cast<uint32_t *>(base + o_word);

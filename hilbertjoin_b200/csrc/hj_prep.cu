@@ -271,7 +271,7 @@ __global__ void k_pack_keys(const void *x, int dtype_bytes, uint64_t n, uint32_t
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t cur_word = 0, acc = 0;
-    for (uint32_t pos = 0; pos < d; ++pos) {
+    for (uint32_t pos = 0; pos < g.dk; ++pos) {
         const uint32_t t = grid_dim_at(g, pos);
         uint32_t w = g.word[t];
         if (w != cur_word) {
@@ -429,8 +429,10 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
     PkPos *prm = reinterpret_cast<PkPos *>(pk_smem + (size_t)d * kPkRows * sizeof(T));  // [d] (16-byte aligned)
     double *cen = reinterpret_cast<double *>(prm + d);                                 // [d]
     for (uint32_t pos = threadIdx.x; pos < d; pos += kPkRows) {
-        const uint32_t dim = grid_dim_at(g, pos);
-        prm[pos] = PkPos{g.off[dim], dim, (g.word[dim] << 8) | g.shift[dim]};
+        if (pos < g.dk) {
+            const uint32_t dim = grid_dim_at(g, pos);
+            prm[pos] = PkPos{g.off[dim], dim, (g.word[dim] << 8) | g.shift[dim]};
+        }
         if (norm_key) cen[pos] = center[pos];
     }
     const uint64_t r0 = (uint64_t)blockIdx.x * kPkRows;
@@ -467,7 +469,7 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
     if (t >= m) return;
     const uint64_t i = r0 + t;
     uint32_t cur_word = 0, acc = 0;
-    for (uint32_t pos = 0; pos < d; ++pos) {
+    for (uint32_t pos = 0; pos < g.dk; ++pos) {
         const PkPos pp = prm[pos];
         const uint32_t w = pp.word_shift >> 8;
         if (w != cur_word) {

@@ -62,3 +62,29 @@ def test_ego_order_is_stable_at_the_sort_s_edges(hj, n, cells):
     want = np.lexsort([cell[:, t] for t in range(x.shape[1] - 1, -1, -1)])
     assert np.array_equal(perm.astype(np.int64), want)
     assert np.array_equal(srt, x[want])
+
+
+@pytest.mark.parametrize("form", ["plain", "fp16", "tf32", "bf16x3"])
+@pytest.mark.parametrize("active", [0, 3, 5])
+@pytest.mark.parametrize("cells", [2, 40, 3000])
+def test_counts_with_a_shortened_key(hj, form, active, cells):
+    """Keys that end before the last dim (one word at these sizes; more where the
+    active dims need them): counts of self-joins, two-set joins, shards and reordered
+    dims equal the oracle's, and ref_compat the reference's convention."""
+    rng = np.random.default_rng(cells)
+    d = 24
+    # clusters, so that neighbours exist in every dim's cells
+    c = rng.random((12, d)) * cells
+    a = (c[rng.integers(0, 12, 1501)] + 0.12 * rng.standard_normal((1501, d))).clip(0, cells)
+    b = (c[rng.integers(0, 12, 1203)] + 0.12 * rng.standard_normal((1203, d))).clip(0, cells)
+    eps = 0.75
+    kw = dict(form=form, active_dims=active)
+    want = O.self_count_brute(a, eps)
+    assert want > 0
+    assert hj.self_join_count(a, eps, **kw) == want
+    assert hj.self_join_count(a, eps, reorder_dims=True, **kw) == want
+    assert sum(hj.self_join_count(a, eps, shard=(k, 3), **kw) for k in range(3)) == want
+    assert hj.join_count(a, b, eps, **kw) == O.join_count_brute(a, b, eps)
+    perm, _ = hj.ego_sort(a, eps)
+    kept = a[perm[:len(a) // 8 * 8].astype(np.int64)]
+    assert hj.self_join_count(a, eps, ref_compat=True, **kw) == O.self_count_brute(kept, eps)
