@@ -404,6 +404,27 @@ struct Prepared {
     std::vector<double> center_host;
 };
 
+// Work list parameters of a distance kernel: the smallest item, the items that keep
+// the SMs balanced (the tensor-core kernel runs one CTA per SM and pays about two
+// tiles per item for its A tile and row data; the plain kernel two CTAs of small
+// tiles), and the operand bytes of the Hilbert rule. A caller's own chunk is kept.
+struct IndexPlan {
+    uint32_t chunk_min, target;
+    uint64_t operand_bytes;
+};
+static IndexPlan index_plan(bool tc, uint32_t own_chunk, int num_sms, const SortedSet &A, const SortedSet &B,
+                            bool self) {
+    auto bytes = [&](const SortedSet &s) -> uint64_t {
+        if (!tc) return hj_ceil_div(s.n, kPlainTile) * kPlainTile * s.d * 8;
+        return s.npad_tc * (s.tf32 ? s.kpad_tf32 * 4ull : s.kpad_bf16 * (s.bf_lo ? 4ull : 2ull));
+    };
+    IndexPlan p;
+    p.chunk_min = own_chunk ? own_chunk : (tc ? 4u : 1u);
+    p.target = (uint32_t)num_sms * (tc ? 8u : 6u);
+    p.operand_bytes = bytes(A) + (self ? 0 : bytes(B));
+    return p;
+}
+
 static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts *opts, int form_override,
                         Prepared *P) {
     int form = form_override >= 0 ? form_override : (opts ? opts->form : HJ_FORM_PLAIN_FP64);
@@ -535,12 +556,14 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
     const bool tc = form_is_tc(form);
     const int tile_a = tc ? kTcTileA : kPlainTile, tile_b = tc ? kTcTileB : kPlainTile;
     // B tiles per work item: 32 x 256 rows (tensor-core forms), 16 x 64 rows (plain), unless set
-    const uint32_t chunk = (opts && opts->item_chunk > 0) ? (uint32_t)opts->item_chunk : (tc ? 32u : 16u);
+    const bool own_chunk = opts && opts->item_chunk > 0;
+    const uint32_t chunk = own_chunk ? (uint32_t)opts->item_chunk : (tc ? 32u : 16u);
+    const IndexPlan plan = index_plan(tc, own_chunk ? chunk : 0, c->num_sms, A, B, in.self);
     IndexResult &idx = P->idx;
     AllocCtx actx{c, st};
     std::string err;
-    int r = build_index(A, B, g, gd, in.self, na_eff, nb_eff, tile_a, tile_b, active_dims, chunk, slot_alloc_cb,
-                        &actx, st, &idx, &launches, &err);
+    int r = build_index(A, B, g, gd, in.self, na_eff, nb_eff, tile_a, tile_b, active_dims, chunk, plan.chunk_min,
+                        plan.target, plan.operand_bytes, slot_alloc_cb, &actx, st, &idx, &launches, &err);
     if (r == 2) return fail(HJ_ERR_OOM, err);
     if (r == 3) return fail(HJ_ERR_CUDA, err);
     if (r) return fail(HJ_ERR_INVALID_ARG, err);
@@ -677,10 +700,13 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
                 // Every item is routed to FP64: the plain form's own work list
                 // (64 x 64 tiles, stripes per 64-rank tile) holds fewer candidate
                 // pairs than the tensor-core one, so it replaces it.
-                const uint32_t chunk = (opts && opts->item_chunk > 0) ? (uint32_t)opts->item_chunk : 16u;
+                const bool own_chunk = opts && opts->item_chunk > 0;
+                const uint32_t chunk = own_chunk ? (uint32_t)opts->item_chunk : 16u;
+                const IndexPlan plan = index_plan(false, own_chunk ? chunk : 0, c->num_sms, A, B, in.self);
                 std::string ierr;
                 int ir = build_index(A, B, P.g, P.gd, in.self, na_eff, nb_eff, kPlainTile, kPlainTile, active_dims,
-                                     chunk, slot_alloc_cb, &actx, st, &idx, &launches, &ierr);
+                                     chunk, plan.chunk_min, plan.target, plan.operand_bytes, slot_alloc_cb, &actx, st,
+                                     &idx, &launches, &ierr);
                 if (ir == 2) return fail(HJ_ERR_OOM, ierr);
                 if (ir) return fail(HJ_ERR_CUDA, ierr);
                 idx_fp = idx;

@@ -22,8 +22,8 @@
 // only: the lexicographic minimum of the lo vectors and the maximum of the
 // (lo_<k, hi_>=k) vectors. So each A tile costs 2 * 3^k binary searches, not
 // 2 * 3^k per point. The ranges are rounded out to B tiles, merged into runs,
-// split into work items of at most `chunk` B tiles, and the items sorted by the
-// Hilbert index of (A tile, B chunk), so that the items that run at the same
+// split into work items of at most `chunk` B tiles, and, where the operands are
+// larger than L2 holds, the items sorted by the Hilbert index of (A tile, B chunk), so that the items that run at the same
 // time on the GPU's SMs share their B tiles in L2 -- the role the Hilbert
 // traversal plays for the CPU caches in the reference.
 #include "hj_common.cuh"
@@ -46,7 +46,7 @@ struct BoundsArgs {
     int self;
     uint2 *runs;       // [n_tiles][kMaxCombos]
     uint32_t *nruns;   // [n_tiles]
-    unsigned long long *cand;  // candidate pairs (tile granularity)
+    unsigned long long *cand;  // candidate pairs (tile granularity), then tile pairs
     uint32_t *lokeys, *hikeys;  // per A row [na][W]: packed digits of cell_lo / cell_hi (k_bound_keys)
 };
 
@@ -118,29 +118,43 @@ __device__ int cmp_up(const BoundsArgs &a, uint64_t p, uint64_t q, uint32_t mw, 
     return 0;
 }
 
-// First index in [0, n) whose key is >= q (strict = 0) or > q (strict = 1).
-// The query is the base words `base` with its first `np` words replaced by `pw`.
-__device__ uint64_t key_search(const uint32_t *__restrict__ keys, uint64_t n, uint32_t W, const uint32_t *base,
-                               const uint32_t *pw, int np, int strict) {
-    uint64_t lo = 0, hi = n;
-    while (lo < hi) {
-        uint64_t mid = lo + ((hi - lo) >> 1);
-        const uint32_t *kr = keys + mid * W;
-        int c = 0;
-        for (uint32_t w = 0; w < W; ++w) {
-            uint32_t kw = __ldg(kr + w);
-            uint32_t qw = (int)w < np ? pw[w] : base[w];
-            if (kw != qw) {
-                c = kw < qw ? -1 : 1;
-                break;
-            }
-        }
-        if (c < 0 || (strict && c == 0))
-            lo = mid + 1;
-        else
-            hi = mid;
+// -1, 0, 1: key row `kr` against the query of base words `base` with its first `np`
+// words replaced by `pw`.
+__device__ __forceinline__ int key_cmp(const uint32_t *__restrict__ kr, uint32_t W, const uint32_t *base,
+                                       const uint32_t *pw, int np) {
+    for (uint32_t w = 0; w < W; ++w) {
+        const uint32_t kw = __ldg(kr + w);
+        const uint32_t qw = (int)w < np ? pw[w] : base[w];
+        if (kw != qw) return kw < qw ? -1 : 1;
     }
-    return lo;
+    return 0;
+}
+
+// The first index in [0, n) whose key is >= the lower query and the first whose key is
+// > the upper query, both searches in step (each is a chain of dependent reads).
+__device__ void key_range(const uint32_t *__restrict__ keys, uint64_t n, uint32_t W, const uint32_t *blo,
+                          const uint32_t *plo, const uint32_t *bhi, const uint32_t *phi, int np, uint64_t *first,
+                          uint64_t *last) {
+    uint64_t l0 = 0, h0 = n, l1 = 0, h1 = n;
+    while (l0 < h0 || l1 < h1) {
+        const uint64_t m0 = l0 + ((h0 - l0) >> 1), m1 = l1 + ((h1 - l1) >> 1);
+        const int c0 = l0 < h0 ? key_cmp(keys + m0 * W, W, blo, plo, np) : 0;
+        const int c1 = l1 < h1 ? key_cmp(keys + m1 * W, W, bhi, phi, np) : 0;
+        if (l0 < h0) {
+            if (c0 < 0)
+                l0 = m0 + 1;
+            else
+                h0 = m0;
+        }
+        if (l1 < h1) {
+            if (c1 <= 0)
+                l1 = m1 + 1;
+            else
+                h1 = m1;
+        }
+    }
+    *first = l0;
+    *last = l1;
 }
 
 constexpr int kBoundsWarps = 4;
@@ -225,60 +239,112 @@ __global__ void __launch_bounds__(kBoundsWarps * 32) k_tile_bounds(BoundsArgs a,
             pl[w] = (pl[w] & ~(mask << sh)) | (vl << sh);
             ph[w] = (ph[w] & ~(mask << sh)) | (vh << sh);
         }
-        uint64_t lower = key_search(a.bkeys, a.nb, a.W, qlo, pl, np, 0);
-        uint64_t upper = key_search(a.bkeys, a.nb, a.W, qhi, ph, np, 1);
+        uint64_t lower, upper;
+        key_range(a.bkeys, a.nb, a.W, qlo, pl, qhi, ph, np, &lower, &upper);
         if (a.self && lower < p0) lower = p0;
         uint2 v = make_uint2(1u, 0u);  // empty
         if (lower < upper) v = make_uint2((uint32_t)(lower / a.tile_b), (uint32_t)hj_ceil_div(upper, a.tile_b));
         iv[c] = v;
     }
     __syncwarp();
-    // 5. merge the intervals into disjoint runs (lane 0)
+    // 5. merge the intervals into disjoint runs
+    uint2 *out = a.runs + tile * kMaxCombos;
+    uint32_t nr;
+    unsigned long long cols = 0, tp = 0;
+    if (ncomb <= 32) {
+        // in the warp's registers: rank by start (empty intervals last), the largest
+        // end before each, a run wherever an interval starts beyond it. (One lane
+        // sorting and merging was most of the kernel at a few hundred tiles.)
+        uint2 v = lane < ncomb ? iv[lane] : make_uint2(1u, 0u);
+        const unsigned long long k = v.x < v.y ? ((unsigned long long)v.x << 32 | lane) : ~0ull - 31 + lane;
+        int rank = 0;
+        for (int o = 0; o < 32; ++o) rank += __shfl_sync(0xffffffffu, k, o) < k ? 1 : 0;
+        __syncwarp();
+        iv[rank] = v;  // 32 entries of the warp's kMaxCombos
+        __syncwarp();
+        v = iv[lane];
+        const bool some = v.x < v.y;
+        uint32_t end = some ? v.y : 0u;  // inclusive prefix maximum of the ends
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end = max(end, y);
+        }
+        const uint32_t before = __shfl_up_sync(0xffffffffu, end, 1);
+        const bool start = some && (lane == 0 || v.x > before);
+        const uint32_t starts = __ballot_sync(0xffffffffu, start), all = __ballot_sync(0xffffffffu, some);
+        nr = __popc(starts);
+        // the run's end: the prefix maximum at the last interval before the next start
+        const uint32_t later = lane < 31 ? starts & ~((2u << lane) - 1u) : 0u;
+        const int last = later ? __ffs(later) - 2 : (all ? 31 - __clz(all) : 0);
+        const uint32_t run_end = __shfl_sync(0xffffffffu, end, last);
+        if (start) {
+            out[__popc(starts & ((1u << lane) - 1u))] = make_uint2(v.x, run_end);
+            const uint64_t b0 = (uint64_t)v.x * a.tile_b, b1 = hj_umin((uint64_t)run_end * a.tile_b, a.nb);
+            cols = b1 > b0 ? b1 - b0 : 0;
+            tp = run_end - v.x;
+        }
+        cols = warp_sum_u64(cols);
+        tp = warp_sum_u64(tp);
+    } else {
+        nr = 0;
+        if (lane == 0) {
+            int m = 0;
+            for (int c = 0; c < ncomb; ++c)
+                if (iv[c].x < iv[c].y) iv[m++] = iv[c];
+            for (int i = 1; i < m; ++i) {  // insertion sort by start
+                uint2 v = iv[i];
+                int j = i - 1;
+                while (j >= 0 && iv[j].x > v.x) {
+                    iv[j + 1] = iv[j];
+                    --j;
+                }
+                iv[j + 1] = v;
+            }
+            uint2 run = make_uint2(0u, 0u);
+            for (int i = 0; i <= m; ++i) {
+                if (i < m && run.x < run.y && iv[i].x <= run.y) {
+                    run.y = max(run.y, iv[i].y);
+                    continue;
+                }
+                if (run.x < run.y) {
+                    out[nr++] = run;
+                    const uint64_t b0 = (uint64_t)run.x * a.tile_b, b1 = hj_umin((uint64_t)run.y * a.tile_b, a.nb);
+                    cols += b1 > b0 ? b1 - b0 : 0;
+                    tp += run.y - run.x;
+                }
+                if (i < m) run = iv[i];
+            }
+        }
+    }
     if (lane == 0) {
-        int m = 0;
-        for (int c = 0; c < ncomb; ++c)
-            if (iv[c].x < iv[c].y) iv[m++] = iv[c];
-        for (int i = 1; i < m; ++i) {  // insertion sort by start
-            uint2 v = iv[i];
-            int j = i - 1;
-            while (j >= 0 && iv[j].x > v.x) {
-                iv[j + 1] = iv[j];
-                --j;
-            }
-            iv[j + 1] = v;
-        }
-        int r = 0;
-        unsigned long long cols = 0;
-        uint2 *out = a.runs + tile * kMaxCombos;
-        for (int i = 0; i < m; ++i) {
-            if (r > 0 && iv[i].x <= out[r - 1].y) {
-                out[r - 1].y = max(out[r - 1].y, iv[i].y);
-            } else {
-                out[r++] = iv[i];
-            }
-        }
-        for (int i = 0; i < r; ++i) {
-            uint64_t b0 = (uint64_t)out[i].x * a.tile_b, b1 = hj_umin((uint64_t)out[i].y * a.tile_b, a.nb);
-            cols += b1 > b0 ? b1 - b0 : 0;
-        }
-        a.nruns[tile] = (uint32_t)r;
-        atomicAdd(a.cand, cols * (p1 - p0));
+        a.nruns[tile] = nr;
+        if (cols) atomicAdd(a.cand, cols * (p1 - p0));
+        if (tp) atomicAdd(a.cand + 1, tp);
     }
 }
 
+// B tiles per work item: `chunk`, less where the join has too few tile pairs for
+// `target` items of that size, so that every SM has several items to balance with
+// (1500 x 8: 32 items of up to 16 tiles kept 32 of the 148 SMs busy, 31 -> 15 us).
+__host__ __device__ inline uint32_t item_chunk(unsigned long long tile_pairs, uint32_t chunk, uint32_t chunk_min,
+                                               uint32_t target) {
+    const unsigned long long c = tile_pairs / target;
+    return c >= chunk ? chunk : (c > chunk_min ? (uint32_t)c : chunk_min);
+}
+
 __global__ void k_item_counts(const uint2 *__restrict__ runs, const uint32_t *__restrict__ nruns, uint64_t n_tiles,
-                              uint32_t chunk, uint32_t *counts, unsigned long long *tile_pairs) {
+                              uint32_t chunk, uint32_t chunk_min, uint32_t target, uint32_t *counts,
+                              const unsigned long long *__restrict__ tile_pairs) {
     uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_tiles) return;
+    const uint32_t ch = item_chunk(*tile_pairs, chunk, chunk_min, target);
     uint32_t c = 0;
-    unsigned long long tp = 0;
     for (uint32_t i = 0; i < nruns[t]; ++i) {
         uint2 r = runs[t * kMaxCombos + i];
-        c += (uint32_t)hj_ceil_div(r.y - r.x, chunk);
-        tp += r.y - r.x;
+        c += (uint32_t)hj_ceil_div(r.y - r.x, ch);
     }
     counts[t] = c;
-    if (tp) atomicAdd(tile_pairs, tp);
 }
 
 // Hilbert index of (x, y) on a side-`side` grid (side a power of two); the
@@ -302,31 +368,33 @@ __device__ __forceinline__ unsigned long long hilbert_index(unsigned long long s
     return dd;
 }
 
-__global__ void k_item_write(const uint2 *__restrict__ runs, const uint32_t *__restrict__ nruns,
-                             const uint32_t *__restrict__ offsets, uint64_t n_tiles, uint32_t chunk,
-                             unsigned long long side, uint32_t key_words, WorkItem *items, uint32_t *keys_wm,
-                             uint64_t n_items) {
-    uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per A tile, lanes over the chunks of each run. keys_wm null: the items stay
+// in order of (A tile, B chunk).
+__global__ void __launch_bounds__(256) k_item_write(const uint2 *__restrict__ runs,
+                                                    const uint32_t *__restrict__ nruns,
+                                                    const uint32_t *__restrict__ offsets, uint64_t n_tiles,
+                                                    uint32_t chunk, unsigned long long side, uint32_t key_words,
+                                                    WorkItem *items, uint32_t *keys_wm, uint64_t n_items) {
+    const uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
     if (t >= n_tiles) return;
     uint64_t o = offsets[t];
     for (uint32_t i = 0; i < nruns[t]; ++i) {
-        uint2 r = runs[t * kMaxCombos + i];
-        for (uint32_t b = r.x; b < r.y; b += chunk) {
-            WorkItem it;
-            it.a = (uint32_t)t;
-            it.b0 = b;
-            it.b1 = min(b + chunk, r.y);
-            it.pad = 0;
-            items[o] = it;
-            unsigned long long h = hilbert_index(side, t, b / chunk);
+        const uint2 r = runs[t * kMaxCombos + i];
+        const uint32_t nc = (uint32_t)hj_ceil_div(r.y - r.x, chunk);
+        for (uint32_t k = lane; k < nc; k += 32) {
+            const uint32_t b = r.x + k * chunk;
+            items[o + k] = WorkItem{(uint32_t)t, b, min(b + chunk, r.y), 0};
+            if (!keys_wm) continue;
+            const unsigned long long h = hilbert_index(side, t, b / chunk);
             if (key_words == 1) {
-                keys_wm[o] = (uint32_t)h;
+                keys_wm[o + k] = (uint32_t)h;
             } else {
-                keys_wm[o] = (uint32_t)(h >> 32);          // word 0: most significant
-                keys_wm[n_items + o] = (uint32_t)h;        // word 1
+                keys_wm[o + k] = (uint32_t)(h >> 32);      // word 0: most significant
+                keys_wm[n_items + o + k] = (uint32_t)h;    // word 1
             }
-            ++o;
         }
+        o += nc;
     }
 }
 
@@ -489,8 +557,17 @@ int split_items_by_precision(const IndexResult &in, const SortedSet &A, const So
     return 0;
 }
 
+// Lists up to this many items over operands of up to so many bytes (both sets) keep
+// the order of (A tile, B chunk): the operands stay in the 126 MB L2 whatever the
+// order, and the sort, the gather and their launches were 15 to 20 us of joins of
+// 0.5 to 3 ms. Longer lists are sorted also where L2 holds the operands: in Hilbert
+// order a CTA's share of the tiles that are full of near pairs is even (200k x 64,
+// 20k items: kernel 3.69 ms, 3.87 unsorted).
+constexpr uint64_t kHilbertMinItems = 8192, kHilbertMinBytes = 64ull << 20;
+
 int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const GridDev &gdev, bool self,
                 uint64_t na_eff, uint64_t nb_eff, int tile_a, int tile_b, int active_dims, uint32_t chunk,
+                uint32_t chunk_min, uint32_t target, uint64_t operand_bytes,
                 void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, cudaStream_t st, IndexResult *out,
                 int *launches, std::string *err) {
     *out = IndexResult();
@@ -534,8 +611,8 @@ int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const 
     size_t smem = (size_t)kBoundsWarps * (2 * grid.W + 2 * kMaxCombos) * sizeof(uint32_t);
     if (smem > 48 * 1024) ensure_max_dynamic_smem((const void *)k_tile_bounds, (int)smem);
     k_tile_bounds<<<(unsigned)hj_ceil_div(n_tiles, kBoundsWarps), kBoundsWarps * 32, smem, st>>>(ba, n_tiles);
-    k_item_counts<<<(unsigned)hj_ceil_div(n_tiles, 256), 256, 0, st>>>(runs, nruns, n_tiles, chunk, counts,
-                                                                     stats + 1);
+    k_item_counts<<<(unsigned)hj_ceil_div(n_tiles, 256), 256, 0, st>>>(runs, nruns, n_tiles, chunk, chunk_min, target,
+                                                                     counts, stats + 1);
     launch_scan_u32(counts, n_tiles, stats + 2, st,
                     (unsigned long long *)alloc(actx, kSlotScanTiles, scan_scratch_bytes(n_tiles)));
     unsigned long long hstats[4];
@@ -551,9 +628,22 @@ int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const 
     out->tile_pairs = hstats[1];
     out->n_items = n_items;
     if (n_items == 0) return 0;
+    chunk = item_chunk(hstats[1], chunk, chunk_min, target);
     if (n_items >= (1ull << 31)) {
         *err = "work list too large";
         return 1;
+    }
+    WorkItem *items = (WorkItem *)alloc(actx, kSlotItems, n_items * sizeof(WorkItem));
+    if (!items) {
+        *err = "out of device memory (work list)";
+        return 2;
+    }
+    const unsigned write_blocks = (unsigned)hj_ceil_div(n_tiles, 8);
+    if (n_items <= kHilbertMinItems && operand_bytes <= kHilbertMinBytes) {
+        k_item_write<<<write_blocks, 256, 0, st>>>(runs, nruns, counts, n_tiles, chunk, 0, 0, items, nullptr, n_items);
+        if (launches) *launches += 1;
+        out->items = items;
+        return 0;
     }
     unsigned long long side = 1;
     const uint64_t n_chunks_b = hj_ceil_div(hj_ceil_div(B.n, tile_b), chunk) + 1;
@@ -562,16 +652,14 @@ int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const 
     while ((1ull << hbits) < side * side) ++hbits;
     const uint32_t key_words = hbits > 32 ? 2 : 1;
     WorkItem *tmp = (WorkItem *)alloc(actx, kSlotItemsTmp, n_items * sizeof(WorkItem));
-    WorkItem *items = (WorkItem *)alloc(actx, kSlotItems, n_items * sizeof(WorkItem));
     uint32_t *keys = (uint32_t *)alloc(actx, kSlotItemKeys, n_items * key_words * sizeof(uint32_t));
     uint32_t *perm = (uint32_t *)alloc(actx, kSlotItemPerm, n_items * sizeof(uint32_t));
     void *rs = alloc(actx, kSlotItemHist, radix_scratch_bytes(n_items));
-    if (!tmp || !items || !keys || !perm || !rs) {
+    if (!tmp || !keys || !perm || !rs) {
         *err = "out of device memory (work list)";
         return 2;
     }
-    k_item_write<<<(unsigned)hj_ceil_div(n_tiles, 256), 256, 0, st>>>(runs, nruns, counts, n_tiles, chunk, side,
-                                                                     key_words, tmp, keys, n_items);
+    k_item_write<<<write_blocks, 256, 0, st>>>(runs, nruns, counts, n_tiles, chunk, side, key_words, tmp, keys, n_items);
     std::vector<std::pair<uint32_t, uint32_t>> passes;
     if (key_words == 1) {
         for (int b = 0; b < hbits; b += 8) passes.push_back({0u, (uint32_t)b});

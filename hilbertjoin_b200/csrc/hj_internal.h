@@ -284,11 +284,14 @@ void launch_gather(const void *x, int dtype_bytes, uint64_t n, uint32_t d, const
                    int *launches);
 
 // Index stage: per A tile the stripe ranges into B's EGO order, merged into
-// runs of B tiles; expanded into work items of at most `chunk` B tiles and
-// sorted in Hilbert order. Synchronises once on `st` (item count).
+// runs of B tiles; expanded into work items of at most `chunk` B tiles (down to
+// chunk_min where that gives fewer than `target` items), and sorted in Hilbert order
+// where the operands (operand_bytes, both sets) exceed what L2 holds. Synchronises
+// once on `st` (item count).
 struct IndexScratch;
 int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const GridDev &gdev, bool self,
                 uint64_t na_eff, uint64_t nb_eff, int tile_a, int tile_b, int active_dims, uint32_t chunk,
+                uint32_t chunk_min, uint32_t target, uint64_t operand_bytes,
                 void *(*alloc)(void *ctx, int slot, size_t bytes), void *alloc_ctx, cudaStream_t st,
                 IndexResult *out, int *launches, std::string *err);
 
