@@ -276,7 +276,7 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
             parts.push_back({w, P.idx_tc.n_items});
             n_items += P.idx_tc.n_items;
         }
-        b->candidate_pairs += P.idx_tc.candidate_pairs;
+        b->candidate_pairs += P.idx_tc.candidate_pairs + P.idx_fp.candidate_pairs;
         b->job_candidates[j] = P.idx_tc.candidate_pairs + P.idx_fp.candidate_pairs;
         // items routed to the FP64 kernel keep their own plain tiles
         if (P.idx_fp.n_items) {

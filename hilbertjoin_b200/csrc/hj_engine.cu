@@ -36,6 +36,11 @@ static int fail(int code, const std::string &msg) {
 
 // ------------------------------------------------------------------ context
 
+// Per-dim host tables of one call, in order: key offsets and centre (8 bytes a dim),
+// bits, word, shift and dim order (4 each); behind them the DimStats read back.
+constexpr size_t kTabBytesPerDim = 2 * 8 + 4 * 4;
+constexpr size_t kTabBytes = kTabBytesPerDim * kMaxDim;
+
 struct Ctx {
     int device = -1;
     cudaStream_t stream = nullptr;
@@ -43,9 +48,10 @@ struct Ctx {
     std::vector<std::pair<void *, size_t>> slots;
     cudaEvent_t ev[8] = {};
     unsigned long long *d_small = nullptr;  // [16] counters
-    unsigned long long *h_small = nullptr;  // pinned [16]
+    unsigned long long *h_small = nullptr;  // pinned [16]: [0, 8) as d_small, [8, 12) index, [12, 14) split
     TcJob *h_job = nullptr;                 // pinned: the job table of a single join
     TcJob *d_job = nullptr;
+    unsigned char *h_tab = nullptr;  // pinned: per-dim tables of a call (kTabBytes), then its statistics
     bool ok = false;
 };
 
@@ -122,7 +128,8 @@ static int get_ctx(int device, Ctx **out) {
     cudaMallocHost(&c->h_small, 16 * sizeof(unsigned long long));
     cudaMallocHost(&c->h_job, sizeof(TcJob));
     cudaMalloc(&c->d_job, sizeof(TcJob));
-    if (!c->d_small || !c->h_small || !c->h_job || !c->d_job) return fail(HJ_ERR_OOM, "context allocation failed");
+    cudaMallocHost(&c->h_tab, kTabBytes + kMaxDim * sizeof(DimStats) + 16);
+    if (!c->d_small || !c->h_small || !c->h_job || !c->d_job || !c->h_tab) return fail(HJ_ERR_OOM, "context allocation failed");
     c->ok = true;
     tl_ctx[dev] = c;
     *out = c;
@@ -156,7 +163,7 @@ static int bitwidth(unsigned long long v) {
 // with the last word that `min_dims` and `min_bits` need (0xffffffff: every dim has
 // a field): a key over the first dims in order is the EGO order of those dims, for
 // which the stripe search is complete, too.
-static int plan_grid(const std::vector<DimStats> &ds, uint32_t d, double eps, double maxabs,
+static int plan_grid(const DimStats *ds, uint32_t d, double eps, double maxabs,
                      const std::vector<uint32_t> &ord, uint32_t min_dims, uint32_t min_bits, Grid *g) {
     g->d = d;
     g->ord = ord;
@@ -401,7 +408,7 @@ struct Prepared {
     int launches = 0;
     double reorder_ms = 0;
     double op_scale = 1.0;  // FP16 form: operand scale 2^s
-    std::vector<double> center_host;
+    double norm_max = 0;    // at least every centred squared norm (from the dims' ranges)
 };
 
 // Work list parameters of a distance kernel: the smallest item, the items that keep
@@ -440,28 +447,45 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
 
     const uint32_t d = in.d;
     // 1. per-dim cell ranges (union of both sets), read back to plan the keys
-    DimStats *ds = (DimStats *)slot_alloc_impl(c, st, kSlotDimStats, d * sizeof(DimStats));
+    // (with max |x| and the error bits behind them: one copy)
+    DimStats *ds = (DimStats *)slot_alloc_impl(c, st, kSlotDimStats, d * sizeof(DimStats) + 16);
     if (!ds) return fail(HJ_ERR_OOM, "out of device memory");
-    unsigned long long *d_maxabs = c->d_small + 0;
-    uint32_t *d_bad = reinterpret_cast<uint32_t *>(c->d_small + 1);
+    unsigned long long *d_maxabs = reinterpret_cast<unsigned long long *>(ds + d);
+    uint32_t *d_bad = reinterpret_cast<uint32_t *>(d_maxabs + 1);
+    const bool reorder = opts && opts->reorder_dims && d > 1;
     launch_dim_stats_init(ds, d, d_maxabs, d_bad, st);
-    launch_dim_stats(in.a, in.dtype_bytes, in.na, d, in.eps, ds, d_maxabs, d_bad, st);
+    launch_dim_stats(in.a, in.dtype_bytes, in.na, d, in.eps, ds, d_maxabs, d_bad, st, false);
     launches += 2;
     if (!in.self) {
-        launch_dim_stats(in.b, in.dtype_bytes, in.nb, d, in.eps, ds, d_maxabs, d_bad, st);
+        launch_dim_stats(in.b, in.dtype_bytes, in.nb, d, in.eps, ds, d_maxabs, d_bad, st, false);
         ++launches;
     }
-    std::vector<DimStats> hds(d);
-    cudaMemcpyAsync(hds.data(), ds, d * sizeof(DimStats), cudaMemcpyDeviceToHost, st);
-    cudaMemcpyAsync(c->h_small, c->d_small, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+    if (reorder) {  // the dimension cost reads the cells on the device
+        launch_dim_stats_cells(ds, d, in.eps, d_bad, st);
+        ++launches;
+    }
+    DimStats *hds = reinterpret_cast<DimStats *>(c->h_tab + kTabBytes);
+    const unsigned long long *h_max = reinterpret_cast<const unsigned long long *>(hds + d);
+    cudaMemcpyAsync(hds, ds, d * sizeof(DimStats) + 16, cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("cell statistics");
     if (int r = check_cuda("cell statistics")) return r;
-    const uint32_t bad = (uint32_t)c->h_small[1];
+    uint32_t bad = (uint32_t)h_max[1];
+    for (uint32_t t = 0; t < d && !reorder; ++t) {  // as k_dim_stats_cells
+        if (hds[t].xmin == ~0ull) continue;
+        const double lo = std::floor(double_from_ordered(hds[t].xmin) / in.eps),
+                     hi = std::floor(double_from_ordered(hds[t].xmax) / in.eps);
+        if (!(std::fabs(lo) < kCellLimit) || !(std::fabs(hi) < kCellLimit)) {
+            bad |= 2u;
+            continue;
+        }
+        hds[t].cmin = (long long)lo;
+        hds[t].cmax = (long long)hi;
+    }
     if (bad & 1u) return fail(HJ_ERR_INVALID_ARG, "input holds a non-finite coordinate");
     if (bad & 2u) return fail(HJ_ERR_INVALID_ARG, "a cell index floor(x/eps) exceeds 2^62");
     double maxabs;
     {
-        unsigned long long bits = c->h_small[0];
+        unsigned long long bits = h_max[0];
         std::memcpy(&maxabs, &bits, 8);
     }
     if (form == HJ_FORM_AUTO) {
@@ -476,7 +500,7 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
     if (form_is_tc(form) && !(maxabs < 1e18)) return fail(HJ_ERR_UNSUPPORTED, "tensor-core forms need |x| < 1e18");
     if (form == HJ_FORM_PLAIN_FP64 && d > 256) return fail(HJ_ERR_UNSUPPORTED, "plain FP64 form supports d <= 256");
     std::vector<uint32_t> ord;
-    if (opts && opts->reorder_dims && d > 1) {
+    if (reorder) {
         auto t0 = std::chrono::steady_clock::now();
         std::vector<unsigned long long> costs;
         if (int r = dim_order_by_cost(c, st, in.a, in.dtype_bytes, in.na, d, in.eps, ds, &ord, &costs)) return r;
@@ -489,27 +513,27 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
     if (int r = plan_grid(hds, d, in.eps, maxabs, ord, min_dims, min_bits, &g)) return r;
     GridDev &gd = P->gd;
     gd.dk = g.dk;
-    if (!ord.empty()) {
-        gd.ord = (uint32_t *)slot_alloc_impl(c, st, kSlotGridOrd, d * 4);
-        if (!gd.ord) return fail(HJ_ERR_OOM, "out of device memory");
-        cudaMemcpyAsync(gd.ord, g.ord.data(), d * 4, cudaMemcpyHostToDevice, st);
-    }
-    gd.off = (long long *)slot_alloc_impl(c, st, kSlotGridOff, d * 8);
-    gd.bits = (uint32_t *)slot_alloc_impl(c, st, kSlotGridBits, d * 4);
-    gd.word = (uint32_t *)slot_alloc_impl(c, st, kSlotGridWord, d * 4);
-    gd.shift = (uint32_t *)slot_alloc_impl(c, st, kSlotGridShift, d * 4);
-    if (!gd.off || !gd.bits || !gd.word || !gd.shift) return fail(HJ_ERR_OOM, "out of device memory");
-    cudaMemcpyAsync(gd.off, g.off.data(), d * 8, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(gd.bits, g.bits.data(), d * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(gd.word, g.word.data(), d * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(gd.shift, g.shift.data(), d * 4, cudaMemcpyHostToDevice, st);
+    // one device table, filled by one copy from pinned memory (the copy of the call
+    // before has been waited for)
+    unsigned char *tab = (unsigned char *)slot_alloc_impl(c, st, kSlotGridOff, kTabBytesPerDim * d);
+    if (!tab) return fail(HJ_ERR_OOM, "out of device memory");
+    const size_t o_bits = 16ull * d, o_word = o_bits + 4ull * d, o_shift = o_word + 4ull * d, o_ord = o_shift + 4ull * d;
+    gd.off = reinterpret_cast<long long *>(tab);
+    double *center = reinterpret_cast<double *>(tab + 8ull * d);
+    gd.bits = reinterpret_cast<uint32_t *>(tab + o_bits);
+    gd.word = reinterpret_cast<uint32_t *>(tab + o_word);
+    gd.shift = reinterpret_cast<uint32_t *>(tab + o_shift);
+    if (!ord.empty()) gd.ord = reinterpret_cast<uint32_t *>(tab + o_ord);
+    std::memcpy(c->h_tab, g.off.data(), d * 8);
+    std::memcpy(c->h_tab + o_bits, g.bits.data(), d * 4);
+    std::memcpy(c->h_tab + o_word, g.word.data(), d * 4);
+    std::memcpy(c->h_tab + o_shift, g.shift.data(), d * 4);
+    std::memcpy(c->h_tab + o_ord, g.ord.data(), d * 4);
 
     // per-dim midpoint of the coordinate range: the shift of the tensor-core operands
-    double *center = (double *)slot_alloc_impl(c, st, kSlotCenter, d * 8);
-    if (!center) return fail(HJ_ERR_OOM, "out of device memory");
     double norm_scale = 0.0;
     {
-        std::vector<double> hc(d);
+        double *hc = reinterpret_cast<double *>(c->h_tab + 8ull * d);
         double nmax = 0.0;
         for (uint32_t t = 0; t < d; ++t) {
             if (hds[t].cmin > hds[t].cmax) {
@@ -530,8 +554,8 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
             rmax = std::fmax(rmax, std::fmax(hi - hc[t], hc[t] - lo));
         }
         P->op_scale = rmax > 0 ? std::ldexp(1.0, 14 - std::ilogb(rmax)) : 1.0;
-        P->center_host = hc;  // outlives the asynchronous copy (the join synchronises later)
-        cudaMemcpyAsync(center, P->center_host.data(), d * 8, cudaMemcpyHostToDevice, st);
+        P->norm_max = nmax * 1.001;
+        cudaMemcpyAsync(tab, c->h_tab, kTabBytesPerDim * d, cudaMemcpyHostToDevice, st);
     }
 
     // 2. EGO sort + layouts
@@ -563,7 +587,8 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
     AllocCtx actx{c, st};
     std::string err;
     int r = build_index(A, B, g, gd, in.self, na_eff, nb_eff, tile_a, tile_b, active_dims, chunk, plan.chunk_min,
-                        plan.target, plan.operand_bytes, slot_alloc_cb, &actx, st, &idx, &launches, &err);
+                        plan.target, plan.operand_bytes, slot_alloc_cb, &actx,
+                        c->h_small + 8, st, &idx, &launches, &err);
     if (r == 2) return fail(HJ_ERR_OOM, err);
     if (r == 3) return fail(HJ_ERR_CUDA, err);
     if (r) return fail(HJ_ERR_INVALID_ARG, err);
@@ -585,6 +610,30 @@ static int prepare_join(Ctx *c, cudaStream_t st, const JoinIn &in, const hj_opts
     P->nb_eff = nb_eff;
     P->launches = launches;
     return HJ_OK;
+}
+
+// The plain form's work list over sets prepared for a tensor-core form: 64 x 64 tiles
+// with stripes per 64-rank tile hold fewer candidate pairs than the tensor-core
+// items cut into 64-rank pieces.
+static int plain_work_list(Ctx *c, cudaStream_t st, const SortedSet &A, const SortedSet &B, const Prepared &P, bool self,
+                           const hj_opts *opts, IndexResult *idx, int *launches) {
+    const bool own_chunk = opts && opts->item_chunk > 0;
+    const uint32_t chunk = own_chunk ? (uint32_t)opts->item_chunk : 16u;
+    const IndexPlan plan = index_plan(false, own_chunk ? chunk : 0, c->num_sms, A, B, self);
+    AllocCtx actx{c, st};
+    std::string err;
+    const int r = build_index(A, B, P.g, P.gd, self, P.na_eff, P.nb_eff, kPlainTile, kPlainTile, P.active_dims, chunk,
+                              plan.chunk_min, plan.target, plan.operand_bytes, slot_alloc_cb, &actx, c->h_small + 8, st,
+                              idx, launches, &err);
+    if (r == 2) return fail(HJ_ERR_OOM, err);
+    return r ? fail(HJ_ERR_CUDA, err) : HJ_OK;
+}
+
+// Whether the error bound of every pair is within `limit`, from a bound on the norms
+// (operand units; the FP32 norms' rounding is within the margin): then no item needs
+// its own check.
+static bool all_within(double c_rel, double c_abs, double norm_max, double limit) {
+    return c_rel * 2.0 * norm_max * 1.0001 + c_abs <= limit;
 }
 
 static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *count, hj_stats *stats,
@@ -613,7 +662,8 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
     unsigned long long *d_band = c->d_small + 4;
     unsigned long long *d_count_fp = c->d_small + 6;
     unsigned long long *d_band_holes = c->d_small + 7;  // band slots reserved but left unused
-    cudaMemsetAsync(c->d_small + 2, 0, 5 * sizeof(unsigned long long), st);
+    cudaMemsetAsync(c->d_small + 2, 0, 6 * sizeof(unsigned long long), st);
+    bool read_back = false;  // d_small has been read and the stream waited for
     uint64_t band_total = 0, band_holes = 0, fp_items = 0;
     double c_rel = 0, c_abs = 0;
     bool bc = false;  // per-block-centred operands (tensor-core forms)
@@ -678,37 +728,33 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
             return attempt > 0 ? -1.0 : bc ? 4.0 * T * bc_scale * bc_scale : 0.5 * T_tc;
         };
         for (int attempt = 0;; ++attempt) {
-            int sr = split_items_by_precision(idx, A, B, c_rel, c_abs, route_limit(attempt), bc ? &bck : nullptr,
-                                              slot_alloc_cb, &actx, st, &idx_tc, &idx_fp);
+            int sr = 0;
+            if (attempt == 0 && !bc && all_within(c_rel, c_abs, P.norm_max * A.op_scale * A.op_scale, route_limit(0))) {
+                idx_tc = idx;  // every item's bound is within the limit: nothing to split
+                idx_fp = IndexResult();
+            } else {
+                sr = split_items_by_precision(idx, A, B, c_rel, c_abs, route_limit(attempt), bc ? &bck : nullptr,
+                                              slot_alloc_cb, &actx, c->h_small + 12, st, &idx_tc, &idx_fp);
+                launches += 2;
+            }
             if (sr == 2) return fail(HJ_ERR_OOM, "out of device memory (work list split)");
             if (sr) return check_cuda("work list split");
-            launches += 2;
             if (attempt == 0 && !bc && bc_ok && centring == HJ_CENTRING_AUTO &&
                 idx_fp.tile_pairs * 8 > idx.tile_pairs) {
                 // the split synchronised the stream: the job's first copy is done
                 if (int r = enable_bc()) return r;
                 fill_job();
                 sr = split_items_by_precision(idx, A, B, c_rel, c_abs, route_limit(attempt), &bck, slot_alloc_cb,
-                                              &actx, st, &idx_tc, &idx_fp);
+                                              &actx, c->h_small + 12, st, &idx_tc, &idx_fp);
                 if (sr == 2) return fail(HJ_ERR_OOM, "out of device memory (work list split)");
                 if (sr) return check_cuda("work list split");
                 launches += 2;
             }
             fp_items = idx_fp.n_items;
-            cudaMemsetAsync(c->d_small + 2, 0, 5 * sizeof(unsigned long long), st);
+            if (attempt) cudaMemsetAsync(c->d_small + 2, 0, 6 * sizeof(unsigned long long), st);
             if (attempt == 0 && idx_tc.n_items == 0 && idx_fp.n_items && !(opts && opts->shard_count > 1)) {
                 // Every item is routed to FP64: the plain form's own work list
-                // (64 x 64 tiles, stripes per 64-rank tile) holds fewer candidate
-                // pairs than the tensor-core one, so it replaces it.
-                const bool own_chunk = opts && opts->item_chunk > 0;
-                const uint32_t chunk = own_chunk ? (uint32_t)opts->item_chunk : 16u;
-                const IndexPlan plan = index_plan(false, own_chunk ? chunk : 0, c->num_sms, A, B, in.self);
-                std::string ierr;
-                int ir = build_index(A, B, P.g, P.gd, in.self, na_eff, nb_eff, kPlainTile, kPlainTile, active_dims,
-                                     chunk, plan.chunk_min, plan.target, plan.operand_bytes, slot_alloc_cb, &actx, st,
-                                     &idx, &launches, &ierr);
-                if (ir == 2) return fail(HJ_ERR_OOM, ierr);
-                if (ir) return fail(HJ_ERR_CUDA, ierr);
+                if (int ir = plain_work_list(c, st, A, B, P, in.self, opts, &idx, &launches)) return ir;
                 idx_fp = idx;
             }
             if (idx_fp.n_items) {
@@ -736,9 +782,11 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
             for (int grow = 0; grow < 4; ++grow) {
                 uint2 *band = (uint2 *)slot_alloc_impl(c, st, kSlotBand, cap * kBandEntryBytes);
                 if (!band) return fail(HJ_ERR_OOM, "out of device memory (band queue)");
-                cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st);
-                cudaMemsetAsync(d_band, 0, 2 * sizeof(unsigned long long), st);
-                cudaMemsetAsync(d_band_holes, 0, sizeof(unsigned long long), st);
+                if (grow) {
+                    cudaMemsetAsync(d_count, 0, sizeof(unsigned long long), st);
+                    cudaMemsetAsync(d_band, 0, 2 * sizeof(unsigned long long), st);
+                    cudaMemsetAsync(d_band_holes, 0, sizeof(unsigned long long), st);
+                }
                 std::string terr;
                 cudaEventRecord(c->ev[6], st);
                 if (launch_join_tc(A, B, form, c->d_job, na_eff, nb_eff, idx_tc, band, cap, d_band, d_err,
@@ -746,20 +794,23 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
                     return fail(HJ_ERR_CUDA, terr);
                 ++launches;
                 cudaEventRecord(c->ev[4], st);
-                cudaMemcpyAsync(c->h_small + 4, d_band, 8, cudaMemcpyDeviceToHost, st);
-                cudaMemcpyAsync(c->h_small + 7, d_band_holes, 8, cudaMemcpyDeviceToHost, st);
+                // The recheck reads the band's size on the device (entries beyond the queue
+                // are not there), so it follows at once, and one read-back tells whether
+                // the band fitted; if not, its counts are reset with the rest.
+                // sorted rows: slot buffers (256-byte aligned) of n rows of d coordinates
+                const bool vec_rows = ((uint64_t)d * A.dtype_bytes) % 16 == 0 &&
+                                      ((uintptr_t)A.rows & 15u) == 0 && ((uintptr_t)B.rows & 15u) == 0;
+                launch_recheck(c->d_job, A.dtype_bytes, band, d_band, cap,
+                               reinterpret_cast<unsigned int *>(c->d_small + 5), st, vec_rows);
+                ++launches;
+                cudaEventRecord(c->ev[5], st);
+                cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                st);
                 if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("tensor-core join");
                 band_total = c->h_small[4];
                 band_holes = c->h_small[7];
-                if (band_total <= cap) {
-                    // sorted rows: slot buffers (256-byte aligned) of n rows of d coordinates
-                    const bool vec_rows = ((uint64_t)d * A.dtype_bytes) % 16 == 0 &&
-                                          ((uintptr_t)A.rows & 15u) == 0 && ((uintptr_t)B.rows & 15u) == 0;
-                    launch_recheck(c->d_job, A.dtype_bytes, band, d_band, cap,
-                                   reinterpret_cast<unsigned int *>(c->d_small + 5), st, vec_rows);
-                    ++launches;
-                    cudaEventRecord(c->ev[5], st);
-                    done = true;
+                if (band_total <= cap || (uint32_t)c->h_small[3]) {  // (or the error word is set: reported below)
+                    done = read_back = true;
                     break;
                 }
                 if (band_total > cap_limit) {  // band too wide to be worth rechecking
@@ -772,8 +823,10 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
             if (!fallback || attempt >= 1) return fail(HJ_ERR_BAND_OVERFLOW, "band queue overflow");
         }
     }
-    cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("distance kernel");
+    if (!read_back) {
+        cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 5 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("distance kernel");
+    }
     if (int rr = check_cuda("distance kernel")) return rr;
     const uint32_t kerr = (uint32_t)c->h_small[3];
     if (kerr & kErrTimeout) {
@@ -1025,7 +1078,7 @@ static int ego_sort_host(const double *pts, uint64_t n, uint32_t d, double eps, 
     double maxabs;
     std::memcpy(&maxabs, &c->h_small[0], 8);
     Grid g;
-    if (int r = plan_grid(hds, d, eps, maxabs, {}, 0xffffffffu, 0xffffffffu, &g)) return r;
+    if (int r = plan_grid(hds.data(), d, eps, maxabs, {}, 0xffffffffu, 0xffffffffu, &g)) return r;
     GridDev gd;
     gd.dk = g.dk;
     gd.off = (long long *)slot_alloc_impl(c, st, kSlotGridOff, d * 8);
@@ -1181,11 +1234,20 @@ int engine_prepare_job(cudaStream_t st_in, const void *a, const void *b, uint64_
     tc_band_constants(P.form, d, P.maxabs, P.A.fold, &J.c_rel, &J.c_abs);
     const double T_tc = eps * eps * J.op_scale * J.op_scale;
     AllocCtx actx{c, st};
-    int sr = split_items_by_precision(P.idx, J.A, J.B, J.c_rel, J.c_abs, 0.5 * T_tc, nullptr, slot_alloc_cb, &actx,
-                                      st, &J.idx_tc, &J.idx_fp);
-    if (sr == 2) return fail(HJ_ERR_OOM, "out of device memory (work list split)");
-    if (sr) return check_cuda("work list split");
-    launches += 2;
+    if (all_within(J.c_rel, J.c_abs, P.norm_max * J.op_scale * J.op_scale, 0.5 * T_tc)) {
+        J.idx_tc = P.idx;
+    } else {
+        int sr = split_items_by_precision(P.idx, J.A, J.B, J.c_rel, J.c_abs, 0.5 * T_tc, nullptr, slot_alloc_cb, &actx,
+                                          c->h_small + 12, st, &J.idx_tc, &J.idx_fp);
+        if (sr == 2) return fail(HJ_ERR_OOM, "out of device memory (work list split)");
+        if (sr) return check_cuda("work list split");
+        launches += 2;
+        if (J.idx_tc.n_items == 0 && J.idx_fp.n_items) {
+            // every item is routed: the plain form's own list, as in a single join
+            if (int ir = plain_work_list(c, st, J.A, J.B, P, self, opts, &J.idx_fp, &launches)) return ir;
+            J.idx_tc.candidate_pairs = 0;
+        }
+    }
     if (J.idx_fp.n_items) {
         if (int rr = ensure_plain_tiles(c, st, &J.A, false, &launches)) return rr;
         if (self)

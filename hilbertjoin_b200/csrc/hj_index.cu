@@ -519,8 +519,8 @@ __global__ void k_item_split(const WorkItem *__restrict__ items, uint64_t n, con
 
 int split_items_by_precision(const IndexResult &in, const SortedSet &A, const SortedSet &B, double c_rel,
                              double c_abs, double limit, const BcConsts *bc,
-                             void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, cudaStream_t st,
-                             IndexResult *tc_out, IndexResult *fp_out) {
+                             void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, unsigned long long *hpin,
+                             cudaStream_t st, IndexResult *tc_out, IndexResult *fp_out) {
     *tc_out = in;
     *fp_out = IndexResult();
     if (in.n_items == 0) return 0;
@@ -538,8 +538,8 @@ int split_items_by_precision(const IndexResult &in, const SortedSet &A, const So
                                                                              flags, stats + 1);
     launch_scan_u32(flags, n, stats, st,
                     (unsigned long long *)alloc(actx, kSlotScanTiles, scan_scratch_bytes(n)));
-    unsigned long long h[2];
-    cudaMemcpyAsync(h, stats, sizeof(h), cudaMemcpyDeviceToHost, st);
+    unsigned long long *h = hpin;
+    cudaMemcpyAsync(h, stats, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return 3;
     const uint64_t n_tc = h[0], n_fp = n - n_tc;
     if (n_fp == 0) return 0;
@@ -568,8 +568,8 @@ constexpr uint64_t kHilbertMinItems = 8192, kHilbertMinBytes = 64ull << 20;
 int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const GridDev &gdev, bool self,
                 uint64_t na_eff, uint64_t nb_eff, int tile_a, int tile_b, int active_dims, uint32_t chunk,
                 uint32_t chunk_min, uint32_t target, uint64_t operand_bytes,
-                void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, cudaStream_t st, IndexResult *out,
-                int *launches, std::string *err) {
+                void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, unsigned long long *hpin,
+                cudaStream_t st, IndexResult *out, int *launches, std::string *err) {
     *out = IndexResult();
     const uint64_t n_tiles = hj_ceil_div(na_eff, tile_a);
     if (n_tiles == 0 || nb_eff == 0) return 0;
@@ -615,8 +615,8 @@ int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const 
                                                                      counts, stats + 1);
     launch_scan_u32(counts, n_tiles, stats + 2, st,
                     (unsigned long long *)alloc(actx, kSlotScanTiles, scan_scratch_bytes(n_tiles)));
-    unsigned long long hstats[4];
-    cudaMemcpyAsync(hstats, stats, sizeof(hstats), cudaMemcpyDeviceToHost, st);
+    unsigned long long *hstats = hpin;
+    cudaMemcpyAsync(hstats, stats, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
     if (launches) *launches += 4;
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {

@@ -215,7 +215,8 @@ struct IndexResult;
 // sets' block summaries, D = 0) and c_rel / c_abs are unused.
 int split_items_by_precision(const IndexResult &tc_in, const SortedSet &A, const SortedSet &B, double c_rel,
                              double c_abs, double limit, const BcConsts *bc,
-                             void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, cudaStream_t st,
+                             void *(*alloc)(void *ctx, int slot, size_t bytes), void *actx, unsigned long long *hpin,
+                             cudaStream_t st,
                              IndexResult *tc_out, IndexResult *fp_out);
 
 // Restricts a work list to shard k of K: the contiguous item range whose
@@ -242,7 +243,12 @@ void ensure_max_dynamic_smem(const void *func, int bytes);
 // Per-dim min/max cell, max |x|, non-finite flag over a row-major set; results
 // accumulate into dstats[d], d_maxabs_bits, d_bad (initialised by the caller).
 void launch_dim_stats(const void *x, int dtype_bytes, uint64_t n, uint32_t d, double eps, DimStats *dstats,
-                      unsigned long long *d_maxabs_bits, uint32_t *d_bad, cudaStream_t st);
+                      unsigned long long *d_maxabs_bits, uint32_t *d_bad, cudaStream_t st, bool cells = true);
+// The cells of each dim's smallest and largest coordinate (cells = false above leaves
+// them to this, or to the host).
+void launch_dim_stats_cells(DimStats *dstats, uint32_t d, double eps, uint32_t *d_bad, cudaStream_t st);
+// Cells beyond +-2^62 cannot be represented; such inputs are rejected.
+constexpr double kCellLimit = 4.611686018427388e18;
 void launch_dim_stats_init(DimStats *dstats, uint32_t d, unsigned long long *d_maxabs_bits, uint32_t *d_bad,
                            cudaStream_t st);
 
@@ -287,13 +293,13 @@ void launch_gather(const void *x, int dtype_bytes, uint64_t n, uint32_t d, const
 // runs of B tiles; expanded into work items of at most `chunk` B tiles (down to
 // chunk_min where that gives fewer than `target` items), and sorted in Hilbert order
 // where the operands (operand_bytes, both sets) exceed what L2 holds. Synchronises
-// once on `st` (item count).
+// once on `st` (item count). hpin: four words of pinned host memory.
 struct IndexScratch;
 int build_index(const SortedSet &A, const SortedSet &B, const Grid &grid, const GridDev &gdev, bool self,
                 uint64_t na_eff, uint64_t nb_eff, int tile_a, int tile_b, int active_dims, uint32_t chunk,
                 uint32_t chunk_min, uint32_t target, uint64_t operand_bytes,
-                void *(*alloc)(void *ctx, int slot, size_t bytes), void *alloc_ctx, cudaStream_t st,
-                IndexResult *out, int *launches, std::string *err);
+                void *(*alloc)(void *ctx, int slot, size_t bytes), void *alloc_ctx, unsigned long long *hpin,
+                cudaStream_t st, IndexResult *out, int *launches, std::string *err);
 
 // Plain FP64 distance kernel over the work list. Adds into *d_count.
 void launch_join_fp64(const SortedSet &A, const SortedSet &B, bool self, uint64_t na_eff, uint64_t nb_eff,

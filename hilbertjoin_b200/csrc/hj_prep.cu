@@ -195,9 +195,6 @@ __global__ void __launch_bounds__(256) k_dim_stats(const T *__restrict__ x, uint
     }
 }
 
-// Cells beyond +-2^62 cannot be represented; such inputs are rejected.
-constexpr double kCellLimit = 4.611686018427388e18;
-
 // Per dim: the cells of its smallest and largest coordinate.
 __global__ void k_dim_stats_cells(DimStats *s, uint32_t d, double eps, uint32_t *bad) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -241,7 +238,7 @@ static void dim_stats_launch(const T *x, uint64_t n, uint32_t d, DimStats *dstat
 }
 
 void launch_dim_stats(const void *x, int dtype_bytes, uint64_t n, uint32_t d, double eps, DimStats *dstats,
-                      unsigned long long *d_maxabs_bits, uint32_t *d_bad, cudaStream_t st) {
+                      unsigned long long *d_maxabs_bits, uint32_t *d_bad, cudaStream_t st, bool cells) {
     const bool vec = ((uintptr_t)x & 15u) == 0;
     if (n) {
         if (dtype_bytes == 8) {
@@ -256,6 +253,10 @@ void launch_dim_stats(const void *x, int dtype_bytes, uint64_t n, uint32_t d, do
                 dim_stats_launch<float, 1>(static_cast<const float *>(x), n, d, dstats, d_maxabs_bits, d_bad, st);
         }
     }
+    if (cells) launch_dim_stats_cells(dstats, d, eps, d_bad, st);
+}
+
+void launch_dim_stats_cells(DimStats *dstats, uint32_t d, double eps, uint32_t *d_bad, cudaStream_t st) {
     k_dim_stats_cells<<<(d + 255) / 256, 256, 0, st>>>(dstats, d, eps, d_bad);
 }
 
