@@ -145,7 +145,7 @@ enum {
     kSlotRowsA, kSlotRowsB, kSlotKeysA, kSlotKeysB, kSlotTilesA, kSlotTilesB,
     kSlotTf32A, kSlotTf32B, kSlotHiA, kSlotLoA, kSlotHiB, kSlotLoB, kSlotNormA, kSlotNormB,
     kSlotTmaxAA, kSlotTmaxAB, kSlotTmaxBA, kSlotTmaxBB, kSlotBand, kSlotCenter, kSlotGminA, kSlotGminB,
-    kSlotItemCnt, kSlotPairKeys, kSlotPairPerm, kSlotPairTmp, kSlotPairHist, kSlotPairOut, kSlotDimCost,
+    kSlotPairKeys, kSlotPairPerm, kSlotPairTmp, kSlotPairHist, kSlotPairOut, kSlotDimCost,
     kSlotGridOrd, kSlotBcOpA, kSlotBcOpB, kSlotBcNormA, kSlotBcNormB, kSlotBcXnA, kSlotBcXnB, kSlotBcBlkA,
     kSlotBcBlkB, kSlotBcCentA, kSlotBcCentB, kSlotScanTiles, kSlotBcOpLoA, kSlotBcOpLoB,
     kSlotEngineEnd
@@ -887,11 +887,12 @@ __global__ void k_pairs_gather(const uint32_t *__restrict__ pi, const uint32_t *
     out[2 * r + 1] = pj[s];
 }
 
-// Pair materialisation: the join on the plain FP64 kernel run twice, once
-// counting the pairs of every work item, once writing them at the exclusive
-// scan of those counts, then a stable radix sort by (i, j) so that the output
-// is the same on every run. Nothing is written to `pairs` unless all of them
-// fit; *n_pairs is always the exact total.
+// Pair materialisation: the plain FP64 kernel lists the pairs as it counts them, into
+// buffers of the caller's capacity (up to kPairRoom; a longer list takes a second run
+// into buffers of its length), then a stable radix sort by (i, j), so that the output
+// is the same on every run. Nothing is written to `pairs` unless all of them fit;
+// *n_pairs is always the exact total.
+constexpr uint64_t kPairRoom = 1ull << 23;  // 64 MB
 static int run_pairs(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *pairs, uint64_t capacity,
                      uint64_t *n_pairs, hj_stats *stats, cudaEvent_t ev_h2d_start) {
     cudaStream_t st = (opts && opts->stream) ? (cudaStream_t)opts->stream : c->stream;
@@ -905,41 +906,47 @@ static int run_pairs(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *pa
     const double T = in.eps * in.eps;
     uint32_t *d_err = reinterpret_cast<uint32_t *>(c->d_small + 3);
     cudaMemsetAsync(c->d_small + 2, 0, 5 * sizeof(unsigned long long), st);
-    const uint64_t n_items = idx.n_items;
-    uint32_t *item_cnt = (uint32_t *)slot_alloc_impl(c, st, kSlotItemCnt, (n_items + 1) * 4);
-    if (!item_cnt) return fail(HJ_ERR_OOM, "out of device memory");
-    cudaMemsetAsync(item_cnt, 0, (n_items + 1) * 4, st);
+    unsigned long long *d_total = c->d_small + 2;
+    uint64_t room = std::min(capacity, kPairRoom);
+    uint32_t *keys = nullptr;  // word-major: word 0 = i (most significant), word 1 = j, `room` entries each
+    uint64_t total = 0;
     cudaEventRecord(c->ev[6], st);
-    launch_pairs_fp64(A, B, in.self, P.na_eff, P.nb_eff, T, idx, item_cnt, nullptr, nullptr, d_err, c->num_sms, st);
-    launch_scan_u32(item_cnt, n_items, c->d_small + 2, st,
-                    (unsigned long long *)slot_alloc_impl(c, st, kSlotScanTiles, scan_scratch_bytes(n_items)));
-    launches += 2;
-    cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("pair count");
-    if (int rr = check_cuda("pair count")) return rr;
-    if ((uint32_t)c->h_small[3] & kErrTimeout) return fail(HJ_ERR_TIMEOUT, "a bounded device-side wait timed out");
-    if ((uint32_t)c->h_small[3]) return fail(HJ_ERR_CUDA, "device error word set");
-    const uint64_t total = c->h_small[2];
-    *n_pairs = total;
-    if (total > capacity)
-        return fail(HJ_ERR_CAPACITY, "the pairs do not fit into the caller's buffer; *n_pairs holds their number");
-    if (total >= (1ull << 32)) return fail(HJ_ERR_UNSUPPORTED, "more than 2^32 - 1 pairs");
+    for (;;) {
+        keys = (uint32_t *)slot_alloc_impl(c, st, kSlotPairKeys, room * 8);
+        if (!keys && total == 0 && room) {  // no room for the guess: count first
+            room = 0;
+            continue;
+        }
+        if (!keys) return fail(HJ_ERR_OOM, "out of device memory (pairs)");
+        launch_pairs_fp64(A, B, in.self, P.na_eff, P.nb_eff, T, idx, d_total, keys, keys + room, room, d_err,
+                          c->num_sms, st);
+        ++launches;
+        cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess) return check_cuda("pair count");
+        if (int rr = check_cuda("pair count")) return rr;
+        if ((uint32_t)c->h_small[3] & kErrTimeout)
+            return fail(HJ_ERR_TIMEOUT, "a bounded device-side wait timed out");
+        if ((uint32_t)c->h_small[3]) return fail(HJ_ERR_CUDA, "device error word set");
+        total = c->h_small[2];
+        *n_pairs = total;
+        if (total > capacity)
+            return fail(HJ_ERR_CAPACITY, "the pairs do not fit into the caller's buffer; *n_pairs holds their number");
+        if (total >= (1ull << 32)) return fail(HJ_ERR_UNSUPPORTED, "more than 2^32 - 1 pairs");
+        if (total <= room) break;
+        room = total;
+        cudaMemsetAsync(d_total, 0, sizeof(unsigned long long), st);
+    }
     if (total) {
-        // keys word-major: word 0 = i (most significant), word 1 = j
-        uint32_t *keys = (uint32_t *)slot_alloc_impl(c, st, kSlotPairKeys, total * 8);
         uint32_t *perm = (uint32_t *)slot_alloc_impl(c, st, kSlotPairPerm, total * 4);
         void *rs = slot_alloc_impl(c, st, kSlotPairHist, radix_scratch_bytes(total));
         unsigned long long *out = (unsigned long long *)slot_alloc_impl(c, st, kSlotPairOut, total * 16);
-        if (!keys || !perm || !rs || !out) return fail(HJ_ERR_OOM, "out of device memory (pairs)");
-        launch_pairs_fp64(A, B, in.self, P.na_eff, P.nb_eff, T, idx, item_cnt, keys, keys + total, d_err,
-                          c->num_sms, st);
-        ++launches;
+        if (!perm || !rs || !out) return fail(HJ_ERR_OOM, "out of device memory (pairs)");
         std::vector<std::pair<uint32_t, uint32_t>> passes;
         const int bj = bitwidth(in.nb ? in.nb - 1 : 0), bi = bitwidth(in.na ? in.na - 1 : 0);
         for (int b = 0; b < bj; b += 8) passes.push_back({1u, (uint32_t)b});
         for (int b = 0; b < bi; b += 8) passes.push_back({0u, (uint32_t)b});
-        radix_sort_perm(keys, total, passes, perm, rs, st, &launches);
-        k_pairs_gather<<<(unsigned)hj_ceil_div(total, 256), 256, 0, st>>>(keys, keys + total, perm, total, out);
+        radix_sort_perm(keys, total, passes, perm, rs, st, &launches, room);
+        k_pairs_gather<<<(unsigned)hj_ceil_div(total, 256), 256, 0, st>>>(keys, keys + room, perm, total, out);
         ++launches;
         cudaEventRecord(c->ev[4], st);
         cudaMemcpyAsync(pairs, out, total * 16, cudaMemcpyDeviceToHost, st);

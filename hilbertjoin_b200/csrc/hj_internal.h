@@ -268,12 +268,13 @@ void launch_norm_key(const void *x, int dtype_bytes, uint64_t n, uint32_t d, con
 // Stable LSD radix sort of a permutation by 8-bit windows of word-major keys
 // ([word][n]); `passes` = (word, shift) in order, least significant first.
 // Needs radix_scratch_bytes(n) of 16-byte aligned device scratch. Result:
-// perm_out[r] = input index of rank r (identity when there is no pass).
+// perm_out[r] = input index of rank r (identity when there is no pass). Word w of the
+// keys starts at keys_wm + w * stride (stride 0: n).
 size_t radix_scratch_bytes(uint64_t n);
 void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32_t, uint32_t> *passes, size_t np,
-                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches);
+                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches, uint64_t stride = 0);
 void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::vector<std::pair<uint32_t, uint32_t>> &passes,
-                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches);
+                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches, uint64_t stride = 0);
 void launch_iota(uint32_t *p, uint64_t n, cudaStream_t st);
 // Exclusive scan of u32 entries in place; total into *total if non-null. With
 // `tile_sums` (scan_scratch_bytes(count) of device scratch) it runs over many
@@ -306,14 +307,12 @@ void launch_join_fp64(const SortedSet &A, const SortedSet &B, bool self, uint64_
                       double T, const IndexResult &idx, unsigned long long *d_count, uint32_t *d_err,
                       int num_sms, cudaStream_t st);
 
-// Pair materialisation on the FP64 kernel. out_i == nullptr: adds each item's
-// pair count into item_cnt[item] (zeroed by the caller). Otherwise item_cnt
-// holds each item's first output slot (exclusive scan of the counts) and the
-// kernel writes the pairs of input indices there (self joins as i < j), in no
-// particular order within an item.
+// Pair materialisation on the FP64 kernel: adds the number of pairs to *d_total (zeroed
+// by the caller) and writes the first `room` of them, in no particular order, as input
+// indices (self joins as i < j).
 void launch_pairs_fp64(const SortedSet &A, const SortedSet &B, bool self, uint64_t na_eff, uint64_t nb_eff,
-                       double T, const IndexResult &idx, uint32_t *item_cnt, uint32_t *out_i, uint32_t *out_j,
-                       uint32_t *d_err, int num_sms, cudaStream_t st);
+                       double T, const IndexResult &idx, unsigned long long *d_total, uint32_t *out_i,
+                       uint32_t *out_j, uint64_t room, uint32_t *d_err, int num_sms, cudaStream_t st);
 
 // Tensor-core kernel + FP64 recheck of the band. Adds into each job's count;
 // band slots reserved into *d_band_total (may exceed `band_cap`: then the

@@ -825,7 +825,7 @@ struct RcPasses {
 constexpr size_t kRcSmem = 4 * (size_t)kRcItems * 4 + (size_t)kRcWarps * 256 * 2 + (4 + 2) * 256 * 4;
 
 __global__ void __cluster_dims__(kRcCtas, 1, 1) __launch_bounds__(kRcThreads)
-    k_rs_cluster(const uint32_t *__restrict__ keys_wm, uint32_t n, uint32_t seg, const __grid_constant__ RcPasses P,
+    k_rs_cluster(const uint32_t *__restrict__ keys_wm, uint64_t stride, uint32_t n, uint32_t seg, const __grid_constant__ RcPasses P,
                  uint32_t *__restrict__ perm_out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -844,7 +844,7 @@ __global__ void __cluster_dims__(kRcCtas, 1, 1) __launch_bounds__(kRcThreads)
     for (uint32_t p = 0; p < P.np; ++p) {
         const uint32_t shift = P.shift[p];
         const bool load = p == 0 || P.word[p] != P.word[p - 1];  // another word: gathered by index
-        const uint32_t *word = keys_wm + (size_t)P.word[p] * n;
+        const uint32_t *word = keys_wm + (size_t)P.word[p] * stride;
         for (uint32_t i = t; i < kRcWarps * 128; i += kRcThreads) reinterpret_cast<uint32_t *>(cnt)[i] = 0;
         __syncthreads();
         uint32_t k[kRcItems / kRcThreads], r[kRcItems / kRcThreads];
@@ -935,8 +935,9 @@ __global__ void k_iota(uint32_t *p, uint64_t n) {
 }
 
 void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32_t, uint32_t> *passes, size_t np,
-                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches) {
+                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches, uint64_t stride) {
     if (n == 0) return;
+    if (stride == 0) stride = n;
     if (np == 0) {
         k_iota<<<(unsigned)hj_ceil_div(n, 256), 256, 0, st>>>(perm_out, n);
         if (launches) *launches += 1;
@@ -955,7 +956,7 @@ void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32
             ensure_max_dynamic_smem((const void *)k_rs_cluster, (int)kRcSmem);
             // whole warps per CTA; eight CTAs cover n
             const uint32_t seg = (uint32_t)hj_ceil_div(hj_ceil_div(n, kRcCtas), 32) * 32;
-            k_rs_cluster<<<kRcCtas, kRcThreads, kRcSmem, st>>>(keys_wm, (uint32_t)n, seg, P, perm_out);
+            k_rs_cluster<<<kRcCtas, kRcThreads, kRcSmem, st>>>(keys_wm, stride, (uint32_t)n, seg, P, perm_out);
             if (launches) *launches += 1;
             return;
         }
@@ -974,12 +975,12 @@ void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32
         const uint32_t shift = passes[p].second;
         // pass 0 reads its word of the input keys (identity order); later
         // passes read the key that the previous pass carried
-        const uint32_t *key_in = p == 0 ? keys_wm + (size_t)passes[0].first * n : kb[p & 1];
+        const uint32_t *key_in = p == 0 ? keys_wm + (size_t)passes[0].first * stride : kb[p & 1];
         const bool vec_key = ((uintptr_t)key_in & 15u) == 0;
         uint32_t *val_out = ((np - 1 - p) & 1) ? vtmp : perm_out;
         uint32_t *key_out = p + 1 < np ? kb[(p + 1) & 1] : nullptr;
         const uint32_t *next_word = nullptr;
-        if (key_out && passes[p + 1].first != passes[p].first) next_word = keys_wm + (size_t)passes[p + 1].first * n;
+        if (key_out && passes[p + 1].first != passes[p].first) next_word = keys_wm + (size_t)passes[p + 1].first * stride;
         k_rs_count<<<nb, kRsThreads, 0, st>>>(key_in, n, shift, nb, vec_key, direct, counts);
         if (direct) {
             k_rs_scatter<true><<<nb, kRsThreads, kRsScatterSmem, st>>>(key_in, val_in, n, shift, nb, vec_key, counts,
@@ -995,8 +996,8 @@ void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::pair<uint32
 }
 
 void radix_sort_perm(const uint32_t *keys_wm, uint64_t n, const std::vector<std::pair<uint32_t, uint32_t>> &passes,
-                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches) {
-    radix_sort_perm(keys_wm, n, passes.data(), passes.size(), perm_out, scratch, st, launches);
+                     uint32_t *perm_out, void *scratch, cudaStream_t st, int *launches, uint64_t stride) {
+    radix_sort_perm(keys_wm, n, passes.data(), passes.size(), perm_out, scratch, st, launches, stride);
 }
 
 void ensure_max_dynamic_smem(const void *func, int bytes) {
