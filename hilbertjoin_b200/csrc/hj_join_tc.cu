@@ -175,7 +175,8 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// Register share of a warpgroup (every warp of it executes one of these once).
+// Register share of a warpgroup: all four warps of it execute the same instruction, once.
+// (Copies of it in the warps' own branches would be undefined behaviour.)
 template <int R>
 __device__ __forceinline__ void reg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
@@ -420,314 +421,313 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // item `i` of the list, an empty one past its end
     auto item_at = [&](uint64_t i) { return i < p.n_items ? p.items[i] : WorkItem{0, 0, 0, 0}; };
 
-    if (warp == 0) {
-        // ------------------------------------------------ TMA producer
-        reg_dec<kCtlRegs>();
-        if (lane == 0) {
-            uint32_t a_cnt = 0, b_cnt = 0;
-            uint32_t abuf = 0, aph = 1;  // A buffer of the next item, parity of its last release
-            uint32_t s = 0, sph = 1;     // B stage of the next atom, parity of its last release
-            bool ok = true;
-            WorkItem w = item_at(blockIdx.x);
-            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
-                const WorkItem wn = item_at(it + stride);
-                const uint32_t ka = p.jobs[w.pad].ka;  // this job's K atoms (<= p.ka)
-                const uint32_t ja_atoms = kBf ? 2 * ka : ka;
-                // parity 1 of a barrier that never completed a phase counts as passed: the first uses do not wait
-                if (!mbar_wait(&bar_aempty[abuf], aph, err, 1)) break;
-                mbar_arrive_expect_tx(&bar_afull[abuf], ja_atoms * kAStageBytes);
-                const uint32_t adst = a_base + abuf * a_buf_bytes;
-                for (uint32_t q = 0; q < ja_atoms; ++q) {
-                    const bool lo = kBf && q >= ka;
-                    const uint32_t kq = kBf ? (lo ? q - ka : q) : q;
-                    tma_load_2d(smem_raw + (adst + q * kAStageBytes - smem_u32(smem_raw)), lo ? &tm_a2 : &tm_a,
-                                (int32_t)(kq * kAtomElems + p.a_xoff), (int32_t)(w.a * kTcTileA), &bar_afull[abuf]);
-                }
-                ++a_cnt;
-                if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
-                for (uint32_t bt = w.b0; ok && bt < w.b1; ++bt) {
+    if (warp < kEpiWarp0) {
+        reg_dec<kCtlRegs>();  // one instruction for the four warps of the warpgroup
+        if (warp == 0) {
+            // ------------------------------------------------ TMA producer
+            if (lane == 0) {
+                uint32_t a_cnt = 0, b_cnt = 0;
+                uint32_t abuf = 0, aph = 1;  // A buffer of the next item, parity of its last release
+                uint32_t s = 0, sph = 1;     // B stage of the next atom, parity of its last release
+                bool ok = true;
+                WorkItem w = item_at(blockIdx.x);
+                for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
+                    const WorkItem wn = item_at(it + stride);
+                    const uint32_t ka = p.jobs[w.pad].ka;  // this job's K atoms (<= p.ka)
+                    const uint32_t ja_atoms = kBf ? 2 * ka : ka;
+                    // parity 1 of a barrier that never completed a phase counts as passed: the first uses do not wait
+                    if (!mbar_wait(&bar_aempty[abuf], aph, err, 1)) break;
+                    mbar_arrive_expect_tx(&bar_afull[abuf], ja_atoms * kAStageBytes);
+                    const uint32_t adst = a_base + abuf * a_buf_bytes;
                     for (uint32_t q = 0; q < ja_atoms; ++q) {
-                        if (!mbar_wait(&bar_bempty[s], sph, err, 2)) {
-                            ok = false;
-                            break;
+                        const bool lo = kBf && q >= ka;
+                        const uint32_t kq = kBf ? (lo ? q - ka : q) : q;
+                        tma_load_2d(smem_raw + (adst + q * kAStageBytes - smem_u32(smem_raw)), lo ? &tm_a2 : &tm_a,
+                                    (int32_t)(kq * kAtomElems + p.a_xoff), (int32_t)(w.a * kTcTileA), &bar_afull[abuf]);
+                    }
+                    ++a_cnt;
+                    if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
+                    for (uint32_t bt = w.b0; ok && bt < w.b1; ++bt) {
+                        for (uint32_t q = 0; q < ja_atoms; ++q) {
+                            if (!mbar_wait(&bar_bempty[s], sph, err, 2)) {
+                                ok = false;
+                                break;
+                            }
+                            mbar_arrive_expect_tx(&bar_bfull[s], kBStageBytes);
+                            const bool lo = kBf && (q & 1u);
+                            const uint32_t kq = kBf ? (q >> 1) : q;
+                            tma_load_2d(smem_raw + (b_base + s * kBStageBytes - smem_u32(smem_raw)), lo ? &tm_b2 : &tm_b,
+                                        (int32_t)(kq * kAtomElems), (int32_t)(bt * kTcTileB), &bar_bfull[s]);
+                            ++b_cnt;
+                            if (++s == p.nst) s = 0, sph ^= 1u;
                         }
-                        mbar_arrive_expect_tx(&bar_bfull[s], kBStageBytes);
-                        const bool lo = kBf && (q & 1u);
-                        const uint32_t kq = kBf ? (q >> 1) : q;
-                        tma_load_2d(smem_raw + (b_base + s * kBStageBytes - smem_u32(smem_raw)), lo ? &tm_b2 : &tm_b,
-                                    (int32_t)(kq * kAtomElems), (int32_t)(bt * kTcTileB), &bar_bfull[s]);
-                        ++b_cnt;
-                        if (++s == p.nst) s = 0, sph ^= 1u;
+                    }
+                    w = wn;
+                }
+                // Drain: on the normal path every copy has been consumed; after an
+                // error (the loops stop at the first failed wait) every copy issued
+                // has landed before the CTA leaves (its full barrier's phase).
+                if (*err) {
+                    const uint64_t deadline = globaltimer_ns() + kWaitLimitNs;
+                    for (uint32_t k = 0; k < p.nst && k < b_cnt; ++k) {
+                        const uint32_t j = b_cnt - 1 - k;
+                        drain_until(&bar_bfull[j % p.nst], (j / p.nst) & 1u, deadline);
+                    }
+                    for (uint32_t k = 0; k < p.a_bufs && k < a_cnt; ++k) {
+                        const uint32_t j = a_cnt - 1 - k;
+                        drain_until(&bar_afull[j % p.a_bufs], (j / p.a_bufs) & 1u, deadline);
                     }
                 }
-                w = wn;
             }
-            // Drain: on the normal path every copy has been consumed; after an
-            // error (the loops stop at the first failed wait) every copy issued
-            // has landed before the CTA leaves (its full barrier's phase).
-            if (*err) {
-                const uint64_t deadline = globaltimer_ns() + kWaitLimitNs;
-                for (uint32_t k = 0; k < p.nst && k < b_cnt; ++k) {
-                    const uint32_t j = b_cnt - 1 - k;
-                    drain_until(&bar_bfull[j % p.nst], (j / p.nst) & 1u, deadline);
-                }
-                for (uint32_t k = 0; k < p.a_bufs && k < a_cnt; ++k) {
-                    const uint32_t j = a_cnt - 1 - k;
-                    drain_until(&bar_afull[j % p.a_bufs], (j / p.a_bufs) & 1u, deadline);
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        // An MMA is accepted about when the one before it ends (128 clocks at N =
-        // 256), so what the thread does between two MMAs beyond that adds to the
-        // tile: the next stage and the next accumulator are looked at before the
-        // current stage's MMAs are issued, descriptors advance by additions, and the
-        // whole warp runs the loop with one elected lane issuing (a lane running it
-        // alone took a third longer per tile).
-        reg_dec<kCtlRegs>();
-        {
-            const bool el = elect_one();
-            constexpr uint32_t idesc = instr_desc<FORM>();
-            uint64_t *bar_a = p.fold ? bar_aready : bar_afull;
-            uint32_t abuf = 0, aph = 0;      // A buffer of the item, its phase
-            uint32_t s = 0, sph = 0;         // B stage of the next atom, its phase
-            uint32_t acc = 0, accph = 1;     // accumulator of the next tile, parity of its last release
-            bool acc_ready = true, b_ready = false;
-            bool issued_any = false, ok = true;
-            const uint64_t b_desc0 = sw128_desc(b_base);
-            WorkItem w = item_at(blockIdx.x);
-            for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
-                const WorkItem wn = item_at(it + stride);
-                const uint32_t ka = p.jobs[w.pad].ka, ksteps = p.jobs[w.pad].ksteps;
-                const uint32_t jb_atoms = kBf ? 2 * ka : ka;
-                if (!mbar_wait(&bar_a[abuf], aph, err, 3)) break;
-                tc_fence_after();
-                const uint64_t a_desc0 = sw128_desc(a_base + abuf * a_buf_bytes);
-                for (uint32_t n = w.b1 - w.b0; ok && n > 0; --n) {
-                    if (!acc_ready && !mbar_wait(&bar_accempty[acc], accph, err, 4)) {
-                        ok = false;
-                        break;
-                    }
+        } else if (warp == 1) {
+            // ------------------------------------------------ MMA issuer
+            // An MMA is accepted about when the one before it ends (128 clocks at N =
+            // 256), so what the thread does between two MMAs beyond that adds to the
+            // tile: the next stage and the next accumulator are looked at before the
+            // current stage's MMAs are issued, descriptors advance by additions, and the
+            // whole warp runs the loop with one elected lane issuing (a lane running it
+            // alone took a third longer per tile).
+            {
+                const bool el = elect_one();
+                constexpr uint32_t idesc = instr_desc<FORM>();
+                uint64_t *bar_a = p.fold ? bar_aready : bar_afull;
+                uint32_t abuf = 0, aph = 0;      // A buffer of the item, its phase
+                uint32_t s = 0, sph = 0;         // B stage of the next atom, its phase
+                uint32_t acc = 0, accph = 1;     // accumulator of the next tile, parity of its last release
+                bool acc_ready = true, b_ready = false;
+                bool issued_any = false, ok = true;
+                const uint64_t b_desc0 = sw128_desc(b_base);
+                WorkItem w = item_at(blockIdx.x);
+                for (uint64_t it = blockIdx.x; ok && it < p.n_items; it += stride) {
+                    const WorkItem wn = item_at(it + stride);
+                    const uint32_t ka = p.jobs[w.pad].ka, ksteps = p.jobs[w.pad].ksteps;
+                    const uint32_t jb_atoms = kBf ? 2 * ka : ka;
+                    if (!mbar_wait(&bar_a[abuf], aph, err, 3)) break;
                     tc_fence_after();
-                    const uint32_t dcol = tmem + acc * kTcTileB;
-                    uint64_t *bar_full = &bar_accfull[acc];
-                    acc ^= 1u;
-                    accph ^= acc ^ 1u;
-                    uint32_t accumulate = 0;
-                    for (uint32_t q = 0; q < jb_atoms; ++q) {
-                        if (!b_ready && !mbar_wait(&bar_bfull[s], sph, err, 5)) {
+                    const uint64_t a_desc0 = sw128_desc(a_base + abuf * a_buf_bytes);
+                    for (uint32_t n = w.b1 - w.b0; ok && n > 0; --n) {
+                        if (!acc_ready && !mbar_wait(&bar_accempty[acc], accph, err, 4)) {
                             ok = false;
                             break;
                         }
-                        const uint64_t bdesc = b_desc0 + s * (kBStageBytes / 16);
-                        uint64_t *bar_release = &bar_bempty[s];
-                        if (++s == p.nst) s = 0, sph ^= 1u;
-                        b_ready = mbar_test(&bar_bfull[s], sph);
-                        if (q + 1 == jb_atoms) acc_ready = mbar_test(&bar_accempty[acc], accph);
-                        // a K step advances both descriptors by 32 bytes (2 in their 16-byte units)
-                        if constexpr (!kBf) {
-                            const uint64_t adesc = a_desc0 + q * (kAStageBytes / 16);
-                            // 4 K steps per atom, fewer in the last (zero columns not multiplied)
-                            const uint32_t kk_end = ksteps - 4 * q < 4 ? ksteps - 4 * q : 4;
-                            if (kk_end == 4) {
+                        tc_fence_after();
+                        const uint32_t dcol = tmem + acc * kTcTileB;
+                        uint64_t *bar_full = &bar_accfull[acc];
+                        acc ^= 1u;
+                        accph ^= acc ^ 1u;
+                        uint32_t accumulate = 0;
+                        for (uint32_t q = 0; q < jb_atoms; ++q) {
+                            if (!b_ready && !mbar_wait(&bar_bfull[s], sph, err, 5)) {
+                                ok = false;
+                                break;
+                            }
+                            const uint64_t bdesc = b_desc0 + s * (kBStageBytes / 16);
+                            uint64_t *bar_release = &bar_bempty[s];
+                            if (++s == p.nst) s = 0, sph ^= 1u;
+                            b_ready = mbar_test(&bar_bfull[s], sph);
+                            if (q + 1 == jb_atoms) acc_ready = mbar_test(&bar_accempty[acc], accph);
+                            // a K step advances both descriptors by 32 bytes (2 in their 16-byte units)
+                            if constexpr (!kBf) {
+                                const uint64_t adesc = a_desc0 + q * (kAStageBytes / 16);
+                                // 4 K steps per atom, fewer in the last (zero columns not multiplied)
+                                const uint32_t kk_end = ksteps - 4 * q < 4 ? ksteps - 4 * q : 4;
+                                if (kk_end == 4) {
 #pragma unroll
-                                for (uint32_t kk = 0; kk < 4; ++kk) {
-                                    if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
-                                    accumulate = 1;
-                                }
-                            } else {
-#pragma unroll
-                                for (uint32_t kk = 0; kk < 3; ++kk) {
-                                    if (kk < kk_end) {
+                                    for (uint32_t kk = 0; kk < 4; ++kk) {
                                         if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
                                     }
+                                } else {
+#pragma unroll
+                                    for (uint32_t kk = 0; kk < 3; ++kk) {
+                                        if (kk < kk_end) {
+                                            if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                            accumulate = 1;
+                                        }
+                                    }
+                                }
+                            } else {
+                                const uint32_t kq = q >> 1;
+                                const uint32_t kk_end = ksteps - 4 * kq < 4 ? ksteps - 4 * kq : 4;
+                                const uint64_t a_hi = a_desc0 + kq * (kAStageBytes / 16);
+                                const uint64_t a_lo = a_desc0 + (ka + kq) * (kAStageBytes / 16);
+                                if ((q & 1u) == 0) {  // B_hi atom: A_hi.B_hi + A_lo.B_hi
+#pragma unroll
+                                    for (uint32_t kk = 0; kk < 4; ++kk) {
+                                        if (kk >= kk_end) break;
+                                        if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                        accumulate = 1;
+                                        if (el) mma_issue<FORM>(dcol, a_lo + 2 * kk, bdesc + 2 * kk, idesc, 1);
+                                    }
+                                } else {  // B_lo atom: A_hi.B_lo
+#pragma unroll
+                                    for (uint32_t kk = 0; kk < 4; ++kk)
+                                        if (kk < kk_end) if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, 1);
                                 }
                             }
-                        } else {
-                            const uint32_t kq = q >> 1;
-                            const uint32_t kk_end = ksteps - 4 * kq < 4 ? ksteps - 4 * kq : 4;
-                            const uint64_t a_hi = a_desc0 + kq * (kAStageBytes / 16);
-                            const uint64_t a_lo = a_desc0 + (ka + kq) * (kAStageBytes / 16);
-                            if ((q & 1u) == 0) {  // B_hi atom: A_hi.B_hi + A_lo.B_hi
+                            if (el) mma_commit(bar_release);  // stage free once these MMAs have read it
+                            issued_any = true;
+                        }
+                        if (!ok) break;
+                        if (el) mma_commit(bar_full);
+                    }
+                    if (el) mma_commit(&bar_aempty[abuf]);
+                    if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
+                    w = wn;
+                }
+                // all MMAs complete before the tensor memory is released
+                if (issued_any) {
+                    if (el) mma_commit(&bar_drain);
+                    drain_until(&bar_drain, 0, globaltimer_ns() + kWaitLimitNs);
+                }
+            }
+        } else if (warp == kFoldWarp && p.fold) {
+            // ------------------------------------------------ A side of folded norms
+            // A folded row holds the pieces of |x|^2 / 2 in its columns d .. d + 2.
+            // As a B operand they meet the A side's constants; here those replace
+            // the pieces of the A tile that has landed (once per item, 128 rows of
+            // 3 columns), before the MMA warp is told that the tile is ready.
+            uint32_t abuf = 0, aph = 0;
+            for (uint64_t it = blockIdx.x; it < p.n_items; it += stride) {
+                const TcJob &J = p.jobs[p.items[it].pad];
+                const bool fold = J.fold != 0;
+                const uint32_t d = J.d, ka = J.ka;
+                const bool landed = mbar_wait(&bar_afull[abuf], aph, err, 7);
+                if (!__all_sync(0xffffffffu, landed)) break;
+                if (fold) {
+                    const uint32_t abase = a_base + abuf * a_buf_bytes;
+                    for (uint32_t r = lane; r < (uint32_t)kTcTileA; r += 32) {
 #pragma unroll
-                                for (uint32_t kk = 0; kk < 4; ++kk) {
-                                    if (kk >= kk_end) break;
-                                    if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
-                                    accumulate = 1;
-                                    if (el) mma_issue<FORM>(dcol, a_lo + 2 * kk, bdesc + 2 * kk, idesc, 1);
-                                }
-                            } else {  // B_lo atom: A_hi.B_lo
-#pragma unroll
-                                for (uint32_t kk = 0; kk < 4; ++kk)
-                                    if (kk < kk_end) if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, 1);
+                        for (uint32_t m = 0; m < 3; ++m) {
+                            const uint32_t col = d + m, q = col / kAtomElems;
+                            const uint32_t byte = (col % kAtomElems) * (kAtomBytes / kAtomElems);
+                            const uint32_t off = q * kAStageBytes + r * kAtomBytes + (((byte >> 4) ^ (r & 7u)) << 4) +
+                                                 (byte & 15u);
+                            if constexpr (FORM == HJ_FORM_TC_TF32) {
+                                asm volatile("st.shared.b32 [%0], %1;" ::"r"(abase + off), "r"(0xBF800000u) : "memory");
+                            } else if constexpr (kBf) {  // -1 and 0
+                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"((uint16_t)0xBF80) : "memory");
+                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + ka * kAStageBytes + off),
+                                             "h"((uint16_t)0)
+                                             : "memory");
+                            } else {  // -2^15, -2^4, -2^-7
+                                const uint16_t c = m == 0 ? 0xF800 : (m == 1 ? 0xCC00 : 0xA000);
+                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"(c) : "memory");
                             }
                         }
-                        if (el) mma_commit(bar_release);  // stage free once these MMAs have read it
-                        issued_any = true;
                     }
-                    if (!ok) break;
-                    if (el) mma_commit(bar_full);
+                    fence_proxy_async();
                 }
-                if (el) mma_commit(&bar_aempty[abuf]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar_aready[abuf]);
                 if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
-                w = wn;
             }
-            // all MMAs complete before the tensor memory is released
-            if (issued_any) {
-                if (el) mma_commit(&bar_drain);
-                drain_until(&bar_drain, 0, globaltimer_ns() + kWaitLimitNs);
-            }
-        }
-    } else if (warp == kFoldWarp && p.fold) {
-        // ------------------------------------------------ A side of folded norms
-        reg_dec<kCtlRegs>();
-        // A folded row holds the pieces of |x|^2 / 2 in its columns d .. d + 2.
-        // As a B operand they meet the A side's constants; here those replace
-        // the pieces of the A tile that has landed (once per item, 128 rows of
-        // 3 columns), before the MMA warp is told that the tile is ready.
-        uint32_t abuf = 0, aph = 0;
-        for (uint64_t it = blockIdx.x; it < p.n_items; it += stride) {
-            const TcJob &J = p.jobs[p.items[it].pad];
-            const bool fold = J.fold != 0;
-            const uint32_t d = J.d, ka = J.ka;
-            const bool landed = mbar_wait(&bar_afull[abuf], aph, err, 7);
-            if (!__all_sync(0xffffffffu, landed)) break;
-            if (fold) {
-                const uint32_t abase = a_base + abuf * a_buf_bytes;
-                for (uint32_t r = lane; r < (uint32_t)kTcTileA; r += 32) {
+        } else {
+            // ------------------------------------------------ near warps
+            // Warp 3, and warp 2 where no job folds its norms: each works off the queues
+            // of its share of the epilogue warps. Lane r < kEpiWarps keeps queue r.
+            const bool mine = lane < (uint32_t)kEpiWarps && (p.fold || (lane & 1u) == (warp & 1u));
+            uint32_t head = 0, slot = 0;  // entries worked off, and the next one's slot
+            uint32_t job = 0xffffffffu;
+            unsigned long long cnt = 0;
+            BandWriter band(p, lane, BC ? kBandChunk : kBandChunkRare);
+            auto flush = [&]() {
+                const unsigned long long wc = warp_sum_u64(cnt);
+                if (lane == 0 && wc) atomicAdd(p.jobs[job].count, wc);
+                cnt = 0;
+            };
+            // every epilogue warp ends its queue (its own waits are bounded), so this
+            // loop ends; the time limit is a second line only
+            const uint64_t t0 = globaltimer_ns();
+            for (uint32_t idle = 0;;) {
+                const uint32_t tail = mine ? lds_acquire(&near_tail[lane]) : kNearDone;
+                __syncwarp();  // the acquiring lanes' view becomes the warp's
+                const uint32_t avail = mine ? (tail - head) & ~kNearDone : 0u;
+                if (!__any_sync(0xffffffffu, avail != 0)) {
+                    if (__all_sync(0xffffffffu, (tail & kNearDone) != 0)) break;
+                    if ((++idle & 1023u) == 0 && globaltimer_ns() - t0 > kIdleLimitNs) {
+                        atomicOr((uint32_t *)err, kErrTimeout | (10u << 8));
+                        break;
+                    }
+                    __nanosleep(64);
+                    continue;
+                }
+                // lane i takes row i of the queues in order
+                uint32_t my_q = 0, my_i = 0, taken = 0, took = 0;
 #pragma unroll
-                    for (uint32_t m = 0; m < 3; ++m) {
-                        const uint32_t col = d + m, q = col / kAtomElems;
-                        const uint32_t byte = (col % kAtomElems) * (kAtomBytes / kAtomElems);
-                        const uint32_t off = q * kAStageBytes + r * kAtomBytes + (((byte >> 4) ^ (r & 7u)) << 4) +
-                                             (byte & 15u);
-                        if constexpr (FORM == HJ_FORM_TC_TF32) {
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(abase + off), "r"(0xBF800000u) : "memory");
-                        } else if constexpr (kBf) {  // -1 and 0
-                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"((uint16_t)0xBF80) : "memory");
-                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + ka * kAStageBytes + off),
-                                         "h"((uint16_t)0)
-                                         : "memory");
-                        } else {  // -2^15, -2^4, -2^-7
-                            const uint16_t c = m == 0 ? 0xF800 : (m == 1 ? 0xCC00 : 0xA000);
-                            asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"(c) : "memory");
+                for (uint32_t r = 0; r < (uint32_t)kEpiWarps; ++r) {
+                    const uint32_t have = __shfl_sync(0xffffffffu, avail, r), n = have < 32 - taken ? have : 32 - taken;
+                    if (lane >= taken && lane < taken + n) my_q = r, my_i = lane - taken;
+                    if (lane == r) took = n;
+                    taken += n;
+                }
+                const bool row = lane < taken;
+                uint32_t at = __shfl_sync(0xffffffffu, slot, my_q) + my_i;
+                if (at >= p.near_cap) at -= p.near_cap;
+                const float *ent = near_base + my_q * near_ring + at * kNearWords;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                uint4 u = make_uint4(0u, 0u, 0u, 0u);
+                uint32_t g_in = 0, bbits = 0;
+                if (row) {
+                    q = *reinterpret_cast<const float4 *>(ent + 32);
+                    u = *reinterpret_cast<const uint4 *>(ent + 36);
+                    const float4 *nrm = reinterpret_cast<const float4 *>(BC || u.w ? nullptr : p.norm_b + u.x);
+                    float4 nb[8];
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) nb[k] = nrm ? __ldg(nrm + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    uint32_t g_out = 0;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const float4 v = *reinterpret_cast<const float4 *>(ent + 4 * k);
+                        const float t[4] = {fmaf(-2.0f, v.x, nb[k].x), fmaf(-2.0f, v.y, nb[k].y),
+                                            fmaf(-2.0f, v.z, nb[k].z), fmaf(-2.0f, v.w, nb[k].w)};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            g_in |= t[j] <= q.y ? 1u << (4 * k + j) : 0u;
+                            g_out |= t[j] <= q.z ? 1u << (4 * k + j) : 0u;
                         }
                     }
+                    g_in &= u.y;
+                    bbits = g_out & u.y & ~g_in;
                 }
-                fence_proxy_async();
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bar_aready[abuf]);
-            if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
-        }
-    } else if (warp < kEpiWarp0) {
-        // ------------------------------------------------ near warps
-        // Warp 3, and warp 2 where no job folds its norms: each works off the queues
-        // of its share of the epilogue warps. Lane r < kEpiWarps keeps queue r.
-        reg_dec<kCtlRegs>();
-        const bool mine = lane < (uint32_t)kEpiWarps && (p.fold || (lane & 1u) == (warp & 1u));
-        uint32_t head = 0, slot = 0;  // entries worked off, and the next one's slot
-        uint32_t job = 0xffffffffu;
-        unsigned long long cnt = 0;
-        BandWriter band(p, lane, BC ? kBandChunk : kBandChunkRare);
-        auto flush = [&]() {
-            const unsigned long long wc = warp_sum_u64(cnt);
-            if (lane == 0 && wc) atomicAdd(p.jobs[job].count, wc);
-            cnt = 0;
-        };
-        // every epilogue warp ends its queue (its own waits are bounded), so this
-        // loop ends; the time limit is a second line only
-        const uint64_t t0 = globaltimer_ns();
-        for (uint32_t idle = 0;;) {
-            const uint32_t tail = mine ? lds_acquire(&near_tail[lane]) : kNearDone;
-            __syncwarp();  // the acquiring lanes' view becomes the warp's
-            const uint32_t avail = mine ? (tail - head) & ~kNearDone : 0u;
-            if (!__any_sync(0xffffffffu, avail != 0)) {
-                if (__all_sync(0xffffffffu, (tail & kNearDone) != 0)) break;
-                if ((++idle & 1023u) == 0 && globaltimer_ns() - t0 > kIdleLimitNs) {
-                    atomicOr((uint32_t *)err, kErrTimeout | (10u << 8));
-                    break;
+                // counts, into the job that every row of the batch belongs to as a rule
+                const uint32_t j0 = __shfl_sync(0xffffffffu, u.z, 0);
+                if (__all_sync(0xffffffffu, !row || u.z == j0)) {
+                    if (j0 != job) {
+                        if (job != 0xffffffffu) flush();
+                        job = j0;
+                    }
+                    cnt += __popc(g_in);
+                } else if (g_in) {
+                    atomicAdd(p.jobs[u.z].count, (unsigned long long)__popc(g_in));
                 }
-                __nanosleep(64);
-                continue;
-            }
-            // lane i takes row i of the queues in order
-            uint32_t my_q = 0, my_i = 0, taken = 0, took = 0;
+                if (__any_sync(0xffffffffu, bbits != 0)) {
+                    const uint32_t nbits = __popc(bbits);
+                    uint32_t incl = nbits;
 #pragma unroll
-            for (uint32_t r = 0; r < (uint32_t)kEpiWarps; ++r) {
-                const uint32_t have = __shfl_sync(0xffffffffu, avail, r), n = have < 32 - taken ? have : 32 - taken;
-                if (lane >= taken && lane < taken + n) my_q = r, my_i = lane - taken;
-                if (lane == r) took = n;
-                taken += n;
-            }
-            const bool row = lane < taken;
-            uint32_t at = __shfl_sync(0xffffffffu, slot, my_q) + my_i;
-            if (at >= p.near_cap) at -= p.near_cap;
-            const float *ent = near_base + my_q * near_ring + at * kNearWords;
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint4 u = make_uint4(0u, 0u, 0u, 0u);
-            uint32_t g_in = 0, bbits = 0;
-            if (row) {
-                q = *reinterpret_cast<const float4 *>(ent + 32);
-                u = *reinterpret_cast<const uint4 *>(ent + 36);
-                const float4 *nrm = reinterpret_cast<const float4 *>(BC || u.w ? nullptr : p.norm_b + u.x);
-                float4 nb[8];
-#pragma unroll
-                for (int k = 0; k < 8; ++k) nb[k] = nrm ? __ldg(nrm + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-                uint32_t g_out = 0;
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float4 v = *reinterpret_cast<const float4 *>(ent + 4 * k);
-                    const float t[4] = {fmaf(-2.0f, v.x, nb[k].x), fmaf(-2.0f, v.y, nb[k].y),
-                                        fmaf(-2.0f, v.z, nb[k].z), fmaf(-2.0f, v.w, nb[k].w)};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        g_in |= t[j] <= q.y ? 1u << (4 * k + j) : 0u;
-                        g_out |= t[j] <= q.z ? 1u << (4 * k + j) : 0u;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= (uint32_t)o) incl += y;
+                    }
+                    const BandSlots sl = band.reserve(__shfl_sync(0xffffffffu, incl, 31));
+                    uint32_t rank = incl - nbits;
+                    while (bbits) {
+                        const int j = __ffs(bbits) - 1;
+                        bbits &= bbits - 1;
+                        const float t = fmaf(-2.0f, ent[j], BC || u.w ? 0.f : __ldg(p.norm_b + u.x + j));
+                        band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[u.z].s_unscale, u.z);
                     }
                 }
-                g_in &= u.y;
-                bbits = g_out & u.y & ~g_in;
-            }
-            // counts, into the job that every row of the batch belongs to as a rule
-            const uint32_t j0 = __shfl_sync(0xffffffffu, u.z, 0);
-            if (__all_sync(0xffffffffu, !row || u.z == j0)) {
-                if (j0 != job) {
-                    if (job != 0xffffffffu) flush();
-                    job = j0;
-                }
-                cnt += __popc(g_in);
-            } else if (g_in) {
-                atomicAdd(p.jobs[u.z].count, (unsigned long long)__popc(g_in));
-            }
-            if (__any_sync(0xffffffffu, bbits != 0)) {
-                const uint32_t nbits = __popc(bbits);
-                uint32_t incl = nbits;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= (uint32_t)o) incl += y;
-                }
-                const BandSlots sl = band.reserve(__shfl_sync(0xffffffffu, incl, 31));
-                uint32_t rank = incl - nbits;
-                while (bbits) {
-                    const int j = __ffs(bbits) - 1;
-                    bbits &= bbits - 1;
-                    const float t = fmaf(-2.0f, ent[j], BC || u.w ? 0.f : __ldg(p.norm_b + u.x + j));
-                    band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[u.z].s_unscale, u.z);
+                __syncwarp();  // the rows have been read
+                if (took) {
+                    head = (head + took) & ~kNearDone;
+                    slot = slot + took < p.near_cap ? slot + took : slot + took - p.near_cap;
+                    sts_release(&near_head[lane], head);
                 }
             }
-            __syncwarp();  // the rows have been read
-            if (took) {
-                head = (head + took) & ~kNearDone;
-                slot = slot + took < p.near_cap ? slot + took : slot + took - p.near_cap;
-                sts_release(&near_head[lane], head);
-            }
+            if (job != 0xffffffffu) flush();
+            band.finish();
         }
-        if (job != 0xffffffffu) flush();
-        band.finish();
     } else {
         // ------------------------------------------------ epilogue
         reg_inc<kEpiRegs>();
