@@ -41,9 +41,9 @@
 //
 // What bounds it (one B200, 1.965 GHz, distance kernel alone, before -> after the
 // epilogue took this form): one global centre, 1M x 64 FP16, 32 neighbours: 79.7 ->
-// 70 ms; 200k x 64: 4.25 -> 3.7; 200k x 200k x 20 (folded norms): 15.4 -> 6.6; 30k x
-// 70k x 100: 1.17 -> 0.56; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
-// clustered FP16: 53 -> 38.3; 300k x 32 TF32: 2.9 -> 1.96. At K = 64 a tile's MMAs
+// 69 ms; 200k x 64: 4.25 -> 3.4; 200k x 200k x 20 (folded norms): 15.4 -> 6.0; 30k x
+// 70k x 100: 1.17 -> 0.54; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
+// clustered FP16: 53 -> 37.9; 300k x 32 TF32: 2.9 -> 1.93. At K = 64 a tile's MMAs
 // take 512 clocks and a tile without near rows about 1100: the chain MMA -> commit
 // -> TMEM load -> release -> MMA over two accumulators. Near rows add the rest. An
 // instruction of the epilogue costs its warp four to six clocks and a ready barrier,
@@ -84,7 +84,8 @@ constexpr int kChunkCols = 64;
 // Block centring, where near pairs are common, takes larger chunks.
 constexpr uint32_t kBandChunk = 256, kBandChunkRare = 32;
 constexpr uint32_t kBandHole = 0xffffffffu;
-static_assert(kEpiWarps * kEpiCols == 4 * kTcTileB && kEpiCols == 2 * kChunkCols && kChunkCols == 64, "the shared-memory plan and the epilogue assume 8 warps of two chunks");
+static_assert(kEpiWarps * kEpiCols == 4 * kTcTileB && kEpiCols == 2 * kChunkCols && kChunkCols == 64,
+              "the shared-memory plan and the epilogue assume 8 warps of two chunks");
 // Warpgroup 0 holds the control and near warps, warpgroups 1 and 2 the epilogue. The
 // block launches with 168 registers a thread (64512); warpgroup 0 gives part of its
 // share to the epilogue: 128 x 88 + 256 x 208 = 64512.
@@ -105,17 +106,21 @@ constexpr uint32_t kTmemCols = 512;
 // classification takes one to two thousand clocks of latency (the B norms, a slot in
 // the band queue), and one near row in a tile used to hold the accumulator of all
 // eight warps for it; at 1M x 64 and 32 neighbours six tiles in ten have one.
-// An entry: 32 values | |a|^2, thr_in, thr_out, A rank | first B rank, column mask,
-// job, norms folded | 4 unused words (an odd number of 16-byte units, so that lanes
+// An entry: 32 values | |a|^2, thr_in, thr_out, A rank | first B rank, job, norms
+// folded, 0 | 4 unused words (an odd number of 16-byte units, so that lanes
 // reading their rows do not meet in a bank).
 constexpr uint32_t kNearWords = 44;
 constexpr uint32_t kNearCap = 24;    // entries per warp, at most
 // A group with more near rows is classified by the epilogue warp (lane = row): about
 // 1000 clocks however many rows, against the queue's per-row cost. With one centre, 30k x
-// 70k x 100: 0.57 ms at 0, 0.56 at 3, 0.75 at 10; 1M x 64: 78, 70, 70 ms. Block
-// centres, 4M x 28: 40.2 ms at 0, 39.5 at 3, 38.5 at 5 and at 8.
-constexpr uint32_t kNearDenseBc = 6, kNearDenseOne = 3;
+// 70k x 100: 0.54 ms at 3, 0.62 at 6; 1M x 64: 78 ms at 0, 69 at 3, 68 at 6. Block
+// centres, 4M x 28: 37.9 ms at 6, 40.5 at 8.
+constexpr int kNearDenseBc = 6, kNearDenseOne = 3;
 constexpr uint32_t kNearMinCap = 8;  // fewer entries than this are not worth a B stage
+// Rows that a near warp waits for before it starts on a batch, unless a queue is half
+// full, instead of at the first row: 200k x 200k x 20 6.7 -> 6.35 ms, 1M x 64 72 -> 69.6;
+// at 12 rows half of that.
+constexpr uint32_t kNearBatch = 24;
 constexpr uint32_t kNearDone = 0x80000000u;  // in a queue's tail: its warp has finished
 
 constexpr uint64_t kIdleLimitNs = 600000000000ull;  // the near warps' longest run: 10 minutes
@@ -175,8 +180,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// Register share of a warpgroup: all four warps of it execute the same instruction, once.
-// (Copies of it in the warps' own branches would be undefined behaviour.)
+// Register share of a warpgroup: all its warps execute the same one of these, once.
 template <int R>
 __device__ __forceinline__ void reg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
@@ -191,14 +195,17 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
     return r != 0;
 }
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
+__device__ __forceinline__ void mma_commit(bool issue, uint64_t *bar) {
+    if (!issue) return;
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
 
+// This and mma_commit act in the warp's elected lane only (`issue`).
 template <int FORM>
-__device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void mma_issue(bool issue, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
+    if (!issue) return;
     if constexpr (FORM == HJ_FORM_TC_TF32) {
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -357,6 +364,15 @@ __device__ __forceinline__ void sts_release(uint32_t *a, uint32_t v) {
     asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(smem_u32(a)), "r"(v) : "memory");
 }
 
+// Columns of the 32 from rank gj that row gi may count: below b_end, and above its own
+// rank for a self-join.
+__device__ __forceinline__ uint32_t count_mask(uint32_t gi, uint32_t gj, uint32_t b_end, bool self) {
+    const int hi = (int)b_end - (int)gj, lo = self ? (int)gi + 1 - (int)gj : 0;
+    const uint32_t mh = hi >= 32 ? 0xffffffffu : (hi <= 0 ? 0u : (1u << hi) - 1u);
+    const uint32_t ml = lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
+    return mh & ml;
+}
+
 // ---------------------------------------------------------------- the kernel
 
 template <int FORM, bool BC>
@@ -421,8 +437,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     // item `i` of the list, an empty one past its end
     auto item_at = [&](uint64_t i) { return i < p.n_items ? p.items[i] : WorkItem{0, 0, 0, 0}; };
 
+    // every warp of a warpgroup executes the same setmaxnreg
     if (warp < kEpiWarp0) {
-        reg_dec<kCtlRegs>();  // one instruction for the four warps of the warpgroup
+        reg_dec<kCtlRegs>();
         if (warp == 0) {
             // ------------------------------------------------ TMA producer
             if (lane == 0) {
@@ -534,14 +551,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                 if (kk_end == 4) {
 #pragma unroll
                                     for (uint32_t kk = 0; kk < 4; ++kk) {
-                                        if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                        mma_issue<FORM>(el, dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
                                     }
                                 } else {
 #pragma unroll
                                     for (uint32_t kk = 0; kk < 3; ++kk) {
                                         if (kk < kk_end) {
-                                            if (el) mma_issue<FORM>(dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                            mma_issue<FORM>(el, dcol, adesc + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                             accumulate = 1;
                                         }
                                     }
@@ -555,29 +572,29 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 #pragma unroll
                                     for (uint32_t kk = 0; kk < 4; ++kk) {
                                         if (kk >= kk_end) break;
-                                        if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
+                                        mma_issue<FORM>(el, dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, accumulate);
                                         accumulate = 1;
-                                        if (el) mma_issue<FORM>(dcol, a_lo + 2 * kk, bdesc + 2 * kk, idesc, 1);
+                                        mma_issue<FORM>(el, dcol, a_lo + 2 * kk, bdesc + 2 * kk, idesc, 1);
                                     }
                                 } else {  // B_lo atom: A_hi.B_lo
 #pragma unroll
                                     for (uint32_t kk = 0; kk < 4; ++kk)
-                                        if (kk < kk_end) if (el) mma_issue<FORM>(dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, 1);
+                                        if (kk < kk_end) mma_issue<FORM>(el, dcol, a_hi + 2 * kk, bdesc + 2 * kk, idesc, 1);
                                 }
                             }
-                            if (el) mma_commit(bar_release);  // stage free once these MMAs have read it
+                            mma_commit(el, bar_release);  // stage free once these MMAs have read it
                             issued_any = true;
                         }
                         if (!ok) break;
-                        if (el) mma_commit(bar_full);
+                        mma_commit(el, bar_full);
                     }
-                    if (el) mma_commit(&bar_aempty[abuf]);
+                    mma_commit(el, &bar_aempty[abuf]);
                     if (++abuf == p.a_bufs) abuf = 0, aph ^= 1u;
                     w = wn;
                 }
                 // all MMAs complete before the tensor memory is released
                 if (issued_any) {
-                    if (el) mma_commit(&bar_drain);
+                    mma_commit(el, &bar_drain);
                     drain_until(&bar_drain, 0, globaltimer_ns() + kWaitLimitNs);
                 }
             }
@@ -643,13 +660,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const uint32_t tail = mine ? lds_acquire(&near_tail[lane]) : kNearDone;
                 __syncwarp();  // the acquiring lanes' view becomes the warp's
                 const uint32_t avail = mine ? (tail - head) & ~kNearDone : 0u;
-                if (!__any_sync(0xffffffffu, avail != 0)) {
-                    if (__all_sync(0xffffffffu, (tail & kNearDone) != 0)) break;
+                // a batch costs the same for one row and for 32, and its instructions
+                // compete with the epilogue's: it waits for rows, or a queue half full
+                const uint32_t rows = __reduce_add_sync(0xffffffffu, avail);
+                const bool last = __all_sync(0xffffffffu, (tail & kNearDone) != 0);
+                if (last && rows == 0) break;
+                if (!last && rows < kNearBatch && 2 * __reduce_max_sync(0xffffffffu, avail) < p.near_cap) {
                     if ((++idle & 1023u) == 0 && globaltimer_ns() - t0 > kIdleLimitNs) {
                         atomicOr((uint32_t *)err, kErrTimeout | (10u << 8));
                         break;
                     }
-                    __nanosleep(64);
+                    __nanosleep(200);
                     continue;
                 }
                 // lane i takes row i of the queues in order
@@ -667,11 +688,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const float *ent = near_base + my_q * near_ring + at * kNearWords;
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                 uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                uint32_t g_in = 0, bbits = 0;
+                uint32_t g_in = 0, bbits = 0, ejob = 0;
                 if (row) {
                     q = *reinterpret_cast<const float4 *>(ent + 32);
                     u = *reinterpret_cast<const uint4 *>(ent + 36);
-                    const float4 *nrm = reinterpret_cast<const float4 *>(BC || u.w ? nullptr : p.norm_b + u.x);
+                    ejob = u.y;
+                    const TcJob &J = p.jobs[ejob];
+                    const uint32_t mask = count_mask(__float_as_uint(q.w), u.x, (uint32_t)J.b_end, J.self != 0);
+                    const float4 *nrm = reinterpret_cast<const float4 *>(BC || u.z ? nullptr : p.norm_b + u.x);
                     float4 nb[8];
 #pragma unroll
                     for (int k = 0; k < 8; ++k) nb[k] = nrm ? __ldg(nrm + k) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -687,19 +711,19 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                             g_out |= t[j] <= q.z ? 1u << (4 * k + j) : 0u;
                         }
                     }
-                    g_in &= u.y;
-                    bbits = g_out & u.y & ~g_in;
+                    g_in &= mask;
+                    bbits = g_out & mask & ~g_in;
                 }
                 // counts, into the job that every row of the batch belongs to as a rule
-                const uint32_t j0 = __shfl_sync(0xffffffffu, u.z, 0);
-                if (__all_sync(0xffffffffu, !row || u.z == j0)) {
+                const uint32_t j0 = __shfl_sync(0xffffffffu, ejob, 0);
+                if (__all_sync(0xffffffffu, !row || ejob == j0)) {
                     if (j0 != job) {
                         if (job != 0xffffffffu) flush();
                         job = j0;
                     }
                     cnt += __popc(g_in);
                 } else if (g_in) {
-                    atomicAdd(p.jobs[u.z].count, (unsigned long long)__popc(g_in));
+                    atomicAdd(p.jobs[ejob].count, (unsigned long long)__popc(g_in));
                 }
                 if (__any_sync(0xffffffffu, bbits != 0)) {
                     const uint32_t nbits = __popc(bbits);
@@ -714,8 +738,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     while (bbits) {
                         const int j = __ffs(bbits) - 1;
                         bbits &= bbits - 1;
-                        const float t = fmaf(-2.0f, ent[j], BC || u.w ? 0.f : __ldg(p.norm_b + u.x + j));
-                        band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[u.z].s_unscale, u.z);
+                        const float t = fmaf(-2.0f, ent[j], BC || u.z ? 0.f : __ldg(p.norm_b + u.x + j));
+                        band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[ejob].s_unscale, ejob);
                     }
                 }
                 __syncwarp();  // the rows have been read
@@ -869,14 +893,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             thr_in = (T_lo - tau_max) - na - marg;
             if (!row_ok) thr_out = thr_in = -3.0e38f;
         };
-        // columns of the 32 from rank gj that the lane's row may count: below
-        // b_end, and above the row's own rank for a self-join
-        auto col_mask = [&](uint32_t gj) -> uint32_t {
-            const int hi = (int)b_end - (int)gj, lo = self ? (int)gi + 1 - (int)gj : 0;
-            const uint32_t mh = hi >= 32 ? 0xffffffffu : (hi <= 0 ? 0u : (1u << hi) - 1u);
-            const uint32_t ml = lo <= 0 ? 0xffffffffu : (lo >= 32 ? 0u : ~((1u << lo) - 1u));
-            return row_ok ? mh & ml : 0u;
-        };
         // Band entries of a lane's row: the columns `bbits` of the 32 from rank gj.
         // Ranks by a warp prefix sum, slots from one warp-wide reservation. The
         // estimates are not kept here: NaN, which the recheck's error statistic skips.
@@ -900,7 +916,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // Groups of 32 columns in which many rows are near: every lane classifies its
         // own row from its registers.
         auto dense_rows = [&](const float *v, bool need, uint32_t gj) {
-            const uint32_t colmask = need ? col_mask(gj) : 0u;
+            const uint32_t colmask = need && row_ok ? count_mask(gi, gj, b_end, self) : 0u;
             uint32_t g_in = 0, g_out = 0;
             if (BC || fold) {
                 // t = -2 w, so t <= thr  <=>  w >= -thr / 2 (exact scaling)
@@ -928,42 +944,59 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             cnt += __popc(g_in);
             put_band_bits(g_out & colmask & ~g_in, gj);
         };
-        // A group's near rows (bits of `rows`) into the near queue; waits for room
-        auto queue_rows = [&](const float *v, uint32_t rows, uint32_t gj) {
-            while (rows) {
-                uint32_t room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
-                if (room == 0) {
-                    const uint64_t t0 = globaltimer_ns();
-                    for (uint32_t i = 1; room == 0; ++i) {
-                        n_head = lds_acquire(&near_head[ew]);
-                        room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
-                        if ((i & 255u) == 0 && (*err != 0 || globaltimer_ns() - t0 > kWaitLimitNs)) {
-                            if (lane == 0 && *err == 0) atomicOr((uint32_t *)err, kErrTimeout | (8u << 8));
-                            break;
-                        }
+        // waits until the near queue has room for a row; false: the error word is set
+        auto wait_room = [&]() -> bool {
+            const uint64_t t0 = globaltimer_ns();
+            for (uint32_t i = 1;; ++i) {
+                n_head = __shfl_sync(0xffffffffu, lds_acquire(&near_head[ew]), 0);
+                if (((n_tail - n_head) & ~kNearDone) < p.near_cap) return true;
+                if ((i & 255u) == 0) {
+                    const bool late = globaltimer_ns() - t0 > kWaitLimitNs;
+                    if (__any_sync(0xffffffffu, *err != 0 || late)) {
+                        if (lane == 0 && *err == 0) atomicOr((uint32_t *)err, kErrTimeout | (8u << 8));
+                        return false;
                     }
-                    if (!__all_sync(0xffffffffu, room != 0)) return;  // the error word is set: the count is void
-                    n_head = __shfl_sync(0xffffffffu, n_head, 0);
-                    room = p.near_cap - ((n_tail - n_head) & ~kNearDone);
                 }
-                const uint32_t k = __popc(rows), rank = __popc(rows & ((1u << lane) - 1u));
-                const uint32_t take = k < room ? k : room;
-                const bool put = (rows >> lane) & 1u && rank < take;
-                if (put) {
-                    const uint32_t at = n_slot + rank < p.near_cap ? n_slot + rank : n_slot + rank - p.near_cap;
-                    float *ent = near + at * kNearWords;
+            }
+        };
+        auto put_row = [&](const float *v, uint32_t rank, uint32_t gj) {
+            const uint32_t at = n_slot + rank < p.near_cap ? n_slot + rank : n_slot + rank - p.near_cap;
+            float4 *ent = reinterpret_cast<float4 *>(near + at * kNearWords);
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        reinterpret_cast<float4 *>(ent)[q] =
-                            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                    reinterpret_cast<float4 *>(ent)[8] = make_float4(na, thr_in, thr_out, __uint_as_float(gi));
-                    reinterpret_cast<uint4 *>(ent)[9] = make_uint4(gj, col_mask(gj), job, BC || fold ? 1u : 0u);
+            for (int q = 0; q < 8; ++q) ent[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            ent[8] = make_float4(na, thr_in, thr_out, __uint_as_float(gi));
+            *reinterpret_cast<uint4 *>(ent + 9) = make_uint4(gj, job, BC || fold ? 1u : 0u, 0u);
+        };
+        auto publish = [&](uint32_t k) {
+            n_slot = n_slot + k < p.near_cap ? n_slot + k : n_slot + k - p.near_cap;
+            n_tail = (n_tail + k) & ~kNearDone;
+            __syncwarp();
+            if (lane == 0) sts_release(&near_tail[ew], n_tail);
+        };
+        // The near rows of a chunk's two groups (bits of r0, r1; the columns from rank
+        // gj, their values in v) into the near queue.
+        auto queue_rows = [&](const float *v, uint32_t r0, uint32_t r1, uint32_t gj) {
+            const uint32_t lt = (1u << lane) - 1u, k0 = __popc(r0), k = k0 + __popc(r1);
+            if (((n_tail + k - n_head) & ~kNearDone) > p.near_cap)
+                n_head = __shfl_sync(0xffffffffu, lds_acquire(&near_head[ew]), 0);
+            if (((n_tail + k - n_head) & ~kNearDone) <= p.near_cap) {
+                if ((r0 >> lane) & 1u) put_row(v, __popc(r0 & lt), gj);
+                if ((r1 >> lane) & 1u) put_row(v + 32, k0 + __popc(r1 & lt), gj + 32);
+                publish(k);
+                return;
+            }
+            // no room for all of them: one by one
+            while (r0 | r1) {
+                if (!wait_room()) return;  // (the count is void)
+                const uint32_t first = r0 ? r0 & (0u - r0) : r1 & (0u - r1);
+                if (r0) {
+                    if ((first >> lane) & 1u) put_row(v, 0, gj);
+                    r0 ^= first;
+                } else {
+                    if ((first >> lane) & 1u) put_row(v + 32, 0, gj + 32);
+                    r1 ^= first;
                 }
-                n_slot = n_slot + take < p.near_cap ? n_slot + take : n_slot + take - p.near_cap;
-                n_tail = (n_tail + take) & ~kNearDone;
-                rows &= ~__ballot_sync(0xffffffffu, put);
-                __syncwarp();
-                if (lane == 0) sts_release(&near_tail[ew], n_tail);
+                publish(1);
             }
         };
         Rows rn{};
@@ -976,8 +1009,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             float4 gmin32 = rn.gmin;
             const bool more = it + stride < p.n_items;
             if (more) rn = load_rows(wn);
-            // testing hook: every pair is estimated
-            float thr_fast = p.dbg != nullptr && row_ok ? 3.0e38f : thr_out;
+            // rows that are not counted compare false (NaN); testing hook: every pair
+            // is estimated
+            const float thr_none = __int_as_float(0x7fc00000);
+            float thr_fast = !row_ok ? thr_none : (p.dbg != nullptr ? 3.0e38f : thr_out);
             uint32_t gj = w.b0 * kTcTileB + half * kEpiCols;
             const uint32_t gj_end = w.b1 * kTcTileB;
             // after the item's last tile, the next item's first (prefetch)
@@ -1001,7 +1036,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     na = p_row + D;
                     thr_out = row_ok ? (t_hi + tau) - p_row - D + marg : -3.0e38f;
                     thr_in = row_ok ? (t_lo - tau) - p_row - D - marg : -3.0e38f;
-                    thr_fast = p.dbg != nullptr && row_ok ? 3.0e38f : thr_out;
+                    thr_fast = !row_ok ? thr_none : (p.dbg != nullptr ? 3.0e38f : thr_out);
                     prefetch(gj + kTcTileB < gj_end ? gj + kTcTileB : gj_next);
                 }
                 float gmin[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1036,15 +1071,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     // exact); one vote for the chunk
                     const float m0 = fmaf(-2.0f, max32(v), c ? gmin[2] : gmin[0]);
                     const float m1 = fmaf(-2.0f, max32(v + 32), c ? gmin[3] : gmin[1]);
-                    if (!__any_sync(0xffffffffu, fminf(m0, m1) <= thr_fast)) continue;
-                    // groups of a few near rows go to the queue
                     const uint32_t r0 = __ballot_sync(0xffffffffu, m0 <= thr_fast);
                     const uint32_t r1 = __ballot_sync(0xffffffffu, m1 <= thr_fast);
-                    const uint32_t k0 = __popc(r0), k1 = __popc(r1);
-                    constexpr uint32_t kNearDense = BC ? kNearDenseBc : kNearDenseOne;
-                    const bool dense0 = k0 > kNearDense, dense1 = k1 > kNearDense;
-                    if (!dense0) queue_rows(v, r0, gj + c);
-                    if (!dense1) queue_rows(v + 32, r1, gj + c + 32);
+                    if ((r0 | r1) == 0) continue;
+                    // groups of a few near rows go to the queue
+                    constexpr int kNearDense = BC ? kNearDenseBc : kNearDenseOne;
+                    const bool dense0 = __popc(r0) > kNearDense, dense1 = __popc(r1) > kNearDense;
+                    if ((r0 && !dense0) || (r1 && !dense1)) queue_rows(v, dense0 ? 0u : r0, dense1 ? 0u : r1, gj + c);
                     if (dense0) dense_rows(v, (r0 >> lane) & 1u, gj + c);
                     if (dense1) dense_rows(v + 32, (r1 >> lane) & 1u, gj + c + 32);
                     if (p.dbg != nullptr && gi < p.na) {  // testing hook: every estimate
