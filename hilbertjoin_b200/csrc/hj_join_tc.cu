@@ -42,8 +42,8 @@
 // What bounds it (one B200, 1.965 GHz, distance kernel alone, before -> after the
 // epilogue took this form): one global centre, 1M x 64 FP16, 32 neighbours: 79.7 ->
 // 69 ms; 200k x 64: 4.25 -> 3.4; 200k x 200k x 20 (folded norms): 15.4 -> 6.0; 30k x
-// 70k x 100: 1.17 -> 0.54; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
-// clustered FP16: 53 -> 37.9; 300k x 32 TF32: 2.9 -> 1.93. At K = 64 a tile's MMAs
+// 70k x 100: 1.17 -> 0.49; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
+// clustered FP16: 53 -> 37.3; 300k x 32 TF32: 2.9 -> 1.89. At K = 64 a tile's MMAs
 // take 512 clocks and a tile without near rows about 1100: the chain MMA -> commit
 // -> TMEM load -> release -> MMA over two accumulators. Near rows add the rest. An
 // instruction of the epilogue costs its warp four to six clocks and a ready barrier,
@@ -113,9 +113,10 @@ constexpr uint32_t kNearWords = 44;
 constexpr uint32_t kNearCap = 24;    // entries per warp, at most
 // A group with more near rows is classified by the epilogue warp (lane = row): about
 // 1000 clocks however many rows, against the queue's per-row cost. With one centre, 30k x
-// 70k x 100: 0.54 ms at 3, 0.62 at 6; 1M x 64: 78 ms at 0, 69 at 3, 68 at 6. Block
-// centres, 4M x 28: 37.9 ms at 6, 40.5 at 8.
-constexpr int kNearDenseBc = 6, kNearDenseOne = 3;
+// 70k x 100: 0.54 ms at 0, 0.50 at 1, 0.49 at 2, 0.54 at 3, 0.62 at 6; 1M x 64: 80, 70,
+// 69, 69, 68 ms. Block centres, 4M x 28: 38.8 ms at 2, 37.7 at 3, 37.3 at 4, 37.9 at 6,
+// 40.5 at 8.
+constexpr int kNearDenseBc = 4, kNearDenseOne = 2;
 constexpr uint32_t kNearMinCap = 8;  // fewer entries than this are not worth a B stage
 // Rows that a near warp waits for before it starts on a batch, unless a queue is half
 // full, instead of at the first row: 200k x 200k x 20 6.7 -> 6.35 ms, 1M x 64 72 -> 69.6;
