@@ -88,8 +88,9 @@ __device__ __forceinline__ void fma_dim(const double *pa, const double *pb, doub
         }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(kPlainThreads, 2) k_join_fp64(PlainArgs a) {
+// CTAS: CTAs per SM that the registers are held to (kPlainDims3 says which).
+template <int MODE, int CTAS>
+__global__ void __launch_bounds__(kPlainThreads, CTAS) k_join_fp64(PlainArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_a, bar_full[2], bar_empty[2];
     const uint32_t d = a.d;
@@ -261,18 +262,34 @@ __global__ void __launch_bounds__(kPlainThreads, 2) k_join_fp64(PlainArgs a) {
     }
 }
 
-template <int MODE>
+// Three CTAs per SM up to the dims where shared memory holds three: FP64 issue waits on
+// the 16-lane pipe and on the B stages, and a third CTA fills the gaps. Two -> three:
+// d = 16, 20k points 180 -> 165 us; d = 40, 50k points 6.40 -> 5.87 ms; four spill.
+// Above, the tighter register bound alone costs up to 2.5% (d = 100, 30k points: 7.18
+// against 7.36 ms).
+constexpr uint32_t kPlainDims3 = 48;
+static_assert(3 * (plain_smem_bytes(kPlainDims3) + 2048) <= 228 * 1024, "three CTAs of kPlainDims3 dims per SM");
+
+template <int MODE, int CTAS>
 static void launch_plain(const PlainArgs &a, uint64_t n_items, int num_sms, cudaStream_t st) {
     const size_t smem = plain_smem_bytes(a.d);
     // the largest this kernel ever needs (d = 128 and d = 256 both take 192 KB), set once
     static_assert(plain_smem_bytes(128) == plain_smem_bytes(kPlainMaxDims), "plain smem maximum");
-    ensure_max_dynamic_smem((const void *)k_join_fp64<MODE>, (int)plain_smem_bytes(kPlainMaxDims));
+    ensure_max_dynamic_smem((const void *)k_join_fp64<MODE, CTAS>, (int)plain_smem_bytes(kPlainMaxDims));
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_join_fp64<MODE>, kPlainThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_join_fp64<MODE, CTAS>, kPlainThreads, smem);
     if (per_sm < 1) per_sm = 1;
     uint64_t grid = (uint64_t)per_sm * num_sms;
     if (grid > n_items) grid = n_items;
-    k_join_fp64<MODE><<<(unsigned)grid, kPlainThreads, smem, st>>>(a);
+    k_join_fp64<MODE, CTAS><<<(unsigned)grid, kPlainThreads, smem, st>>>(a);
+}
+
+template <int MODE>
+static void launch_plain(const PlainArgs &a, uint64_t n_items, int num_sms, cudaStream_t st) {
+    if (a.d <= kPlainDims3)
+        launch_plain<MODE, 3>(a, n_items, num_sms, st);
+    else
+        launch_plain<MODE, 2>(a, n_items, num_sms, st);
 }
 
 static PlainArgs plain_args(const SortedSet &A, const SortedSet &B, bool self, uint64_t na_eff, uint64_t nb_eff,
