@@ -6,18 +6,17 @@
 // on AVX-512 FMAs, early exit every KBLOCK dims once all 64 exceed eps^2,
 // counted by sign bit, summed per thread (egojoin.cpp:466-474).
 //
-// Here a persistent CTA of 256 threads takes work items (an A tile of 64 EGO
-// ranks against a run of B tiles of 64 ranks) in Hilbert order. The A tile is
-// staged once per item and the B tiles are double-buffered, each by one 1D
-// bulk copy (cp.async.bulk, the non-tensor TMA) of its [d][64] FP64 block into
-// shared memory (above d = 128 by 64-dim chunks, which keeps d <= 256 within
-// 192 KB), completion tracked by mbarriers. Each thread owns a 4 x 4
-// block of pairs and evaluates the pair test exactly as the oracle defines it:
-// acc = fma(a_k - b_k, a_k - b_k, acc) in IEEE FP64, k = 0..d-1 in order,
-// count iff acc <= eps*eps. The partial sums never decrease, so a warp whose
-// 512 pairs all exceed eps^2 after some dims stops early (checked every 8
-// dims) without changing any decision. Counts are reduced by warp shuffles and
-// one 64-bit atomic per warp.
+// Here a persistent CTA of 256 threads takes work items (an A tile of 64 EGO ranks
+// against a run of B tiles of 64 ranks) in Hilbert order. The A tile is staged once
+// per item and the B tiles are double-buffered, each by one 1D bulk copy
+// (cp.async.bulk, the non-tensor TMA) of its [d][64] FP64 block into shared memory
+// (in chunks of dims above d = 49, plain_chunk_dims), completion tracked by
+// mbarriers. Each thread owns a 4 x 4 block of pairs and evaluates the pair test
+// exactly as the oracle defines it: acc = fma(a_k - b_k, a_k - b_k, acc) in IEEE
+// FP64, k = 0..d-1 in order, count iff acc <= eps*eps. The partial sums never
+// decrease, so a warp whose 512 pairs all exceed eps^2 after some dims stops early
+// (checked every 8 dims) without changing any decision. Counts are reduced by warp
+// shuffles and one 64-bit atomic per warp.
 //
 // The same kernel materialises the pairs (hj_self_join_pairs / hj_join_pairs) in
 // kModeEmit: every qualifying pair goes to the output arrays as (input index of the A
@@ -52,10 +51,29 @@ enum PlainMode { kModeCount = 0, kModeEmit = 1 };
 constexpr int kPlainThreads = 256;
 constexpr int kPlainWarps = kPlainThreads / 32;
 
-// Dims per B stage: the whole tile up to d = 128; above, 64-dim chunks, so that
-// the A tile (d <= 256: at most 128 KB) and two B stages fit one CTA's smem.
-__host__ __device__ constexpr uint32_t plain_chunk_dims(uint32_t d) { return d <= 128 ? d : 64; }
 constexpr uint32_t kPlainMaxDims = 256;
+
+// CTAs per SM, and dims per B stage. A CTA holds its A tile and two B stages; the stages
+// are cut to chunks of dims (multiples of 8, at least 16) where that lets one more CTA
+// onto the SM, since FP64 issue waits on the pipe, the loads and the stages' barriers and
+// another CTA fills the gaps. Two CTAs -> three (whole tiles up to 49 dims): d = 16, 20k
+// points 180 -> 165 us; d = 40, 50k points 6.40 -> 5.87 ms; four spill. With chunks: d =
+// 64, 20k points 1.69 -> 1.59 ms; d = 100, 30k 6.98 -> 6.01 (one CTA -> three); d = 116,
+// 30k 8.05 -> 7.15; d = 128, 20k 4.05 -> 3.69 (one -> two); d = 192, 20k 6.20 -> 5.91.
+// `plain_rows`: 512-byte rows of dims that a CTA may hold.
+__host__ __device__ constexpr uint32_t plain_rows(uint32_t ctas) {
+    return ((228u * 1024u) / ctas - 2048u) / (kPlainTile * 8u);
+}
+__host__ __device__ constexpr uint32_t plain_ctas(uint32_t d) {
+    return d + 32 <= plain_rows(3) ? 3 : (d + 32 <= plain_rows(2) ? 2 : 1);
+}
+__host__ __device__ constexpr uint32_t plain_chunk_dims(uint32_t d) {
+    const uint32_t ctas = plain_ctas(d);
+    const uint32_t most = ctas == 1 ? 64 : (plain_rows(ctas) - d) / 2;  // dims that fit a stage
+    if (d <= most) return d;
+    const uint32_t chunks = (d + (most & ~7u) - 1) / (most & ~7u);
+    return ((d + chunks - 1) / chunks + 7) & ~7u;
+}
 
 __host__ __device__ constexpr size_t plain_smem_bytes(uint32_t d) {
     return ((size_t)d + 2 * plain_chunk_dims(d)) * kPlainTile * sizeof(double);
@@ -102,7 +120,7 @@ __device__ __forceinline__ int least_high(const double (&acc)[4][4]) {
     return m;
 }
 
-// CTAS: CTAs per SM that the registers are held to (kPlainDims3 says which).
+// CTAS: CTAs per SM that the registers are held to (plain_ctas).
 template <int MODE, int CTAS>
 __global__ void __launch_bounds__(kPlainThreads, CTAS) k_join_fp64(PlainArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -269,19 +287,11 @@ __global__ void __launch_bounds__(kPlainThreads, CTAS) k_join_fp64(PlainArgs a) 
     }
 }
 
-// Three CTAs per SM up to the dims where shared memory holds three: FP64 issue waits on
-// the 16-lane pipe and on the B stages, and a third CTA fills the gaps. Two -> three:
-// d = 16, 20k points 180 -> 165 us; d = 40, 50k points 6.40 -> 5.87 ms; four spill.
-// Above, the tighter register bound alone costs up to 2.5% (d = 100, 30k points: 7.18
-// against 7.36 ms).
-constexpr uint32_t kPlainDims3 = 48;
-static_assert(3 * (plain_smem_bytes(kPlainDims3) + 2048) <= 228 * 1024, "three CTAs of kPlainDims3 dims per SM");
-
 template <int MODE, int CTAS>
 static void launch_plain(const PlainArgs &a, uint64_t n_items, int num_sms, cudaStream_t st) {
     const size_t smem = plain_smem_bytes(a.d);
-    // the largest this kernel ever needs (d = 128 and d = 256 both take 192 KB), set once
-    static_assert(plain_smem_bytes(128) == plain_smem_bytes(kPlainMaxDims), "plain smem maximum");
+    // the largest this kernel ever needs, set once
+    static_assert(plain_smem_bytes(kPlainMaxDims) == 192 * 1024, "plain smem maximum");
     ensure_max_dynamic_smem((const void *)k_join_fp64<MODE, CTAS>, (int)plain_smem_bytes(kPlainMaxDims));
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_join_fp64<MODE, CTAS>, kPlainThreads, smem);
@@ -293,7 +303,7 @@ static void launch_plain(const PlainArgs &a, uint64_t n_items, int num_sms, cuda
 
 template <int MODE>
 static void launch_plain(const PlainArgs &a, uint64_t n_items, int num_sms, cudaStream_t st) {
-    if (a.d <= kPlainDims3)
+    if (plain_ctas(a.d) == 3)
         launch_plain<MODE, 3>(a, n_items, num_sms, st);
     else
         launch_plain<MODE, 2>(a, n_items, num_sms, st);

@@ -1,5 +1,5 @@
-"""Plain form on both sides of the dims where its kernel goes from three CTAs per SM to
-two: counts and pair lists against the brute-force oracle."""
+"""Plain form on both sides of the dims where its kernel changes the CTAs per SM or the
+dims per B stage: counts and pair lists against the brute-force oracle."""
 import numpy as np
 import pytest
 
@@ -17,7 +17,7 @@ def hj():
     return hj
 
 
-@pytest.mark.parametrize("d", [1, 47, 48, 49, 50])
+@pytest.mark.parametrize("d", [1, 47, 48, 49, 50, 115, 116, 117, 191, 192, 193, 256])
 def test_counts_and_pairs(hj, d):
     x = np.random.default_rng(d).random((1500, d))
     # eps^2 one standard deviation below the mean of |x - y|^2 (d / 6, variance 7 d / 180)
