@@ -404,8 +404,7 @@ void launch_dim_cost(const void *x, int dtype_bytes, uint64_t n, uint32_t d, dou
 // Packing with the rows staged in shared memory: a block of kPkRows threads
 // packs kPkRows consecutive points, whose rows form one contiguous range of
 // kPkRows * d coordinates. The block loads it with 128-bit loads (coalesced)
-// into a [d][kPkRows] layout, so that thread t then reads its own row with
-// consecutive threads on consecutive banks. The quantised norm key of the
+// into shared memory (stage_rows), where thread t then reads its own row. The quantised norm key of the
 // tensor-core forms comes out of the same pass (norm_key != null): the rows
 // are read from memory once for both. Rows of up to 512 bytes (d <= 128 FP32,
 // d <= 64 FP64) take this path.
@@ -426,8 +425,8 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
                                                               const double *__restrict__ center, double nscale,
                                                               uint32_t *__restrict__ norm_key, bool vec) {
     extern __shared__ __align__(16) unsigned char pk_smem[];
-    T *cols = reinterpret_cast<T *>(pk_smem);  // [d][kPkRows]
-    PkPos *prm = reinterpret_cast<PkPos *>(pk_smem + (size_t)d * kPkRows * sizeof(T));  // [d] (16-byte aligned)
+    T *rows = reinterpret_cast<T *>(pk_smem);  // [kPkRows][stage_pitch(d)]
+    PkPos *prm = reinterpret_cast<PkPos *>(rows + (size_t)kPkRows * stage_pitch(d));  // [d] (16-byte aligned)
     double *cen = reinterpret_cast<double *>(prm + d);                                 // [d]
     for (uint32_t pos = threadIdx.x; pos < d; pos += kPkRows) {
         if (pos < g.dk) {
@@ -438,37 +437,12 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
     }
     const uint64_t r0 = (uint64_t)blockIdx.x * kPkRows;
     const uint32_t m = (uint32_t)(n - r0 < (uint64_t)kPkRows ? n - r0 : kPkRows);
-    const uint32_t ne = m * d;
-    const T *src = x + r0 * d;
-    const float inv_d = 1.0f / (float)d;
-    // element e of the block's range -> (row e / d, col e % d); e < 2^17, so
-    // the FP32 quotient is off by at most one and one correction step fixes it
-    auto put = [&](uint32_t e, T v) {
-        uint32_t r = (uint32_t)((float)e * inv_d);
-        int c = (int)e - (int)(r * d);
-        if (c < 0) c += (int)d, --r;
-        if (c >= (int)d) c -= (int)d, ++r;
-        cols[(uint32_t)c * kPkRows + r] = v;
-    };
-    constexpr uint32_t V = 16 / sizeof(T);
-    if (vec) {
-        const uint32_t nv = ne / V;
-        const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
-        for (uint32_t u = threadIdx.x; u < nv; u += kPkRows) {
-            const uint4 q = __ldg(s4 + u);
-            T v[V];
-            memcpy(v, &q, 16);
-#pragma unroll
-            for (uint32_t j = 0; j < V; ++j) put(u * V + j, v[j]);
-        }
-        for (uint32_t e = nv * V + threadIdx.x; e < ne; e += kPkRows) put(e, __ldg(src + e));
-    } else {
-        for (uint32_t e = threadIdx.x; e < ne; e += kPkRows) put(e, __ldg(src + e));
-    }
+    stage_rows(x + r0 * d, m, d, rows, (uint32_t)kPkRows, vec);
     __syncthreads();
     const uint32_t t = threadIdx.x;
     if (t >= m) return;
     const uint64_t i = r0 + t;
+    const T *row = rows + (size_t)t * stage_pitch(d);
     uint32_t cur_word = 0, acc = 0;
     for (uint32_t pos = 0; pos < g.dk; ++pos) {
         const PkPos pp = prm[pos];
@@ -479,7 +453,7 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
             cur_word = w;
             acc = 0;
         }
-        const double c = cell_of((double)cols[pp.dim * kPkRows + t], eps, inv_eps);
+        const double c = cell_of((double)row[pp.dim], eps, inv_eps);
         const long long dig = (long long)c - pp.off;
         acc |= (uint32_t)dig << (pp.word_shift & 255u);
     }
@@ -488,7 +462,7 @@ __global__ void __launch_bounds__(kPkRows) k_pack_keys_staged(const T *__restric
     if (norm_key) {
         double sum = 0.0;
         for (uint32_t k = 0; k < d; ++k) {
-            const double v = (double)cols[k * kPkRows + t] - cen[k];
+            const double v = (double)row[k] - cen[k];
             sum = fma(v, v, sum);
         }
         const double q = floor(sum * nscale);
@@ -503,9 +477,9 @@ void launch_pack_keys(const void *x, int dtype_bytes, uint64_t n, uint32_t d, do
     const bool vec = ((uintptr_t)x & 15u) == 0;
     if ((uint64_t)d * dtype_bytes <= kPkMaxRowBytes) {
         const unsigned blocks = (unsigned)hj_ceil_div(n, kPkRows);
-        // rows (<= 64 KB; a multiple of 16 bytes), then the positions and the centre
-        const size_t smem = (size_t)kPkRows * d * dtype_bytes + (size_t)d * (sizeof(PkPos) + 8);
-        const int smem_max = (int)(64 * 1024 + (kPkMaxRowBytes / 4) * (sizeof(PkPos) + 8));
+        // rows (a multiple of 16 bytes), then the positions and the centre
+        const size_t smem = (size_t)kPkRows * stage_pitch(d) * dtype_bytes + (size_t)d * (sizeof(PkPos) + 8);
+        const int smem_max = (int)(kPkRows * (kPkMaxRowBytes + 8) + (kPkMaxRowBytes / 4) * (sizeof(PkPos) + 8));
         if (dtype_bytes == 8) {
             ensure_max_dynamic_smem((const void *)k_pack_keys_staged<double>, smem_max);
             k_pack_keys_staged<double><<<blocks, kPkRows, smem, st>>>(static_cast<const double *>(x), n, d, eps,

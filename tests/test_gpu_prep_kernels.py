@@ -109,3 +109,23 @@ def test_stripe_runs_merge(hj, active, kind):
             assert g2 == want and s2["tile_pairs"] == st["tile_pairs"]
     rows = -(-n // 64)
     assert st["tile_pairs"] <= rows * rows
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("d", [2, 5, 33, 64, 65, 128, 129])
+def test_index_on_cell_borders(hj, dtype, d):
+    # coordinates on, and one ulp beside, the borders of cells of eps: the index takes the
+    # neighbour cells from the point's own cell only clear of them. 512-byte rows and
+    # longer ones.
+    rng = np.random.default_rng(d)
+    eps = 0.3
+    x = rng.integers(-3, 4, size=(700, d)) * eps * rng.choice([0.0, 0.5, 1.0], size=d, p=[0.6, 0.2, 0.2])
+    x[:, 0] = rng.integers(-40, 40, size=700) * eps
+    x = x.astype(dtype)
+    x = np.where(rng.random(x.shape) < 0.3, np.nextafter(x, dtype(np.inf)), x)
+    x = np.where(rng.random(x.shape) < 0.3, np.nextafter(x, dtype(-np.inf)), x).astype(dtype)
+    x[350:] = x[:350]
+    x[350:, 0] += dtype(eps)  # partners at about eps
+    want = O.self_count_brute(x.astype(np.float64), eps)
+    assert want > 0
+    assert hj.self_join_count(x, eps, form="plain") == want
