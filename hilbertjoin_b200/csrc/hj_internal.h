@@ -7,6 +7,7 @@
 
 #include <string.h>
 
+#include <limits>
 #include <string>
 #include <vector>
 
@@ -194,7 +195,10 @@ BcConsts bc_constants(int form, uint32_t d, double T, double op_scale);
 void launch_bc_prepare(const SortedSet &s, const double *center, double scale, void *op, void *op_lo, float *norms,
                        float *xn, float4 *blk, float *cent, cudaStream_t st, int *launches);
 
-constexpr float kPadNorm = 1.0e30f;
+// The norm of a padding row: no real row's (TF32 and BF16x3 operands are unscaled, and
+// |x| < 1e18 in d <= 256 dims gives norms up to 2.6e38, still finite in FP32), so that
+// the norm summaries tell padding apart by it at every scale.
+constexpr float kPadNorm = std::numeric_limits<float>::infinity();
 
 // Work item of the persistent distance kernels: A tile `a` against the B tiles
 // [b0, b1). Produced by the index stage in Hilbert order.

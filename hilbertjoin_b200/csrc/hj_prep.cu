@@ -1346,7 +1346,7 @@ __global__ void __launch_bounds__(32 * kNormTilesPerBlock) k_norm_summaries(cons
     float mx = 0.0f, mn = 3.0e38f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        if (v[i] < 1e29f) mx = fmaxf(mx, v[i]);
+        if (v[i] < kPadNorm) mx = fmaxf(mx, v[i]);
         mn = fminf(mn, v[i]);
     }
 #pragma unroll
