@@ -115,7 +115,8 @@ static int batch_enqueue(hj_batch *b, cudaStream_t st) {
     if (launch_join_tc(b->ops, b->ops, b->form, b->d_jobs, 0, 0, b->idx, b->band, b->band_cap, b->d_band_total,
                        b->d_err, b->num_sms, st, &err, nullptr, b->d_band_total + 1))
         return engine_fail(HJ_ERR_CUDA, err);
-    launch_recheck(b->d_jobs, b->dtype, b->band, b->d_band_total, b->band_cap, b->d_maxerr, st);
+    launch_recheck(b->d_jobs, b->dtype, b->band, b->d_band_total, b->band_cap, b->d_maxerr, st, false, b->ops.norms,
+                   b->ops.norms);
     for (const FpJob &f : b->fp)
         launch_join_fp64(f.A, f.B, f.self, f.na_eff, f.nb_eff, f.T, f.idx, b->d_counts + f.job, b->d_err,
                          b->num_sms, st);

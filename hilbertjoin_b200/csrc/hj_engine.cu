@@ -801,7 +801,8 @@ static int run_join(Ctx *c, const JoinIn &in, const hj_opts *opts, uint64_t *cou
                 const bool vec_rows = ((uint64_t)d * A.dtype_bytes) % 16 == 0 &&
                                       ((uintptr_t)A.rows & 15u) == 0 && ((uintptr_t)B.rows & 15u) == 0;
                 launch_recheck(c->d_job, A.dtype_bytes, band, d_band, cap,
-                               reinterpret_cast<unsigned int *>(c->d_small + 5), st, vec_rows);
+                               reinterpret_cast<unsigned int *>(c->d_small + 5), st, vec_rows, bc ? nullptr : A.norms,
+                               bc ? nullptr : B.norms);
                 ++launches;
                 cudaEventRecord(c->ev[5], st);
                 cudaMemcpyAsync(c->h_small + 2, c->d_small + 2, 6 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,

@@ -128,7 +128,8 @@ constexpr uint64_t kIdleLimitNs = 600000000000ull;  // the near warps' longest r
 
 struct BandEntry {
     uint32_t ia, jb;  // EGO ranks in A and B
-    float s_hat;      // tensor-core estimate of dist^2
+    float s_hat;      // one centre: the pair's accumulator value, from which the recheck forms the
+                      // estimate of dist^2; block centring: the estimate, NaN where not kept
     uint32_t pad;
 };
 
@@ -275,6 +276,19 @@ __device__ __forceinline__ float max32(const float *v) {
     const float u0 = fmax3(t[0], t[1], t[2]), u1 = fmax3(t[3], t[4], t[5]);
     const float u2 = fmax3(t[6], t[7], t[8]), u3 = fmax3(t[9], v[30], v[31]);
     return fmaxf(fmax3(u0, u1, u2), u3);
+}
+
+// v[j] of 32 values in registers: a tree of selects (31; an index would put v in local
+// memory).
+__device__ __forceinline__ float pick32(const float *v, int j) {
+    float t[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) t[i] = (j & 16) ? v[16 + i] : v[i];
+#pragma unroll
+    for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) t[i] = (j & h) ? t[h + i] : t[i];
+    return t[0];
 }
 
 // Shared-memory matrix descriptor: K-major operand in 128-byte swizzle atoms
@@ -739,8 +753,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     while (bbits) {
                         const int j = __ffs(bbits) - 1;
                         bbits &= bbits - 1;
-                        const float t = fmaf(-2.0f, ent[j], BC || u.z ? 0.f : __ldg(p.norm_b + u.x + j));
-                        band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j, (q.x + t) * p.jobs[ejob].s_unscale, ejob);
+                        const float w = ent[j];
+                        band.store(sl.at(rank++), __float_as_uint(q.w), u.x + j,
+                                   BC ? fmaf(-2.0f, w, q.x) * p.jobs[ejob].s_unscale : w, ejob);
                     }
                 }
                 __syncwarp();  // the rows have been read
@@ -894,10 +909,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             thr_in = (T_lo - tau_max) - na - marg;
             if (!row_ok) thr_out = thr_in = -3.0e38f;
         };
-        // Band entries of a lane's row: the columns `bbits` of the 32 from rank gj.
-        // Ranks by a warp prefix sum, slots from one warp-wide reservation. The
-        // estimates are not kept here: NaN, which the recheck's error statistic skips.
-        auto put_band_bits = [&](uint32_t bbits, uint32_t gj) {
+        // Band entries of a lane's row: the columns `bbits` of the 32 from rank gj, whose
+        // values are v. Ranks by a warp prefix sum, slots from one warp-wide reservation.
+        // The error statistic reads the estimates: with one centre the pair's value is
+        // kept (200k x 20 3.13 -> 3.18 ms, 100k x 100 1.096 -> 1.108, 20k x 32 with eps at
+        // the median 0.182 -> 0.196) and the recheck forms the estimate from it; formed
+        // here, 3.19, 1.118 and 0.204. With block centres the value alone would not do,
+        // and keeping the estimate took 2M x 28 clustered from 7.3 to 8.1 ms: NaN there.
+        auto put_band_bits = [&](const float *v, uint32_t bbits, uint32_t gj) {
             if (!__any_sync(0xffffffffu, bbits != 0)) return;
             const uint32_t nbits = __popc(bbits);
             uint32_t incl = nbits;
@@ -911,7 +930,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             while (bbits) {
                 const int j = __ffs(bbits) - 1;
                 bbits &= bbits - 1;
-                band.store(sl.at(rank++), gi, gj + j, __int_as_float(0x7fc00000), job);
+                band.store(sl.at(rank++), gi, gj + j, BC ? __int_as_float(0x7fc00000) : pick32(v, j), job);
             }
         };
         // Groups of 32 columns in which many rows are near: every lane classifies its
@@ -943,7 +962,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
             g_in &= colmask;
             cnt += __popc(g_in);
-            put_band_bits(g_out & colmask & ~g_in, gj);
+            put_band_bits(v, g_out & colmask & ~g_in, gj);
         };
         // waits until the near queue has room for a row; false: the error word is set
         auto wait_room = [&]() -> bool {
@@ -1111,8 +1130,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
 // ---------------------------------------------------------------- recheck
 
 // FP64 pair test (the oracle's) on every band pair, against the pair's job
-// (BandEntry.pad); also the largest |s_hat - dist2| seen, as FP32 bits in
-// max_err_bits.
+// (BandEntry.pad); also the largest |estimate - dist2| seen, as FP32 bits in
+// max_err_bits. norm_a, norm_b: the squared norms per rank with one centre, whose
+// entries hold accumulator values (the column norm is in those of folded jobs); null
+// with block centres.
 // 16-byte loads of both rows where the rows allow it (every job's d * sizeof(TIn)
 // a multiple of 16: `vec`); the FP64 sum runs over the dims in order either way.
 template <typename TIn>
@@ -1144,7 +1165,8 @@ __device__ __forceinline__ double pair_dist2(const TIn *a, const TIn *b, uint32_
 
 template <typename TIn>
 __global__ void k_recheck(const TcJob *__restrict__ jobs, const BandEntry *__restrict__ band,
-                          const unsigned long long *band_total, uint64_t cap, unsigned int *max_err_bits, bool vec) {
+                          const unsigned long long *band_total, uint64_t cap, unsigned int *max_err_bits, bool vec,
+                          const float *__restrict__ norm_a, const float *__restrict__ norm_b) {
     const uint64_t n = min((unsigned long long)cap, *band_total);
     const uint32_t lane = threadIdx.x & 31u;
     float emax = 0.f;
@@ -1165,7 +1187,9 @@ __global__ void k_recheck(const TcJob *__restrict__ jobs, const BandEntry *__res
             c_acc = 0;
         }
         c_acc += acc <= J.T ? 1ull : 0ull;
-        emax = fmaxf(emax, (float)fabs((double)e.s_hat - acc));  // NaN estimates (not kept) are skipped
+        float s = e.s_hat;
+        if (norm_a) s = (__ldg(norm_a + e.ia) + fmaf(-2.0f, s, J.fold ? 0.f : __ldg(norm_b + e.jb))) * J.s_unscale;
+        emax = fmaxf(emax, (float)fabs((double)s - acc));  // NaN estimates (not kept) are skipped
     }
     // one atomic per warp when the warp's lanes end in the same job (the usual case)
     const uint32_t j0 = __shfl_sync(0xffffffffu, cur, 0);
@@ -1517,12 +1541,15 @@ uint64_t band_slack(int num_sms, bool bc) {
 }
 
 void launch_recheck(const TcJob *d_jobs, int dtype_bytes, const uint2 *band, const unsigned long long *d_band_total,
-                    uint64_t band_cap, unsigned int *d_max_err_bits, cudaStream_t st, bool vec_rows) {
+                    uint64_t band_cap, unsigned int *d_max_err_bits, cudaStream_t st, bool vec_rows,
+                    const float *norm_a, const float *norm_b) {
     const BandEntry *b = reinterpret_cast<const BandEntry *>(band);
     if (dtype_bytes == 8)
-        k_recheck<double><<<1184, 256, 0, st>>>(d_jobs, b, d_band_total, band_cap, d_max_err_bits, vec_rows);
+        k_recheck<double><<<1184, 256, 0, st>>>(d_jobs, b, d_band_total, band_cap, d_max_err_bits, vec_rows, norm_a,
+                                                norm_b);
     else
-        k_recheck<float><<<1184, 256, 0, st>>>(d_jobs, b, d_band_total, band_cap, d_max_err_bits, vec_rows);
+        k_recheck<float><<<1184, 256, 0, st>>>(d_jobs, b, d_band_total, band_cap, d_max_err_bits, vec_rows, norm_a,
+                                               norm_b);
 }
 
 void set_tc_debug_output(float *dbg) { g_dbg_out = dbg; }

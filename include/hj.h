@@ -143,7 +143,10 @@ typedef struct {
     uint64_t band_pairs;    /* pairs sent to the FP64 recheck */
     double band_fraction;   /* band_pairs / candidate_pairs */
     double band_halfwidth_rel; /* tensor-core bound: |dist2 - est| <= c * (|a|^2 + |b|^2) + abs; this is c */
-    double max_abs_err_band;   /* largest |est - dist2| over the band pairs (tensor-core forms) */
+    double max_abs_err_band;   /* largest |est - dist2| over the band pairs (tensor-core forms); with
+                                  block centring, over those found one by one: the estimates of a
+                                  group of 32 partners that many neighbouring points are near to
+                                  are not kept (0 if none was) */
     uint64_t fp64_items;    /* tensor-core forms: work items routed to the FP64 kernel because
                                their error band would exceed eps^2 / 2 */
     int32_t form_used;      /* hj_form actually run */
