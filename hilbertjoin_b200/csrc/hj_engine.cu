@@ -1418,6 +1418,13 @@ int hj_debug_set_wait_gate(uint64_t gate_ns) {
     return HJ_OK;
 }
 
+int hj_debug_set_near_limit(uint64_t limit_ns) {
+    tl_error.clear();
+    if (limit_ns > kWaitLimitNs) return fail(HJ_ERR_INVALID_ARG, "limit longer than the wait limit");
+    set_tc_near_limit(limit_ns);
+    return HJ_OK;
+}
+
 int hj_self_join_count_device(const void *pts, int dtype_bytes, uint64_t n, uint32_t d, double eps,
                               const hj_opts *opts, uint64_t *count, hj_stats *stats) {
     return join_device(pts, n, pts, n, dtype_bytes, d, eps, true, opts, count, stats);

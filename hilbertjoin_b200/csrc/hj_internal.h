@@ -396,6 +396,8 @@ void set_tc_debug_output(float *dbg);
 // Test hook: with ns > 0 the tensor-core kernel's epilogue first waits ns on a
 // barrier that nothing arrives on, then raises kErrTimeout (0 = off).
 void set_tc_wait_gate(uint64_t ns);
+// Test hook: the limit of the kernel's near warps (0 = the wait limit).
+void set_tc_near_limit(uint64_t ns);
 // Error-bound constant of a tensor-core form for dimension d.
 void tc_band_constants(int form, uint32_t d, double maxabs, bool fold, double *c_rel, double *c_abs);
 

@@ -124,8 +124,6 @@ constexpr uint32_t kNearMinCap = 8;  // fewer entries than this are not worth a 
 constexpr uint32_t kNearBatch = 24;
 constexpr uint32_t kNearDone = 0x80000000u;  // in a queue's tail: its warp has finished
 
-constexpr uint64_t kIdleLimitNs = 600000000000ull;  // the near warps' longest run: 10 minutes
-
 struct BandEntry {
     uint32_t ia, jb;  // EGO ranks in A and B
     float s_hat;      // one centre: the pair's accumulator value, from which the recheck forms the
@@ -157,6 +155,7 @@ struct TcArgs {
     uint32_t fold;                  // some job's norms are folded: the fold warp completes every A tile
     uint64_t gate_ns;               // test hook: > 0 makes the epilogue wait this long on a barrier
                                     // that nothing arrives on, then raise kErrTimeout
+    uint64_t near_ns;               // the near warps' limit for the queues to end after an error
     // per-block centring (BC kernels): norm_a is then q of the A rows (norm_b and
     // gmin_b unused: the accumulator holds w = v - q_j / 2); |h| of the A rows,
     // block summaries and centres of both sets
@@ -668,9 +667,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 if (lane == 0 && wc) atomicAdd(p.jobs[job].count, wc);
                 cnt = 0;
             };
-            // every epilogue warp ends its queue (its own waits are bounded), so this
-            // loop ends; the time limit is a second line only
-            const uint64_t t0 = globaltimer_ns();
+            // Every epilogue warp ends its queue: its own waits are bounded, and it stops
+            // at the next one once the error word is set. So the loop ends, however long
+            // the join; its own limit, a second line, runs from the first sight of an error.
+            uint64_t t_err = 0;
             for (uint32_t idle = 0;;) {
                 const uint32_t tail = mine ? lds_acquire(&near_tail[lane]) : kNearDone;
                 __syncwarp();  // the acquiring lanes' view becomes the warp's
@@ -681,9 +681,10 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 const bool last = __all_sync(0xffffffffu, (tail & kNearDone) != 0);
                 if (last && rows == 0) break;
                 if (!last && rows < kNearBatch && 2 * __reduce_max_sync(0xffffffffu, avail) < p.near_cap) {
-                    if ((++idle & 1023u) == 0 && globaltimer_ns() - t0 > kIdleLimitNs) {
-                        atomicOr((uint32_t *)err, kErrTimeout | (10u << 8));
-                        break;
+                    if ((++idle & 1023u) == 0 && __any_sync(0xffffffffu, *err != 0)) {
+                        const uint64_t now = __shfl_sync(0xffffffffu, globaltimer_ns(), 0);
+                        if (t_err == 0) t_err = now;
+                        if (now - t_err > p.near_ns) break;
                     }
                     __nanosleep(200);
                     continue;
@@ -1389,6 +1390,7 @@ BcConsts bc_constants(int form, uint32_t d, double T, double op_scale) {
 
 static float *g_dbg_out = nullptr;  // set by tests through hj_debug_tc_estimates
 static uint64_t g_gate_ns = 0;      // set by tests through hj_debug_set_wait_gate
+static uint64_t g_near_ns = kWaitLimitNs;  // set by tests through hj_debug_set_near_limit
 
 void fill_tc_job(TcJob *j, int form, uint32_t d, double T, double op_scale, double maxabs, uint64_t a_row0,
                  uint64_t na_eff, uint64_t b_row0, uint64_t nb_eff, bool self, unsigned long long *count,
@@ -1493,6 +1495,7 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
     a.perm_a = A.perm;
     a.perm_b = B.perm;
     a.gate_ns = g_gate_ns;
+    a.near_ns = g_near_ns;
     a.fold = !bc && A.fold ? 1u : 0u;
     if (bc) {
         a.norm_a = A.bc_norms;
@@ -1555,5 +1558,7 @@ void launch_recheck(const TcJob *d_jobs, int dtype_bytes, const uint2 *band, con
 void set_tc_debug_output(float *dbg) { g_dbg_out = dbg; }
 
 void set_tc_wait_gate(uint64_t ns) { g_gate_ns = ns; }
+
+void set_tc_near_limit(uint64_t ns) { g_near_ns = ns ? ns : kWaitLimitNs; }
 
 }  // namespace hj

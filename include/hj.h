@@ -293,6 +293,12 @@ HJ_API int hj_debug_tc_estimates_ex(const float *A, uint64_t nA, const float *B,
  * must not exceed the engine's wait limit (2 s). Not thread-safe; no
  * reference counterpart (the reference has no device waits). */
 HJ_API int hj_debug_set_wait_gate(uint64_t gate_ns);
+/* Testing hook: the time that the tensor-core kernel's near warps, which work
+ * off queued rows, go on waiting for the queues' end after an error was raised
+ * (0 restores the engine's wait limit, 2 s, which it must not exceed). A join
+ * without an error has no such limit, however long it runs. Not thread-safe;
+ * no reference counterpart. */
+HJ_API int hj_debug_set_near_limit(uint64_t limit_ns);
 
 /* ---------------------------------------------------------------- batching
  * Many joins of uneven n, d and eps in one persistent tensor-core launch. The
