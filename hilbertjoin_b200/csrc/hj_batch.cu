@@ -327,17 +327,20 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
         cudaError_t e = cudaGetLastError();
         return engine_fail(HJ_ERR_CUDA, std::string("batch planning: ") + cudaGetErrorString(e));
     }
-    // size the band queue with one run (regrown once if it overflows)
-    b->band_cap = std::max<uint64_t>(1ull << 20, b->candidate_pairs / 4096) + band_slack(b->num_sms, false);
+    // Size the band queue with one run. Every run has the same band pairs, but the
+    // slots that its warps leave unused differ with their timing: the queue holds the
+    // most that a later run can reserve.
+    const uint64_t slack = band_slack(b->num_sms, false);
+    b->band_cap = std::max<uint64_t>(1ull << 20, b->candidate_pairs / 4096) + slack;
     for (int attempt = 0; attempt < 3; ++attempt) {
         b->band = (uint2 *)b->alloc(b->band_cap * kBandEntryBytes);
         if (!b->band) return engine_fail(HJ_ERR_OOM, "out of device memory (band queue)");
         if (int r = batch_enqueue(b, st)) return r;
         uint64_t bt = 0;
         int r = batch_finish(b, &bt);
-        if (r == HJ_OK) return HJ_OK;
-        if (r != HJ_ERR_BAND_OVERFLOW) return r;
-        b->band_cap = bt + bt / 4 + 4096;
+        if (r == HJ_OK && bt + slack <= b->band_cap) return HJ_OK;
+        if (r != HJ_OK && r != HJ_ERR_BAND_OVERFLOW) return r;
+        b->band_cap = bt + bt / 4 + slack;
     }
     return engine_fail(HJ_ERR_BAND_OVERFLOW, "band queue overflow");
 }
