@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     drain_until(&bar_drain, 0, globaltimer_ns() + kWaitLimitNs);
                 }
             }
-        } else if (warp == kFoldWarp && p.fold) {
+        } else if (!kBf && warp == kFoldWarp && p.fold) {
             // ------------------------------------------------ A side of folded norms
             // A folded row holds the pieces of |x|^2 / 2 in its columns d .. d + 2.
             // As a B operand they meet the A side's constants; here those replace
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             for (uint64_t it = blockIdx.x; it < p.n_items; it += stride) {
                 const TcJob &J = p.jobs[p.items[it].pad];
                 const bool fold = J.fold != 0;
-                const uint32_t d = J.d, ka = J.ka;
+                const uint32_t d = J.d;
                 const bool landed = mbar_wait(&bar_afull[abuf], aph, err, 7);
                 if (!__all_sync(0xffffffffu, landed)) break;
                 if (fold) {
@@ -636,11 +636,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                                  (byte & 15u);
                             if constexpr (FORM == HJ_FORM_TC_TF32) {
                                 asm volatile("st.shared.b32 [%0], %1;" ::"r"(abase + off), "r"(0xBF800000u) : "memory");
-                            } else if constexpr (kBf) {  // -1 and 0
-                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"((uint16_t)0xBF80) : "memory");
-                                asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + ka * kAStageBytes + off),
-                                             "h"((uint16_t)0)
-                                             : "memory");
                             } else {  // -2^15, -2^4, -2^-7
                                 const uint16_t c = m == 0 ? 0xF800 : (m == 1 ? 0xCC00 : 0xA000);
                                 asm volatile("st.shared.b16 [%0], %1;" ::"r"(abase + off), "h"(c) : "memory");
@@ -1333,7 +1328,9 @@ static TcLayout tc_layout(int form, uint32_t d) {
     return L;
 }
 
-bool tc_fold(int form, uint32_t d) { return tc_layout(form, d + 3).ka == tc_layout(form, d).ka; }
+bool tc_fold(int form, uint32_t d) {
+    return form != HJ_FORM_TC_BF16X3 && tc_layout(form, d + 3).ka == tc_layout(form, d).ka;
+}
 uint32_t tc_atoms(int form, uint32_t kcols) { return tc_layout(form, kcols).ka; }
 uint32_t tc_ksteps(int form, uint32_t kcols) {
     const uint32_t k = form == HJ_FORM_TC_TF32 ? 8u : 16u;

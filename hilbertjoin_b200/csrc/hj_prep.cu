@@ -1195,7 +1195,7 @@ __device__ __forceinline__ void norm_pieces(double v, typename BcElem<OP>::E (&m
 // padding ranks kPadNorm). FP16 operands are (x - center) * scale rounded once
 // from FP64 (scale a power of two: exact); TF32 and BF16 from the FP32 value
 // of x - center, BF16 as hi + lo with lo the BF16 of the exact remainder.
-// With `fold`, columns d .. d + 2 hold the pieces of half the rank's norm
+// With `fold` (not BF16), columns d .. d + 2 hold the pieces of half the rank's norm
 // (norm_pieces; padding ranks a norm that no pair reaches).
 template <typename T, int OP>  // OP: 0 TF32, 1 BF16 hi/lo, 2 FP16
 __global__ void __launch_bounds__(256) k_gather_tc_fused(const T *__restrict__ x, uint64_t n, uint32_t d,
@@ -1267,18 +1267,13 @@ __global__ void __launch_bounds__(256) k_gather_tc_fused(const T *__restrict__ x
     part += __shfl_xor_sync(0xffffffffu, part, 2);
     part += __shfl_xor_sync(0xffffffffu, part, 1);
     if (in && j == 0) norms[r] = real ? (float)(part * scale2) : kPadNorm;
-    if (fold) {
-        __syncwarp();  // after the chunk stores of the same columns
-        if (in && j < 3) {
-            typename BcElem<OP>::E m[3];
-            norm_pieces<OP>(real ? 0.5 * (part * scale2) : (OP == 2 ? 0x1.ffcp30 : 1.0e30), m);
-            const typename BcElem<OP>::E e = j == 0 ? m[0] : (j == 1 ? m[1] : m[2]);
-            const uint64_t at = r * kp + d + j;
-            if (OP == 0) {
-                static_cast<uint32_t *>(op_hi)[at] = e;
-            } else {
-                static_cast<uint16_t *>(op_hi)[at] = (uint16_t)e;
-                if (OP == 1) op_lo[at] = (uint16_t)((uint32_t)e >> 16);
+    if constexpr (OP != 1) {
+        if (fold) {
+            __syncwarp();  // after the chunk stores of the same columns
+            if (in && j < 3) {
+                typename BcElem<OP>::E m[3];
+                norm_pieces<OP>(real ? 0.5 * (part * scale2) : (OP == 2 ? 0x1.ffcp30 : 1.0e30), m);
+                static_cast<typename BcElem<OP>::E *>(op_hi)[r * kp + d + j] = j == 0 ? m[0] : (j == 1 ? m[1] : m[2]);
             }
         }
     }
