@@ -117,7 +117,14 @@ constexpr uint32_t kNearCap = 24;    // entries per warp, at most
 // 69, 69, 68 ms. Block centres, 4M x 28: 38.8 ms at 2, 37.7 at 3, 37.3 at 4, 37.9 at 6,
 // 40.5 at 8.
 constexpr int kNearDenseBc = 4, kNearDenseOne = 2;
-constexpr uint32_t kNearMinCap = 8;  // fewer entries than this are not worth a B stage
+// Fewer entries than this are not worth a B stage, and so small a queue is not used:
+// where three B stages and the A tile leave no room (BF16x3 from d = 193, block-centred
+// from 62; TF32 from 225), rows would wait for one another's place, and a tile's MMAs
+// take 3700 clocks and more, behind which the warp classifies all near rows itself. One
+// entry -> none, 60k points, 8 and 64 neighbours: BF16x3 d = 256 2.11 -> 1.77 and 2.52 ->
+// 1.80 ms, TF32 256 1.67 -> 1.20 and 2.37 -> 1.33; block-centred BF16x3, 150k x 64
+// clustered 2.16 -> 1.31.
+constexpr uint32_t kNearMinCap = 8;
 // Rows that a near warp waits for before it starts on a batch, unless a queue is half
 // full, instead of at the first row: 200k x 200k x 20 6.7 -> 6.35 ms, 1M x 64 72 -> 69.6;
 // at 12 rows half of that.
@@ -137,6 +144,7 @@ struct TcArgs {
     uint32_t a_bufs;    // 1 or 2 A buffers
     uint32_t nst;       // B ring stages
     uint32_t near_cap;  // entries of each epilogue warp's near queue (>= 1)
+    int near_rows;      // most near rows of a group that go to the queue (0: it is not used)
     const WorkItem *items;
     uint64_t n_items;
     const float *norm_a, *norm_b;   // FP32 |x|^2 per EGO rank (padding: kPadNorm)
@@ -1091,8 +1099,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     const uint32_t r1 = __ballot_sync(0xffffffffu, m1 <= thr_fast);
                     if ((r0 | r1) == 0) continue;
                     // groups of a few near rows go to the queue
-                    constexpr int kNearDense = BC ? kNearDenseBc : kNearDenseOne;
-                    const bool dense0 = __popc(r0) > kNearDense, dense1 = __popc(r1) > kNearDense;
+                    const bool dense0 = __popc(r0) > p.near_rows, dense1 = __popc(r1) > p.near_rows;
                     if ((r0 && !dense0) || (r1 && !dense1)) queue_rows(v, dense0 ? 0u : r0, dense1 ? 0u : r1, gj + c);
                     if (dense0) dense_rows(v, (r0 >> lane) & 1u, gj + c);
                     if (dense1) dense_rows(v + 32, (r1 >> lane) & 1u, gj + c + 32);
@@ -1474,6 +1481,7 @@ int launch_join_tc(const SortedSet &A, const SortedSet &B, int form, const TcJob
     a.a_bufs = L.a_bufs;
     a.nst = L.nst;
     a.near_cap = L.near_cap;
+    a.near_rows = L.near_cap < kNearMinCap ? 0 : (bc ? kNearDenseBc : kNearDenseOne);
     a.items = idx.items;
     a.n_items = idx.n_items;
     a.norm_a = A.norms;
