@@ -916,10 +916,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         // Band entries of a lane's row: the columns `bbits` of the 32 from rank gj, whose
         // values are v. Ranks by a warp prefix sum, slots from one warp-wide reservation.
         // The error statistic reads the estimates: with one centre the pair's value is
-        // kept (200k x 20 3.13 -> 3.18 ms, 100k x 100 1.096 -> 1.108, 20k x 32 with eps at
-        // the median 0.182 -> 0.196) and the recheck forms the estimate from it; formed
-        // here, 3.19, 1.118 and 0.204. With block centres the value alone would not do,
-        // and keeping the estimate took 2M x 28 clustered from 7.3 to 8.1 ms: NaN there.
+        // kept, and the recheck forms the estimate from it. With block centres the value
+        // alone would not do, and keeping the estimate took 2M x 28 clustered from 7.3 to
+        // 8.1 ms: NaN there.
         auto put_band_bits = [&](const float *v, uint32_t bbits, uint32_t gj) {
             if (!__any_sync(0xffffffffu, bbits != 0)) return;
             const uint32_t nbits = __popc(bbits);
@@ -938,8 +937,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             }
         };
         // Groups of 32 columns in which many rows are near: every lane classifies its
-        // own row from its registers.
-        auto dense_rows = [&](const float *v, bool need, uint32_t gj) {
+        // own row from its registers. With one centre, where hardly any of the rows has
+        // band pairs, those rows are left to the queue (the rows returned), which is
+        // cheaper than picking the values by their column. Values dropped -> all picked
+        // -> this: 200k x 20 3.20 -> 3.31 -> 3.24 ms, 150k x 8 0.635 -> 0.678 -> 0.656,
+        // 150k x 4 0.193 -> 0.225 -> 0.229, 20k x 32 with eps at the median 0.180 -> 0.193
+        // -> 0.200. With up to 4 or 6 rows left to the queue the last two take 0.25 and
+        // 0.22, and 0.26 and 0.35.
+        auto dense_rows = [&](const float *v, bool need, uint32_t gj) -> uint32_t {
             const uint32_t colmask = need && row_ok ? count_mask(gi, gj, b_end, self) : 0u;
             uint32_t g_in = 0, g_out = 0;
             if (BC || fold) {
@@ -965,8 +970,17 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 }
             }
             g_in &= colmask;
+            const uint32_t bbits = g_out & colmask & ~g_in;
+            if constexpr (!BC) {
+                const uint32_t rows = __ballot_sync(0xffffffffu, bbits != 0);
+                if (__popc(rows) <= p.near_rows) {
+                    cnt += bbits ? 0 : __popc(g_in);
+                    return rows;
+                }
+            }
             cnt += __popc(g_in);
-            put_band_bits(v, g_out & colmask & ~g_in, gj);
+            put_band_bits(v, bbits, gj);
+            return 0;
         };
         // waits until the near queue has room for a row; false: the error word is set
         auto wait_room = [&]() -> bool {
@@ -1100,9 +1114,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     if ((r0 | r1) == 0) continue;
                     // groups of a few near rows go to the queue
                     const bool dense0 = __popc(r0) > p.near_rows, dense1 = __popc(r1) > p.near_rows;
-                    if ((r0 && !dense0) || (r1 && !dense1)) queue_rows(v, dense0 ? 0u : r0, dense1 ? 0u : r1, gj + c);
-                    if (dense0) dense_rows(v, (r0 >> lane) & 1u, gj + c);
-                    if (dense1) dense_rows(v + 32, (r1 >> lane) & 1u, gj + c + 32);
+                    const uint32_t q0 = dense0 ? dense_rows(v, (r0 >> lane) & 1u, gj + c) : r0;
+                    const uint32_t q1 = dense1 ? dense_rows(v + 32, (r1 >> lane) & 1u, gj + c + 32) : r1;
+                    if (q0 | q1) queue_rows(v, q0, q1, gj + c);
                     if (p.dbg != nullptr && gi < p.na) {  // testing hook: every estimate
 #pragma unroll
                         for (int j = 0; j < kChunkCols; ++j)
