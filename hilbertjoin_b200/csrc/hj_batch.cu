@@ -84,6 +84,7 @@ struct hj_batch {
     std::vector<void *> allocs;
     cudaStream_t alloc_stream = nullptr;  // planning stream: buffers are stream-ordered on it
     uint64_t candidate_pairs = 0, fp64_items = 0;
+    uint64_t tc_pairs = 0;  // pairs in the tensor-core kernel's tiles
     std::vector<uint64_t> job_candidates;
 
     // Stream-ordered allocations (cudaMallocAsync): no device-wide
@@ -278,6 +279,7 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
             n_items += P.idx_tc.n_items;
         }
         b->candidate_pairs += P.idx_tc.candidate_pairs + P.idx_fp.candidate_pairs;
+        b->tc_pairs += P.idx_tc.tile_pairs * (uint64_t)kTcTileA * kTcTileB;
         b->job_candidates[j] = P.idx_tc.candidate_pairs + P.idx_fp.candidate_pairs;
         // items routed to the FP64 kernel keep their own plain tiles
         if (P.idx_fp.n_items) {
@@ -329,9 +331,10 @@ static int batch_plan(const hj_batch_job *jobs, uint32_t n_jobs, int dtype_bytes
     }
     // Size the band queue with one run. Every run has the same band pairs, but the
     // slots that its warps leave unused differ with their timing: the queue holds the
-    // most that a later run can reserve.
+    // most that a later run can reserve. Its first size is the single join's, 1/4096 of
+    // the pairs that the tensor-core kernel looks at.
     const uint64_t slack = band_slack(b->num_sms, false);
-    b->band_cap = std::max<uint64_t>(1ull << 20, b->candidate_pairs / 4096) + slack;
+    b->band_cap = std::max<uint64_t>(1ull << 20, b->tc_pairs / 4096) + slack;
     for (int attempt = 0; attempt < 3; ++attempt) {
         b->band = (uint2 *)b->alloc(b->band_cap * kBandEntryBytes);
         if (!b->band) return engine_fail(HJ_ERR_OOM, "out of device memory (band queue)");
