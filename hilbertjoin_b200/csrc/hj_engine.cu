@@ -222,18 +222,24 @@ static int plan_grid(const DimStats *ds, uint32_t d, double eps, double maxabs,
 
 // How much of the key a join of n points sorts by. What a count needs of the order is
 // the stripes (the active dims and the one after them, in which a stripe is a range)
-// and that a tile's points lie together; log2(n) and some bits of occupied cells
-// give that, and every further word is up to four radix passes and its share of the
-// key, bound and gather traffic. Whole joins, whole key -> 8 bits more than log2(n)
-// -> 24 bits more: 20k x 16 plain 0.536 -> 0.480 -> 0.553 ms, 200k x 200k x 20 7.43 ->
-// 7.20 -> 7.44, 300k x 32 clustered TF32 3.28 -> 2.87 -> 2.87, 4M x 28 clustered FP16
-// 45.4 -> 45.3 -> 44.2 (its sort 2.6 -> 1.4 -> 1.6, its block-centred kernel 38.1 ->
-// 39.9 -> 38.4: tiles are looser in the dims left out). ref_compat drops the last
-// points of the whole EGO order, so it keeps the whole key.
+// and that a tile's points lie together; every further word is up to four radix
+// passes and its share of the key, bound and gather traffic. So the key stops at the
+// first word boundary past those dims and past log2(n) bits and 8 (above 2^20 points
+// 24) more, counted in field widths: a field is as wide as its dim's range of cells
+// takes, 3 bits for two or three cells, also where single outliers widen it (one at
+// 1000 times the spread in every dim: 2M x 28 clustered 64.1 ms, whole key 83.6; 200k x
+// 16 plain 2.08, without outliers 1.93). Whole calls at 8 and at 24 bits: 20k x 16 plain
+// 0.480 and 0.553 ms (whole key 0.536); clustered, 28 dims, 100k 0.86 and 0.93, 265k 1.15
+// and 1.23, 1M 4.68 and 4.73, 2.5M 13.7 and 14.0, 4M 45.6 and 45.1; 32 dims TF32 300k 2.04
+// and 2.21, 1M 10.4 and 10.5, 2M 35.0 and 34.3; 20 dims FP16 1.6M 7.4 and 7.3, 4M 30.2
+// and 29.1; uniform, 20 dims, 300k 6.86 and 6.92. Up to a million points 8 bits are
+// slower by 3% at most and up to 8% faster; above, tiles looser in the dims left out
+// cost some sets more than the passes. ref_compat drops the last points of the whole
+// EGO order, so it keeps the whole key.
 static void key_budget(uint64_t n, int active_dims, bool ref_compat, uint32_t *min_dims, uint32_t *min_bits) {
     if (ref_compat) return;
     *min_dims = (uint32_t)active_dims + 1;
-    *min_bits = (uint32_t)bitwidth(n) + (n > (1u << 18) ? 24u : 8u);
+    *min_bits = (uint32_t)bitwidth(n) + (n > (1u << 20) ? 24u : 8u);
 }
 
 struct JoinIn {
