@@ -141,12 +141,12 @@ static int get_ctx(int device, Ctx **out) {
 // other still reads it.
 enum {
     kSlotInA = 1, kSlotInB, kSlotDimStats, kSlotGridOff, kSlotGridBits, kSlotGridWord, kSlotGridShift,
-    kSlotKeysWmA, kSlotKeysWmB, kSlotPermA, kSlotPermB, kSlotPermTmp, kSlotHist,
+    kSlotKeysWmA, kSlotKeysWmB, kSlotPermA, kSlotPermB, kSlotHist,
     kSlotRowsA, kSlotRowsB, kSlotKeysA, kSlotKeysB, kSlotTilesA, kSlotTilesB,
     kSlotTf32A, kSlotTf32B, kSlotHiA, kSlotLoA, kSlotHiB, kSlotLoB, kSlotNormA, kSlotNormB,
-    kSlotTmaxAA, kSlotTmaxAB, kSlotTmaxBA, kSlotTmaxBB, kSlotBand, kSlotCenter, kSlotGminA, kSlotGminB,
-    kSlotPairKeys, kSlotPairPerm, kSlotPairTmp, kSlotPairHist, kSlotPairOut, kSlotDimCost,
-    kSlotGridOrd, kSlotBcOpA, kSlotBcOpB, kSlotBcNormA, kSlotBcNormB, kSlotBcXnA, kSlotBcXnB, kSlotBcBlkA,
+    kSlotTmaxAA, kSlotTmaxAB, kSlotTmaxBA, kSlotTmaxBB, kSlotBand, kSlotGminA, kSlotGminB,
+    kSlotPairKeys, kSlotPairPerm, kSlotPairHist, kSlotPairOut, kSlotDimCost,
+    kSlotBcOpA, kSlotBcOpB, kSlotBcNormA, kSlotBcNormB, kSlotBcXnA, kSlotBcXnB, kSlotBcBlkA,
     kSlotBcBlkB, kSlotBcCentA, kSlotBcCentB, kSlotScanTiles, kSlotBcOpLoA, kSlotBcOpLoB,
     kSlotEngineEnd
 };
@@ -227,8 +227,7 @@ static int plan_grid(const DimStats *ds, uint32_t d, double eps, double maxabs,
 // first word boundary past those dims and past log2(n) bits and 8 (above 2^20 points
 // 24) more, counted in field widths: a field is as wide as its dim's range of cells
 // takes, 3 bits for two or three cells, also where single outliers widen it (one at
-// 1000 times the spread in every dim: 2M x 28 clustered 64.1 ms, whole key 83.6; 200k x
-// 16 plain 2.08, without outliers 1.93). Whole calls at 8 and at 24 bits: 20k x 16 plain
+// 1000 times the spread in every dim: 200k x 16 plain 2.08 ms, without 1.93). Whole calls at 8 and at 24 bits: 20k x 16 plain
 // 0.480 and 0.553 ms (whole key 0.536); clustered, 28 dims, 100k 0.86 and 0.93, 265k 1.15
 // and 1.23, 1M 4.68 and 4.73, 2.5M 13.7 and 14.0, 4M 45.6 and 45.1; 32 dims TF32 300k 2.04
 // and 2.21, 1M 10.4 and 10.5, 2M 35.0 and 34.3; 20 dims FP16 1.6M 7.4 and 7.3, 4M 30.2
@@ -419,8 +418,8 @@ struct Prepared {
 
 // Work list parameters of a distance kernel: the smallest item, the items that keep
 // the SMs balanced (the tensor-core kernel runs one CTA per SM and pays about two
-// tiles per item for its A tile and row data; the plain kernel two CTAs of small
-// tiles), and the operand bytes of the Hilbert rule. A caller's own chunk is kept.
+// tiles per item for its A tile and row data; the plain kernel one to three CTAs of
+// small tiles), and the operand bytes of the Hilbert rule. A caller's own chunk is kept.
 struct IndexPlan {
     uint32_t chunk_min, target;
     uint64_t operand_bytes;

@@ -162,7 +162,7 @@ static void launch_bound_keys(const BoundsArgs &a, cudaStream_t st) {
         ensure_max_dynamic_smem((const void *)k_bound_keys<T, true>, most);
         k_bound_keys<T, true><<<blocks, kBkRows, smem, st>>>(a);
     } else {
-        if (prm > 48 * 1024) ensure_max_dynamic_smem((const void *)k_bound_keys<T, false>, (int)prm);
+        static_assert(kMaxDim * sizeof(BkPos) <= 48 * 1024, "the positions fit without an attribute");
         k_bound_keys<T, false><<<blocks, kBkRows, prm, st>>>(a);
     }
 }

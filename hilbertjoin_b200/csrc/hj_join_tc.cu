@@ -39,16 +39,17 @@
 //     rows of the group are near, the group classified by the warp itself,
 //     branch-free from its registers.
 //
-// What bounds it (one B200, 1.965 GHz, distance kernel alone, before -> after the
-// epilogue took this form): one global centre, 1M x 64 FP16, 32 neighbours: 79.7 ->
-// 69 ms; 200k x 64: 4.25 -> 3.4; 200k x 200k x 20 (folded norms): 15.4 -> 6.0; 30k x
-// 70k x 100: 1.17 -> 0.49; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28
-// clustered FP16: 53 -> 37.3; 300k x 32 TF32: 2.9 -> 1.89. At K = 64 a tile's MMAs
+// What bounds it (one B200, distance kernel alone, before -> after the epilogue took
+// this form; SM clock 1.965 GHz, in the two longest 1.8 under the power limit): one
+// global centre, 1M x 64 FP16, 32 neighbours: 83.7 -> 76.4 ms; 600k x 64: 29.3 -> 27.7;
+// 200k x 64: 4.33 -> 3.46; 200k x 200k x 20 (folded norms): 15.1 -> 6.2; 30k x 70k x 100:
+// 1.18 -> 0.51; 150k x 128 BF16x3: 6.3 -> 5.2. Block centres, 4M x 28 clustered FP16:
+// 33.9 -> 27.1; 300k x 32 TF32: 1.63 -> 1.26 to 1.50. At K = 64 a tile's MMAs
 // take 512 clocks and a tile without near rows about 1100: the chain MMA -> commit
 // -> TMEM load -> release -> MMA over two accumulators. Near rows add the rest. An
 // instruction of the epilogue costs its warp four to six clocks and a ready barrier,
 // a vote or a tcgen05 fence 30 to 50, with two epilogue warps per scheduler; so the
-// tile loop is kept short: 64 columns per TMEM load, one vote per load, item data
+// tile loop is kept short: 64 columns per TMEM load, two votes per load, item data
 // one item ahead, group minima in registers (one load per 32 tiles). Measured and
 // dropped: 32-column loads double-buffered (more votes and waits: +25%), 128
 // columns at once (spills), two issuing warps, each set of four epilogue warps on
@@ -154,7 +155,7 @@ struct TcArgs {
     uint64_t na, nb;                // job 0's counted ranks (debug output only)
     BandEntry *band;
     uint64_t band_cap;
-    unsigned long long *band_total;  // slots reserved (chunks of kBandChunk per warp)
+    unsigned long long *band_total;  // slots reserved (chunks of kBandChunk or kBandChunkRare)
     unsigned long long *band_holes;  // reserved slots left unused (marked kBandHole); may be null
     uint32_t *err;
     float *dbg;                     // optional: s_hat for every pair, input order [na][nb] (tests)
@@ -1106,7 +1107,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     }
                     // min_j (|b_j|^2 - 2 v_j) >= gmin - 2 max_j v_j per 32-column group, gmin
                     // the group's minimum norm (0 where the norms are in the accumulator:
-                    // exact); one vote for the chunk
+                    // exact); a vote per group, both taken before any branch
                     const float m0 = fmaf(-2.0f, max32(v), c ? gmin[2] : gmin[0]);
                     const float m1 = fmaf(-2.0f, max32(v + 32), c ? gmin[3] : gmin[1]);
                     const uint32_t r0 = __ballot_sync(0xffffffffu, m0 <= thr_fast);

@@ -317,10 +317,9 @@ void launch_norm_key(const void *x, int dtype_bytes, uint64_t n, uint32_t d, con
 // Dimension cost (the selectivity estimate of the reference's
 // outputStatistics, hilbertjoin/egojoin.cpp:523-592): the pairs of sampled points
 // in equal cells, sum h(h-1)/2, plus the pairs in adjacent cells, sum h[c-1] h[c],
-// of one dim's cell histogram h. A dim of up to kCostSample cells has its histogram
-// in shared memory (a cell more than eps apart from the range's ends holds a
-// sample as a rule, so this is the usual case: 30k x 100 took 85 us sorted, 9 us
-// here). A wider dim's cell indices are sorted (bitonic), and every sample position s
+// of one dim's cell histogram h. Where the dim's cells span fewer than kCostSample (cmax -
+// cmin, over all points: ranges up to 8192 eps), the histogram is kept in shared memory
+// (30k x 100: 9 us, sorted 85). A wider dim's cell indices are sorted (bitonic), and every sample position s
 // counts the positions q > s with cell[q] <= cell[s] + 1 by a binary search -- the
 // same sum.
 __global__ void __launch_bounds__(1024) k_dim_cost(const void *x, int dtype_bytes, uint64_t n, uint32_t d,
@@ -1196,7 +1195,7 @@ __device__ __forceinline__ void norm_pieces(double v, typename BcElem<OP>::E (&m
 // from FP64 (scale a power of two: exact); TF32 and BF16 from the FP32 value
 // of x - center, BF16 as hi + lo with lo the BF16 of the exact remainder.
 // With `fold` (not BF16), columns d .. d + 2 hold the pieces of half the rank's norm
-// (norm_pieces; padding ranks a norm that no pair reaches).
+// (norm_pieces; padding ranks a large norm, no column of theirs is counted).
 template <typename T, int OP>  // OP: 0 TF32, 1 BF16 hi/lo, 2 FP16
 __global__ void __launch_bounds__(256) k_gather_tc_fused(const T *__restrict__ x, uint64_t n, uint32_t d,
                                                          const uint32_t *__restrict__ perm,
